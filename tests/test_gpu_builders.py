@@ -1,0 +1,46 @@
+"""The volume's builders (baked NEE grid, HG table, TR levels, occupancy and
+pyramid) at the sizes and inputs where their kernels take another branch,
+against the CPU oracle."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def blob(R, lo, hi, seed=3, negative=False):
+    """Zero but for the box [lo, hi) per axis."""
+    d = np.zeros((R, R, R), np.float32)
+    rng = np.random.default_rng(seed)
+    d[lo[0]:hi[0], lo[1]:hi[1], lo[2]:hi[2]] = rng.uniform(-0.1 if negative else 0.05, 1.0,
+                                                            [h - l for l, h in zip(lo, hi)])
+    return d
+
+
+@pytest.mark.parametrize("light", [(0.0, 1.0, 0.0), (0.0, 0.0, -1.0), (0.36, -0.48, 0.8)])
+@pytest.mark.parametrize("replicate", [True, False])
+@pytest.mark.parametrize("R,lo,hi,storage", [(24, (2, 9, 3), (9, 20, 24), "fp32"), (17, (0, 0, 0), (17, 17, 17), "fp16"),
+                                             (24, (0, 0, 0), (0, 0, 0), "fp32"), (40, (30, 1, 12), (31, 2, 13), "fp32")])
+def test_baked_voxels(light, replicate, R, lo, hi, storage):
+    """Every voxel's estimate follows the oracle's draws.  A logarithm's last
+    bit moves a step by up to 2^-23 and its density by that times R times the
+    voxel-to-voxel slope (below 1), a few steps a walk: below 1e-4; a walk
+    takes another course where a comparison falls into such a gap: far below
+    1 % of the voxels.  Lights along an axis, an off-centre and a one-voxel
+    box, a full one and an empty one."""
+    import mrpnn_b200 as M
+    M.init()
+    B, alpha = 13, 40.0
+    data = blob(R, lo, hi)
+    if storage == "fp16":
+        data = data.astype(np.float16).astype(np.float32)
+    v = M.VolumeRender(R, storage=storage)
+    v.set_data(data)
+    v.Update()
+    v.SetBakeResolution(B, replicate)
+    v.Update_CachedTR(light, alpha)
+    got = v.read(M.api.RES_BAKED_TR)
+    sc = O.SceneBuf(data.ravel(), R, v.max_density)
+    ref = O.baked_tr_voxels(sc, alpha, np.array(light, np.float32), B, 0, np.arange(B ** 3), replicate)
+    assert np.mean(np.abs(got - ref) > 1e-4) < 0.01
