@@ -8,6 +8,9 @@
 // texture + surface references (core/volume.cu:1322-1400, 1535-1696).  Here
 // every resource is a plain z-fastest fp32 array in HBM produced by one
 // kernel launch per level, on the volume's stream.
+#include <cmath>
+#include <vector>
+
 #include "kernels.h"
 
 namespace mrp {
@@ -270,47 +273,102 @@ __global__ void k_tr_level(float* __restrict__ out, int res, const float* __rest
 // file), the per-texel shift bn comes from the texel's LUT stream instead of
 // a curand draw.
 // ---------------------------------------------------------------------------
-__constant__ uint32_t c_perm[28];
-__constant__ uint32_t c_primes[5] = {2, 3, 5, 7, 11};
-__constant__ uint32_t c_prime_sums[5] = {0, 2, 5, 10, 17};
+constexpr int kHgSamples = 1024;
+// The scrambled radical inverses of samples 0..1023 in bases 2, 3, 5 and 11
+// (x, y, z, w), the same for every texel: filled from the host.
+__device__ float4 d_halton[kHgSamples];
 
-MRP_D float scrambled_radical_inverse(int bi, uint32_t a) {
-    const uint32_t base = c_primes[bi], off = c_prime_sums[bi];
-    const float inv_base = fd(1.0f, (float)base);
+static float scrambled_radical_inverse(uint32_t base, const uint32_t* perm, uint32_t a) {
+    const float inv_base = 1.0f / (float)base;
     uint32_t rev = 0;
     float inv_base_n = 1.0f;
     while (a) {
         uint32_t next = a / base;
         uint32_t digit = a - next * base;
-        rev = rev * base + c_perm[off + digit];
-        inv_base_n = fm(inv_base_n, inv_base);
+        rev = rev * base + perm[digit];
+        inv_base_n = inv_base_n * inv_base;
         a = next;
     }
-    return fminf(fm(inv_base_n, fa((float)rev, fd(fm(inv_base, (float)c_perm[off]), fs(1.0f, inv_base)))), 0.99999994f);
+    const float tail = (inv_base * (float)perm[0]) / (1.0f - inv_base);
+    return std::fmin(inv_base_n * ((float)rev + tail), 0.99999994f);
 }
-MRP_D float fracf_(float f) { return fs(f, (float)(long)f); }
+// frac(f) = f - (float)(long)f for 0 <= f < 2
+MRP_D float frac2(float f) { return f >= 1.0f ? fs(f, 1.0f) : f; }
 
-__global__ void k_hg_lut(float* __restrict__ lut, float g, uint32_t seed) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= kLut || j >= kLut) return;
-    float costheta = (float)((((double)(float)i + 0.5) / kLut) * 2.0 - 1.0);
-    float aa = (float)(((double)(float)j + 0.5) / kLut);
-    float angle = (float)((double)aa * 3.1415926535 * 60.0 / 180.0);
+// One texel's constants and its two sample estimators.  The arithmetic is
+// Fill_Hg's; terms that its vectors carry without effect are left out: the
+// view direction is (1, 0, 0) and the texel's direction has no z, so of
+// sample_hg's vector only x = cos and y = -sin sin(phi) enter the dot
+// product, and dot(normalize(p), view) is p.x / length(p).
+struct HgTexel {
+    float g, radius, bn;
+    f3 dir;
+    MRP_D float phase_sample(float4 q) const {   // a direction drawn from the phase function
+        const float e0 = frac2(fa(q.x, bn)), e1 = frac2(fa(q.y, bn));
+        float cost;
+        if (fabsf(g) < 0.0001) {
+            cost = fs(fm(e0, 2.0f), 1.0f);
+        } else {
+            const float g2 = fm(g, g);
+            const float t0 = fd(fs(1.0f, g2), fa(fs(1.0f, g), fm(fm(2.0f, g), e0)));
+            cost = fd(fs(fa(1.0f, g2), fm(t0, t0)), fm(2.0f, g));
+        }
+        const float phi = (float)(2.0 * 3.14159265359 * (double)e1);
+        const float sint = fsq(fmaxf(0.0f, fs(1.0f, fm(cost, cost))));
+        const float sdotl = fa(fm(dir.x, cost), fm(dir.y, -fm(sint, sinf(phi))));
+        const float p = fa(fs(fm(radius, radius), 1.0f), fm(sdotl, sdotl));
+        if (p <= 0) return 0.0f;
+        const float w = fsq(p);
+        float d0 = fs(sdotl, w);
+        const float d1 = fd(fa(sdotl, w), radius);
+        d0 = fd(fmaxf(0.0f, d0), radius);
+        const float d = fs(fm(fm(d1, d1), d1), fm(fm(d0, d0), d0));
+        return fmaxf(0.0f, fd(d, 4.0f));
+    }
+    MRP_D float cone_sample(float4 q) const {    // a point of the ball around the direction
+        const float rx = frac2(fa(q.x, bn)), ry = frac2(fa(q.y, bn)), rz = frac2(fa(q.z, bn));
+        const float theta = (float)((double)rx * 2.0 * 3.1415926535);
+        const float phi = (float)acos(2.0 * (double)ry - 1.0);
+        const float r = powf(rz, fd(1.0f, 3.0f));
+        const float st_ = sinf(theta), ct = cosf(theta), sp = sinf(phi), cp = cosf(phi);
+        const float rr = fm(radius, r), rs = fm(rr, sp);
+        const f3 rp = add(mk3(fm(rs, ct), fm(rs, st_), fm(rr, cp)), dir);
+        return hg(fd(rp.x, length(rp)), g);
+    }
+};
+
+// One texel a thread, 128 texels of a row a block, 32 samples at a time.  A
+// sample is of one kind or the other (frac(w + bn) < mis); lanes disagree on
+// almost every sample, so the kinds are taken apart: each lane runs through
+// its own phase samples, then through its own cone samples, leaves the terms
+// in its column of shared memory and adds them there in sample order, which
+// keeps the sum's rounding.  Bound by the estimators' instructions (double
+// acos, powf twice, sines and cosines in a cone sample).  One table: 12.85 ms
+// with the digits of every inverse worked out per texel and both kinds run in
+// turn for every sample, 4.19 ms this way (the same bits).
+constexpr int kHgChunk = 32;
+__global__ void __launch_bounds__(128) k_hg_lut(float* __restrict__ lut, float g, uint32_t seed) {
+    __shared__ float4 pts[kHgSamples];
+    __shared__ float term[kHgChunk][128];
+    for (int k = threadIdx.x; k < kHgSamples; k += 128) pts[k] = d_halton[k];
+    const int i = blockIdx.x * 128 + threadIdx.x, j = blockIdx.y;
+    const float costheta = (float)((((double)(float)i + 0.5) / kLut) * 2.0 - 1.0);
+    const float aa = (float)(((double)(float)j + 0.5) / kLut);
+    const float angle = (float)((double)aa * 3.1415926535 * 60.0 / 180.0);
     Stream st(kLutStream, (uint32_t)(j * kLut + i), 0, 0, seed);
-    float bn = st.next();
-    float h = 0.0f;
-    float radius = tanf(angle);
-    f3 view = mk3(1.0f, 0.0f, 0.0f);
-    f3 dir = mk3(costheta, fsq(fs(1.0f, fm(costheta, costheta))), 0.0f);
+    HgTexel T;
+    T.g = g;
+    T.bn = st.next();
+    T.radius = tanf(angle);
+    T.dir = mk3(costheta, fsq(fs(1.0f, fm(costheta, costheta))), 0.0f);
     float mis = 0;
     {
-        float p = fa(fs(fm(radius, radius), 1.0f), fm(dir.x, dir.x));
+        float p = fa(fs(fm(T.radius, T.radius), 1.0f), fm(T.dir.x, T.dir.x));
         if (p > 0) {
-            float sdotl = g > 0 ? dir.x : -dir.x;
+            float sdotl = g > 0 ? T.dir.x : -T.dir.x;
             float w = fsq(p);
-            float d0 = fd(fmaxf(0.0f, fs(sdotl, w)), radius);
-            float d1 = fd(fa(sdotl, w), radius);
+            float d0 = fd(fmaxf(0.0f, fs(sdotl, w)), T.radius);
+            float d1 = fd(fa(sdotl, w), T.radius);
             float d = fs(fm(fm(d1, d1), d1), fm(fm(d0, d0), d0));
             mis = fm((float)(d1 > d0), d);
         }
@@ -320,35 +378,25 @@ __global__ void k_hg_lut(float* __restrict__ lut, float g, uint32_t seed) {
         a = (float)(ad < 0.6 ? 0.0 : (ad < 0.7 ? (ad - 0.6) * 9 : (pow((ad - 0.7) / 0.3, 0.05) * 0.1 + 0.9)));
         mis = fs(1.0f, fd(1.0f, fa(1.0f, fd(fm(a, mis), fs(1.0f, a)))));
     }
-    for (uint32_t k = 0; k < 1024; ++k) {
-        if (fracf_(fa(scrambled_radical_inverse(4, k), bn)) < mis) {
-            float rx = fracf_(fa(scrambled_radical_inverse(0, k), bn));
-            float ry = fracf_(fa(scrambled_radical_inverse(1, k), bn));
-            f3 l = sample_hg(rx, ry, view, g);
-            float sdotl = dot(dir, l);
-            float p = fa(fs(fm(radius, radius), 1.0f), fm(sdotl, sdotl));
-            if (p <= 0) continue;
-            float w = fsq(p);
-            float d0 = fs(sdotl, w);
-            float d1 = fd(fa(sdotl, w), radius);
-            d0 = fd(fmaxf(0.0f, d0), radius);
-            float d = fs(fm(fm(d1, d1), d1), fm(fm(d0, d0), d0));
-            h = fa(h, fmaxf(0.0f, fd(d, 4.0f)));
-        } else {
-            float rx = fracf_(fa(scrambled_radical_inverse(0, k), bn));
-            float ry = fracf_(fa(scrambled_radical_inverse(1, k), bn));
-            float rz = fracf_(fa(scrambled_radical_inverse(2, k), bn));
-            float theta = (float)((double)rx * 2.0 * 3.1415926535);
-            float phi = (float)acos(2.0 * (double)ry - 1.0);
-            float r = powf(rz, fd(1.0f, 3.0f));
-            float st_ = sinf(theta), ct = cosf(theta), sp = sinf(phi), cp = cosf(phi);
-            float x = fm(fm(fm(radius, r), sp), ct), y = fm(fm(fm(radius, r), sp), st_), z = fm(fm(radius, r), cp);
-            f3 rp = add(mk3(x, y, z), dir);
-            float c = dot(normalize(rp), view);
-            h = fa(h, hg(c, g));
+    __syncthreads();
+    float h = 0.0f;
+    float* own = &term[0][threadIdx.x];
+    for (int k0 = 0; k0 < kHgSamples; k0 += kHgChunk) {
+        uint32_t phase = 0;
+#pragma unroll 8
+        for (int k = 0; k < kHgChunk; ++k) phase |= (uint32_t)(frac2(fa(pts[k0 + k].w, T.bn)) < mis) << k;
+        for (uint32_t m = phase; m; m &= m - 1) {
+            const int k = __ffs(m) - 1;
+            own[k * 128] = T.phase_sample(pts[k0 + k]);
         }
+        for (uint32_t m = ~phase; m; m &= m - 1) {
+            const int k = __ffs(m) - 1;
+            own[k * 128] = T.cone_sample(pts[k0 + k]);
+        }
+#pragma unroll 8
+        for (int k = 0; k < kHgChunk; ++k) h = fa(h, own[k * 128]);
     }
-    lut[j * kLut + i] = fd(h, 1024.0f);
+    lut[j * kLut + i] = fd(h, (float)kHgSamples);
 }
 
 MRP_D float density(const VolumeDev& v, f3 p) { return density_tex(v, p); }
@@ -555,10 +603,14 @@ cudaError_t launch_tr_level(float* out, int res, const float* src, const uint8_t
     return cudaGetLastError();
 }
 cudaError_t set_halton_permutations(const uint32_t perm[28]) {
-    return cudaMemcpyToSymbol(c_perm, perm, sizeof(uint32_t) * 28);
+    std::vector<float4> h(kHgSamples);
+    for (uint32_t k = 0; k < (uint32_t)kHgSamples; ++k)
+        h[k] = make_float4(scrambled_radical_inverse(2, perm, k), scrambled_radical_inverse(3, perm + 2, k),
+                           scrambled_radical_inverse(5, perm + 5, k), scrambled_radical_inverse(11, perm + 17, k));
+    return cudaMemcpyToSymbol(d_halton, h.data(), kHgSamples * sizeof(float4));
 }
 cudaError_t launch_hg_lut(float* lut, float g, uint32_t seed, cudaStream_t s) {
-    k_hg_lut<<<dim3(kLut / 16, kLut / 16), dim3(16, 16), 0, s>>>(lut, g, seed);
+    k_hg_lut<<<dim3(kLut / 128, kLut), 128, 0, s>>>(lut, g, seed);
     return cudaGetLastError();
 }
 cudaError_t launch_baked_tr(float* out, const VolumeDev& v, int bake_res, float alpha, const float L[3], uint32_t seed,

@@ -44,3 +44,24 @@ def test_baked_voxels(light, replicate, R, lo, hi, storage):
     sc = O.SceneBuf(data.ravel(), R, v.max_density)
     ref = O.baked_tr_voxels(sc, alpha, np.array(light, np.float32), B, 0, np.arange(B ** 3), replicate)
     assert np.mean(np.abs(got - ref) > 1e-4) < 0.01
+
+
+@pytest.mark.parametrize("g,seed", [(0.857, 5), (0.65, 0), (0.0, 1), (-0.8, 2), (0.00005, 3)])
+def test_hg_table_texels(g, seed):
+    """The table's kinds of sample (only cone samples at g = 0 and below 0.6,
+    both above), its corners and a random choice, with the bars of the
+    existing table test: a texel can flip one of its 1024 samples between the
+    kinds when a transcendental differs in the last bit."""
+    import mrpnn_b200 as M
+    M.init()
+    rng = np.random.default_rng(seed)
+    tex = np.unique(np.concatenate([[0, 511, 512 * 511, 512 * 512 - 1, 127, 128, 255, 256],
+                                    rng.choice(512 * 512, 1500, replace=False)])).astype(np.int32)
+    v = M.VolumeRender(16)
+    v.SetSeed(seed)
+    v.UpdateHGLut(g)
+    got = v.read(M.api.RES_LUT)[tex]
+    ref = O.hg_lut_texels(g, seed, tex)
+    rel = np.abs(got - ref) / np.maximum(np.abs(ref), 1e-6)
+    assert np.mean(rel < 1e-4) > 0.995, np.sort(rel)[-10:]
+    assert np.max(rel) < 0.05
