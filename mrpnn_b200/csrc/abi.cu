@@ -299,6 +299,7 @@ mrp_status mrp_volume_create_ex(int res, mrp_storage storage, mrp_volume** out) 
         (e = mrp::dev_malloc(&v->occ2, (size_t)v->occ2_res * v->occ2_res * v->occ2_res)) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->d_maxbits, sizeof(int))) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->d_bounds, 6 * sizeof(int))) != cudaSuccess ||
+        (e = mrp::dev_malloc(&v->mips_tr, kTrPadFloats * sizeof(float))) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->mips_pad, kPadLevelFloats * sizeof(float))) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->trs_pad, kPadLevelFloats * sizeof(float))) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->mip_tr, mip_tr_offset(5) * sizeof(float2))) != cudaSuccess ||
@@ -320,7 +321,7 @@ mrp_status mrp_volume_destroy(mrp_volume* v) {
     if (v->stream_copy) cudaStreamSynchronize(v->stream_copy);
     mrp::dev_free(v->accum_alt);
     mrp::dev_free(v->density); mrp::dev_free(v->density_h); mrp::dev_free(v->mips); mrp::dev_free(v->trs); mrp::dev_free(v->lut); mrp::dev_free(v->baked);
-    mrp::dev_free(v->occ); mrp::dev_free(v->occ2); mrp::dev_free(v->mip_occ); mrp::dev_free(v->d_maxbits); mrp::dev_free(v->d_bounds); mrp::dev_free(v->mips_pad); mrp::dev_free(v->trs_pad); mrp::dev_free(v->mip_tr); mrp::dev_free(v->pad_pair); mrp::dev_free(v->accum); mrp::dev_free(v->sum3); mrp::dev_free(v->first_pos);
+    mrp::dev_free(v->occ); mrp::dev_free(v->occ2); mrp::dev_free(v->mip_occ); mrp::dev_free(v->d_maxbits); mrp::dev_free(v->d_bounds); mrp::dev_free(v->mips_tr); mrp::dev_free(v->mips_pad); mrp::dev_free(v->trs_pad); mrp::dev_free(v->mip_tr); mrp::dev_free(v->pad_pair); mrp::dev_free(v->accum); mrp::dev_free(v->sum3); mrp::dev_free(v->first_pos);
     mrp::dev_free(v->counter);
     mrp::dev_free(v->hdri);
     drop_density_texture(v);
@@ -587,6 +588,7 @@ mrp_status mrp_volume_update(mrp_volume* v, int process_mips) {
                                 v->stream));
         CU(launch_pad_levels(v->mips + mip_offset(5), v->mips + mip_offset(6), v->mips + mip_offset(7), false,
                              v->mips_pad, v->stream));
+        CU(launch_pad_pyramid(v->mips, v->mips_tr, g.sms, v->stream));
         CU(cudaStreamSynchronize(v->stream));
         mrp::dev_free(tmp[0]);
         mrp::dev_free(tmp[1]);
@@ -712,15 +714,14 @@ mrp_status mrp_volume_read(mrp_volume* v, mrp_resource which, int level, float* 
 namespace mrpi {
 // Fill_TR for all 8 TR levels: level lv (res 128 >> lv) through density mip
 // lv + 1 with alpha / 1.73^(lv + 1) (core/volume.cu:1535-1560).
-cudaError_t build_tr_levels(float* trs, const float* mips, const uint8_t* mip_occ, const float L[3], float alpha,
-                            cudaStream_t s) {
-    for (int lv = 0; lv < 8; ++lv) {
-        float a = alpha / std::pow(1.73f, (float)lv + 1.0f);
-        const uint8_t* occ = mip_occ && lv + 1 < kOccMips ? mip_occ + mip_occ_offset(lv + 1) : nullptr;
-        cudaError_t e = launch_tr_level(trs + tr_offset(lv), 128 >> lv, mips + mip_offset(lv + 1), occ, a, L, g.sms, s);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+cudaError_t build_tr_levels(float* trs, const mrp_volume* v, const float L[3], float alpha, cudaStream_t s) {
+    TrArgs a;
+    for (int lv = 0; lv < 8; ++lv) a.alpha[lv] = alpha / std::pow(1.73f, (float)lv + 1.0f);
+    a.L = mk3(L[0], L[1], L[2]);
+    const VolumeDev d = v->dev();
+    a.lo = d.has_bounds ? d.nz_lo : mk3(-2.0f, -2.0f, -2.0f);
+    a.hi = d.has_bounds ? d.nz_hi : mk3(2.0f, 2.0f, 2.0f);
+    return launch_tr_levels(trs, v->mips, v->mips_tr, v->mip_occ, a, s);
 }
 }  // namespace mrpi
 extern "C" {
@@ -740,7 +741,7 @@ mrp_status update_tr_async(mrp_volume* v, const float L[3], float alpha) {
     if (!v->has_pyramid) return fail(MRP_ERR_NOT_READY, "TR mips need the pyramid (call mrp_volume_update)");
     if (v->has_tr && v->tr_alpha == alpha && v->tr_light[0] == L[0] && v->tr_light[1] == L[1] && v->tr_light[2] == L[2])
         return sync_gather_textures(v);
-    CU(build_tr_levels(v->trs, v->mips, v->mip_occ, L, alpha, v->stream));
+    CU(build_tr_levels(v->trs, v, L, alpha, v->stream));
     CU(launch_pad_levels(v->trs + tr_offset(4), v->trs + tr_offset(5), v->trs + tr_offset(6), true, v->trs_pad,
                          v->stream));
     CU(launch_interleave_mip_tr(v->mips, v->trs, v->mip_tr, g.sms, v->stream));

@@ -50,9 +50,8 @@ extern Lib g;
 
 // Device view of one camera launch (RenderCamera's arguments).
 ViewDev make_view(const mrp_volume* v, const mrp_view* w, int frame, int mean_k);
-// Fill_TR for the 8 TR levels of a pyramid into trs (kTrFloats floats).
-cudaError_t build_tr_levels(float* trs, const float* mips, const uint8_t* mip_occ, const float L[3], float alpha,
-                            cudaStream_t s);
+// Fill_TR for the 8 TR levels of the volume's pyramid into trs (kTrFloats floats).
+cudaError_t build_tr_levels(float* trs, const mrp_volume* v, const float L[3], float alpha, cudaStream_t s);
 
 // Per-volume caches of the predictor, queued on the volume's stream: the HG
 // LUT for g (UpdateHGLut) and the TR mips for (light, alpha) (Update_TR).
@@ -112,6 +111,7 @@ struct mrp_volume {
     uint8_t* occ2 = nullptr;      // coarse occupancy (4^3 bricks each), built with occ
     int occ2_res = 0;
     int* d_maxbits = nullptr;
+    float* mips_tr = nullptr;     // mips 1..8 with a border of zeros, built with the pyramid for the TR levels
     float* mips_pad = nullptr;    // padded mips 5..7 (pad_offset layout), built with the pyramid
     float* trs_pad = nullptr;     // padded TR levels 4..6, built with the TR levels
     float2* mip_tr = nullptr;     // (mip L, TR L - 1) texel pairs, L = 1..4, built with the TR levels

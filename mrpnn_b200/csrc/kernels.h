@@ -34,8 +34,18 @@ cudaError_t launch_pad_levels(const float* l8, const float* l4, const float* l2,
 // max y, max z}, which must start at {R, R, R, -1, -1, -1}.
 cudaError_t launch_nonzero_bounds(const float* d, int R, int* out6, int sms, cudaStream_t s);
 cudaError_t launch_nonzero_bounds(const __half* d, int R, int* out6, int sms, cudaStream_t s);
-cudaError_t launch_tr_level(float* out, int res, const float* src, const uint8_t* src_occ, float alpha, const float L[3], int sms,
-                            cudaStream_t s);
+// Copies of mips 1..8 with a border of zeros (kTrPadFloats floats), which the
+// TR levels are marched through.
+cudaError_t launch_pad_pyramid(const float* mips, float* mips_tr, int sms, cudaStream_t s);
+// The eight TR levels (trs: tr_offset layout) from the pyramid and its padded
+// copies; mip_occ may be null.
+struct TrArgs {
+    float alpha[8];   // extinction scale of each level
+    f3 L;             // toward the light
+    f3 lo, hi;        // VolumeDev::nz_lo, nz_hi (anything that holds the cube when not known)
+};
+cudaError_t launch_tr_levels(float* trs, const float* mips, const float* mips_tr, const uint8_t* mip_occ,
+                             const TrArgs& args, cudaStream_t s);
 cudaError_t set_halton_permutations(const uint32_t perm[28]);
 cudaError_t launch_hg_lut(float* lut, float g, uint32_t seed, cudaStream_t s);
 cudaError_t launch_baked_tr(float* out, const VolumeDev& v, int bake_res, float alpha, const float L[3], uint32_t seed,

@@ -381,7 +381,7 @@ bool mrp_server::admit() {
         HitRecords rec = s.records();
         const GtexLevel* trl = &s.gtr0;
         const float* trsrc = s.trs;
-        if ((e = build_tr_levels(s.trs, v->mips, v->mip_occ, w.light_dir, w.alpha, s.stream)) != cudaSuccess ||
+        if ((e = build_tr_levels(s.trs, v, w.light_dir, w.alpha, s.stream)) != cudaSuccess ||
             (use_tex && ((e = gtex_fill(&trl, &trsrc, 1, g.sms, s.stream)) != cudaSuccess ||
                          (e = gtex_fill_pairs(s.gpair, v->mips, s.trs, g.sms, s.stream)) != cudaSuccess)) ||
             (e = launch_hit(s.vd, s.view, rec, s.accum, s.stream)) != cudaSuccess ||

@@ -244,26 +244,151 @@ __global__ void k_occupancy_coarse(const uint8_t* __restrict__ occ, int nb, int 
 // Fill_TR (core/volume.cu:1535-1560): transmittance of TR level `level`
 // (res 128>>level) marched 128 steps toward the light through density level
 // level+1 with alpha scaled by 1.73^(level+1) (core/volume.cu:1636-1653).
+//
+// One launch for all eight levels, the small ones first: their 128 steps in
+// series take about as long as a level of any size (28 to 56 us each when
+// launched one after the other), so they run beside level 0's blocks.  Bound
+// by level 0's instructions (2 M voxels x 128 steps).  The levels are read
+// from copies with a border of zeros (tr_pad_off): a voxel at a face takes
+// 128 tiny steps there, and with another kind of fetch for the edge one such
+// lane sends its whole warp through both.  All levels of a 256^3 cloud:
+// 1.13 ms in eight launches, 0.84 ms in one, 0.51 ms from the padded copies
+// with floor taken by an addition, 0.43 ms with the steps cut to the box of
+// nonzero voxels.
 // ---------------------------------------------------------------------------
-// src_occ (may be null): 8^3 brick flags of src; empty bricks add exactly 0.
-__global__ void k_tr_level(float* __restrict__ out, int res, const float* __restrict__ src,
-                           const uint8_t* __restrict__ src_occ, float alpha, f3 L) {
-    size_t n = (size_t)res * res * res;
-    float rf = (float)res;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        int z = (int)(i % res), y = (int)((i / res) % res), x = (int)(i / ((size_t)res * res));
-        f3 uv = div(adds(mk3((float)x, (float)y, (float)z), 0.5f), rf);
-        f3 ori = subs(uv, 0.5f);
-        float dis = ray_box_distance(ori, L);
-        float step = fd(dis, 128.0f);
-        f3 lp = ori;
-        float acc = 0;
-        for (int s = 0; s < 128; ++s) {
-            lp = add(lp, mul(L, step));
-            acc = fa(acc, src_occ ? tex3_occ(src, res, src_occ, (res + 7) >> 3, lp) : tex3<false>(src, res, lp));
-        }
-        out[i] = fm(1.0f, fm(expf(fm(fm(-acc, alpha), step)), 1.0f));
+constexpr int kTrLevels = 8, kTrThreads = 128;
+__host__ __device__ constexpr int tr_blocks(int lv) {   // blocks of level lv
+    const int n = 128 >> lv;
+    return (n * n * n + kTrThreads - 1) / kTrThreads;
+}
+__host__ __device__ constexpr int tr_first_block(int lv) {   // levels 7, 6, ..., 0 in that order
+    int o = 0;
+    for (int l = kTrLevels - 1; l > lv; --l) o += tr_blocks(l);
+    return o;
+}
+// Padded copy of mip lv + 1 (edge n = 128 >> lv): (n + 2)^3 floats, texel
+// (x, y, z) at ((x + 1) P + y + 1) P + z + 1 with P = n + 2, zeros around.
+__host__ __device__ constexpr int tr_pad_off(int lv) {
+    int o = 0;
+    for (int l = 0; l < lv; ++l) { const int p = (128 >> l) + 2; o += p * p * p; }
+    return o;
+}
+static_assert(tr_pad_off(kTrLevels) == (int)kTrPadFloats, "padded pyramid size");
+__global__ void k_pad_pyramid(const float* __restrict__ mips, float* __restrict__ out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (int)kTrPadFloats; i += gridDim.x * blockDim.x) {
+        int lv = 0;
+        while (lv + 1 < kTrLevels && i >= tr_pad_off(lv + 1)) ++lv;
+        const int n = 128 >> lv, P = n + 2, j = i - tr_pad_off(lv);
+        const int x = j / (P * P) - 1, y = (j / P) % P - 1, z = j % P - 1;
+        out[i] = fetch_border(mips + mip_offset(lv + 1), n, x, y, z);
     }
+}
+
+
+// Sum of the density over 128 steps of d from p through level LV, in tex3's
+// arithmetic: the edge is a power of two, so u N is exact and u N - 0.5 one
+// fused operation, and adding 1.5 2^23 rounding down leaves floor in the low
+// mantissa bits (the offsets of those bits fold into the addresses).  An
+// empty brick adds exactly 0 and is skipped.  Steps before `first` only move
+// p, steps from `last` on are left out (both read 0).  The steps must stay
+// within a quarter of a texel of the unit cube.
+template <int LV>
+MRP_D float tr_march(const float* __restrict__ pad, const uint8_t* __restrict__ occ, f3 p, f3 d, int first, int last) {
+    constexpr int N = 128 >> LV, P = N + 2, NB = (N + 7) >> 3;
+    constexpr float kFloor = 12582912.0f;
+    constexpr uint32_t kBits = 0x4B400000u;
+    constexpr uint32_t kBase = (kBits - 1u) * (uint32_t)(P * P + P + 1);
+    constexpr uint32_t kBrick = (kBits >> 3) * (uint32_t)(NB * NB + NB + 1);
+    float acc = 0.0f;
+    int s = 0;
+    for (; s < first; ++s) p = add(p, d);
+    for (; s < last; ++s) {
+        p = add(p, d);
+        const float px = fmaf(fa(p.x, 0.5f), (float)N, -0.5f), py = fmaf(fa(p.y, 0.5f), (float)N, -0.5f),
+                    pz = fmaf(fa(p.z, 0.5f), (float)N, -0.5f);
+        const float tx = __fadd_rd(px, kFloor), ty = __fadd_rd(py, kFloor), tz = __fadd_rd(pz, kFloor);
+        const uint32_t x = __float_as_uint(tx), y = __float_as_uint(ty), z = __float_as_uint(tz);
+        if (occ) {   // voxel -1 belongs to brick 0
+            const uint32_t bx = max(x, kBits) >> 3, by = max(y, kBits) >> 3, bz = max(z, kBits) >> 3;
+            if (__ldg(occ + ((bx * NB + by) * NB + bz - kBrick)) == 0) continue;
+        }
+        const float wx = fs(px, fs(tx, kFloor)), wy = fs(py, fs(ty, kFloor)), wz = fs(pz, fs(tz, kFloor));
+        const float ox = fs(1.0f, wx), oy = fs(1.0f, wy), oz = fs(1.0f, wz);
+        const float* b = pad + ((x * P + y) * P + z - kBase);
+        const float c00 = lerp_w(__ldg(b), __ldg(b + 1), wz, oz), c01 = lerp_w(__ldg(b + P), __ldg(b + P + 1), wz, oz);
+        const float c10 = lerp_w(__ldg(b + P * P), __ldg(b + P * P + 1), wz, oz),
+                    c11 = lerp_w(__ldg(b + P * P + P), __ldg(b + P * P + P + 1), wz, oz);
+        acc = fa(acc, lerp_w(lerp_w(c00, c01, wy, oy), lerp_w(c10, c11, wy, oy), wx, ox));
+    }
+    return acc;
+}
+// The same by general fetches, for rays that leave the cube (a light
+// direction that is not a number).
+__device__ __noinline__ float tr_march_any(const float* __restrict__ mip, int n, f3 p, f3 d) {
+    float acc = 0.0f;
+    for (int s = 0; s < 128; ++s) {
+        p = add(p, d);
+        acc = fa(acc, tex3<false>(mip, n, p));
+    }
+    return acc;
+}
+// One voxel of level LV; mip_occ (may be null): 8^3 brick flags of mip levels 0..kOccMips-1.
+template <int LV>
+MRP_D void tr_voxel(float* __restrict__ trs, const float* __restrict__ mips, const float* __restrict__ mips_tr,
+                    const uint8_t* __restrict__ mip_occ, const TrArgs& A) {
+    constexpr int N = 128 >> LV;
+    const f3 L = A.L;
+    const int i = ((int)blockIdx.x - tr_first_block(LV)) * kTrThreads + (int)threadIdx.x;
+    if (i >= N * N * N) return;
+    const int z = i % N, y = (i / N) % N, x = i / (N * N);
+    const f3 uv = div(adds(mk3((float)x, (float)y, (float)z), 0.5f), (float)N);
+    const f3 ori = subs(uv, 0.5f);
+    const float dis = ray_box_distance(ori, L);
+    const float step = fd(dis, 128.0f);
+    const f3 d = mul(L, step);
+    constexpr float lim = 0.5f + 0.25f / N;
+    const bool inside = fabsf(ori.x + 128.0f * d.x) <= lim && fabsf(ori.y + 128.0f * d.y) <= lim &&
+                        fabsf(ori.z + 128.0f * d.z) <= lim;
+    // the steps whose fetch can touch a nonzero texel: a nonzero voxel lies
+    // within 1/R + 2/N of it (a voxel of every level on the way down, half as
+    // large each, and the fetch's own footprint); the box of nonzero voxels
+    // has 2/R of margin already, and two steps cover the divisions' rounding
+    const float o[3] = {ori.x, ori.y, ori.z}, dd[3] = {d.x, d.y, d.z}, lo[3] = {A.lo.x, A.lo.y, A.lo.z},
+                hi[3] = {A.hi.x, A.hi.y, A.hi.z};
+    constexpr float grow = 2.25f / N;
+    float s0 = 0.0f, s1 = 128.0f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float l = lo[a] - grow - o[a], h = hi[a] + grow - o[a];
+        if (fabsf(dd[a]) < 1e-30f) {   // does not move along this axis
+            if (l > 0.0f || h < 0.0f) s1 = -1.0f;
+        } else {
+            const float r = 1.0f / dd[a], ta = l * r, tb = h * r;
+            s0 = fmaxf(s0, fminf(ta, tb));
+            s1 = fminf(s1, fmaxf(ta, tb));
+        }
+    }
+    const int last = s0 > s1 ? 0 : (int)fminf(s1 + 2.0f, 128.0f), first = (int)fmaxf(fminf(s0, 128.0f) - 3.0f, 0.0f);
+    const float acc =
+        inside ? tr_march<LV>(mips_tr + tr_pad_off(LV),
+                              LV + 1 < kOccMips && mip_occ ? mip_occ + mip_occ_offset(LV + 1) : nullptr, ori, d,
+                              first, last)
+               : tr_march_any(mips + mip_offset(LV + 1), N, ori, d);
+    trs[tr_offset(LV) + i] = fm(1.0f, fm(expf(fm(fm(-acc, A.alpha[LV]), step)), 1.0f));
+}
+__global__ void __launch_bounds__(kTrThreads) k_tr_levels(float* __restrict__ trs, const float* __restrict__ mips,
+                                                          const float* __restrict__ mips_tr,
+                                                          const uint8_t* __restrict__ mip_occ,
+                                                          const __grid_constant__ TrArgs A) {
+    const int b = (int)blockIdx.x;
+    if (b >= tr_first_block(0)) tr_voxel<0>(trs, mips, mips_tr, mip_occ, A);
+    else if (b >= tr_first_block(1)) tr_voxel<1>(trs, mips, mips_tr, mip_occ, A);
+    else if (b >= tr_first_block(2)) tr_voxel<2>(trs, mips, mips_tr, mip_occ, A);
+    else if (b >= tr_first_block(3)) tr_voxel<3>(trs, mips, mips_tr, mip_occ, A);
+    else if (b >= tr_first_block(4)) tr_voxel<4>(trs, mips, mips_tr, mip_occ, A);
+    else if (b >= tr_first_block(5)) tr_voxel<5>(trs, mips, mips_tr, mip_occ, A);
+    else if (b >= tr_first_block(6)) tr_voxel<6>(trs, mips, mips_tr, mip_occ, A);
+    else tr_voxel<7>(trs, mips, mips_tr, mip_occ, A);
 }
 
 // ---------------------------------------------------------------------------
@@ -596,10 +721,13 @@ cudaError_t launch_occupancy_coarse(const uint8_t* occ, int nb, uint8_t* coarse,
     k_occupancy_coarse<<<grid_for((size_t)total, 128, sms), 128, 0, s>>>(occ, nb, nc, coarse);
     return cudaGetLastError();
 }
-cudaError_t launch_tr_level(float* out, int res, const float* src, const uint8_t* src_occ, float alpha,
-                            const float L[3], int sms, cudaStream_t s) {
-    k_tr_level<<<grid_for((size_t)res * res * res, 128, sms), 128, 0, s>>>(out, res, src, src_occ, alpha,
-                                                                           mk3(L[0], L[1], L[2]));
+cudaError_t launch_pad_pyramid(const float* mips, float* mips_tr, int sms, cudaStream_t s) {
+    k_pad_pyramid<<<grid_for(kTrPadFloats, 256, sms), 256, 0, s>>>(mips, mips_tr);
+    return cudaGetLastError();
+}
+cudaError_t launch_tr_levels(float* trs, const float* mips, const float* mips_tr, const uint8_t* mip_occ,
+                             const TrArgs& args, cudaStream_t s) {
+    k_tr_levels<<<tr_first_block(0) + tr_blocks(0), kTrThreads, 0, s>>>(trs, mips, mips_tr, mip_occ, args);
     return cudaGetLastError();
 }
 cudaError_t set_halton_permutations(const uint32_t perm[28]) {

@@ -65,3 +65,24 @@ def test_hg_table_texels(g, seed):
     rel = np.abs(got - ref) / np.maximum(np.abs(ref), 1e-6)
     assert np.mean(rel < 1e-4) > 0.995, np.sort(rel)[-10:]
     assert np.max(rel) < 0.05
+
+
+@pytest.mark.parametrize("light", [(0.0, 1.0, 0.0), (0.0, 0.0, -1.0), (0.36, -0.48, 0.8), (-0.99, 0.1, 0.1)])
+@pytest.mark.parametrize("R,lo,hi", [(64, (0, 0, 0), (64, 64, 64)), (40, (30, 1, 12), (31, 2, 13)),
+                                     (33, (0, 31, 7), (5, 33, 26)), (24, (0, 0, 0), (0, 0, 0))])
+def test_tr_levels(light, R, lo, hi):
+    """All eight levels, rays along an axis and along the grid's faces, dense
+    to the border, in one corner, a single voxel and an empty grid; the
+    exponential's last bits are what may differ (the bar of the existing TR
+    test)."""
+    import mrpnn_b200 as M
+    M.init()
+    data = blob(R, lo, hi)
+    v = M.VolumeRender(R)
+    v.set_data(data)
+    v.Update()
+    v.Update_TR(light, 48.0)
+    mips = np.concatenate([v.read(M.api.RES_MIP, m) for m in range(9)])
+    got = np.concatenate([v.read(M.api.RES_TR, m) for m in range(8)])
+    ref = O.tr_mips(mips, 48.0, np.array(light, np.float32))
+    np.testing.assert_allclose(got, ref, rtol=2e-6, atol=1e-7)
