@@ -297,8 +297,8 @@ mrp_status mrp_volume_create_ex(int res, mrp_storage storage, mrp_volume** out) 
         (e = mrp::dev_malloc(&v->lut, kLutAlloc * sizeof(float))) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->occ, nocc)) != cudaSuccess || (e = mrp::dev_malloc(&v->mip_occ, kMipOccBytes)) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->occ2, (size_t)v->occ2_res * v->occ2_res * v->occ2_res)) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->d_maxbits, sizeof(int))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->d_bounds, 6 * sizeof(int))) != cudaSuccess ||
+        (e = mrp::dev_malloc(&v->d_stats, 7 * sizeof(int))) != cudaSuccess ||
+        (e = mrp::dev_malloc(&v->occ_rows, std::max(occ_row_words(res), kMipOccRows) * sizeof(uint4))) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->mips_tr, kTrPadFloats * sizeof(float))) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->mips_pad, kPadLevelFloats * sizeof(float))) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->trs_pad, kPadLevelFloats * sizeof(float))) != cudaSuccess ||
@@ -321,7 +321,7 @@ mrp_status mrp_volume_destroy(mrp_volume* v) {
     if (v->stream_copy) cudaStreamSynchronize(v->stream_copy);
     mrp::dev_free(v->accum_alt);
     mrp::dev_free(v->density); mrp::dev_free(v->density_h); mrp::dev_free(v->mips); mrp::dev_free(v->trs); mrp::dev_free(v->lut); mrp::dev_free(v->baked);
-    mrp::dev_free(v->occ); mrp::dev_free(v->occ2); mrp::dev_free(v->mip_occ); mrp::dev_free(v->d_maxbits); mrp::dev_free(v->d_bounds); mrp::dev_free(v->mips_tr); mrp::dev_free(v->mips_pad); mrp::dev_free(v->trs_pad); mrp::dev_free(v->mip_tr); mrp::dev_free(v->pad_pair); mrp::dev_free(v->accum); mrp::dev_free(v->sum3); mrp::dev_free(v->first_pos);
+    mrp::dev_free(v->occ); mrp::dev_free(v->occ2); mrp::dev_free(v->mip_occ); mrp::dev_free(v->d_stats); mrp::dev_free(v->occ_rows); mrp::dev_free(v->mips_tr); mrp::dev_free(v->mips_pad); mrp::dev_free(v->trs_pad); mrp::dev_free(v->mip_tr); mrp::dev_free(v->pad_pair); mrp::dev_free(v->accum); mrp::dev_free(v->sum3); mrp::dev_free(v->first_pos);
     mrp::dev_free(v->counter);
     mrp::dev_free(v->hdri);
     drop_density_texture(v);
@@ -529,30 +529,18 @@ mrp_status mrp_volume_update(mrp_volume* v, int process_mips) {
     if (!v) return fail(MRP_ERR_INVALID, "null volume");
     if (!v->has_data) return fail(MRP_ERR_NOT_READY, "update: no data set");
     int R = v->res;
-    size_t n = (size_t)R * R * R;
-    if (!v->max_override) {
-        int init;
-        { float f0 = 0.00001f; std::memcpy(&init, &f0, sizeof init); }
-        CU(cudaMemcpyAsync(v->d_maxbits, &init, sizeof(int), cudaMemcpyHostToDevice, v->stream));
-        if (v->density_h) CU(launch_max_density(v->density_h, n, v->d_maxbits, g.sms, v->stream));
-        else CU(launch_max_density(v->density, n, v->d_maxbits, g.sms, v->stream));
-        int bits = 0;
-        CU(cudaMemcpyAsync(&bits, v->d_maxbits, sizeof(int), cudaMemcpyDeviceToHost, v->stream));
-        CU(cudaStreamSynchronize(v->stream));
-        std::memcpy(&v->max_density, &bits, sizeof(float));
-    }
-    if (v->density_h) CU(launch_occupancy(v->density_h, R, v->occ_shift, v->occ_res, v->occ, g.sms, v->stream));
-    else CU(launch_occupancy(v->density, R, v->occ_shift, v->occ_res, v->occ, g.sms, v->stream));
-    CU(launch_occupancy_coarse(v->occ, v->occ_res, v->occ2, g.sms, v->stream));
-    {
-        const int init[6] = {R, R, R, -1, -1, -1};
-        CU(cudaMemcpyAsync(v->d_bounds, init, sizeof init, cudaMemcpyHostToDevice, v->stream));
-        if (v->density_h) CU(launch_nonzero_bounds(v->density_h, R, v->d_bounds, g.sms, v->stream));
-        else CU(launch_nonzero_bounds(v->density, R, v->d_bounds, g.sms, v->stream));
-        CU(cudaMemcpyAsync(v->nz_bounds, v->d_bounds, sizeof v->nz_bounds, cudaMemcpyDeviceToHost, v->stream));
-        CU(cudaStreamSynchronize(v->stream));
-        v->has_bounds = true;
-    }
+    // one pass over the grid: occupancy, nonzero bounds, majorant
+    int stats[7] = {R, R, R, -1, -1, -1, 0};
+    { float f0 = 0.00001f; std::memcpy(&stats[6], &f0, sizeof(int)); }
+    CU(cudaMemcpyAsync(v->d_stats, stats, sizeof stats, cudaMemcpyHostToDevice, v->stream));
+    const OccJob grid{nullptr, R, v->occ_rows, v->occ, v->occ2};
+    if (v->density_h) CU(launch_scan_grid(v->density_h, grid, v->d_stats, g.sms, v->stream));
+    else CU(launch_scan_grid(v->density, grid, v->d_stats, g.sms, v->stream));
+    CU(cudaMemcpyAsync(stats, v->d_stats, sizeof stats, cudaMemcpyDeviceToHost, v->stream));
+    CU(cudaStreamSynchronize(v->stream));
+    std::memcpy(v->nz_bounds, stats, sizeof v->nz_bounds);
+    v->has_bounds = true;
+    if (!v->max_override) std::memcpy(&v->max_density, &stats[6], sizeof(float));
     if (process_mips) {
         // core/volume.cu:1476-1514: halve to the largest power of two >= 256
         // below the input, then 9 levels 256 >> m, each from the previous one.
@@ -583,9 +571,13 @@ mrp_status mrp_volume_update(mrp_volume* v, int process_mips) {
             src = dst;
             src_res = r;
         }
-        for (int m = 0; m < kOccMips; ++m)
-            CU(launch_occupancy(v->mips + mip_offset(m), 256 >> m, 3, 32 >> m, v->mip_occ + mip_occ_offset(m), g.sms,
-                                v->stream));
+        OccJob level[kOccMips];
+        size_t row = 0;
+        for (int m = 0; m < kOccMips; ++m) {
+            level[m] = OccJob{v->mips + mip_offset(m), 256 >> m, v->occ_rows + row, v->mip_occ + mip_occ_offset(m), nullptr};
+            row += occ_row_words(256 >> m);
+        }
+        CU(launch_scan_levels(level, kOccMips, g.sms, v->stream));
         CU(launch_pad_levels(v->mips + mip_offset(5), v->mips + mip_offset(6), v->mips + mip_offset(7), false,
                              v->mips_pad, v->stream));
         CU(launch_pad_pyramid(v->mips, v->mips_tr, g.sms, v->stream));

@@ -110,13 +110,13 @@ struct mrp_volume {
     int occ_shift = 3, occ_res = 0;
     uint8_t* occ2 = nullptr;      // coarse occupancy (4^3 bricks each), built with occ
     int occ2_res = 0;
-    int* d_maxbits = nullptr;
+    uint4* occ_rows = nullptr;    // scratch of the occupancy scans
     float* mips_tr = nullptr;     // mips 1..8 with a border of zeros, built with the pyramid for the TR levels
     float* mips_pad = nullptr;    // padded mips 5..7 (pad_offset layout), built with the pyramid
     float* trs_pad = nullptr;     // padded TR levels 4..6, built with the TR levels
     float2* mip_tr = nullptr;     // (mip L, TR L - 1) texel pairs, L = 1..4, built with the TR levels
     float2* pad_pair = nullptr;   // (padded mip, padded TR) pairs, built with the TR levels
-    int* d_bounds = nullptr;      // nonzero-voxel index bounds (6 ints) of the last update
+    int* d_stats = nullptr;       // nonzero-voxel index bounds (6 ints) and majorant bits of the last update
     int nz_bounds[6] = {0, 0, 0, -1, -1, -1};
     bool has_bounds = false;
     bool has_data = false, has_pyramid = false, has_lut = false, has_tr = false, has_baked = false;

@@ -16,12 +16,27 @@ cudaError_t launch_narrow(const float* in, size_t n, __half* out, int sms, cudaS
 cudaError_t launch_widen(const __half* in, size_t n, float* out, int sms, cudaStream_t s);
 cudaError_t launch_resample(float* out, int res, const float* src, int src_res, int sms, cudaStream_t s);
 cudaError_t launch_resample(float* out, int res, const __half* src, int src_res, int sms, cudaStream_t s);
-cudaError_t launch_max_density(const float* d, size_t n, int* out_bits, int sms, cudaStream_t s);
-cudaError_t launch_max_density(const __half* d, size_t n, int* out_bits, int sms, cudaStream_t s);
-cudaError_t launch_occupancy(const float* d, int R, int shift, int nb, uint8_t* occ, int sms, cudaStream_t s);
-cudaError_t launch_occupancy(const __half* d, int R, int shift, int nb, uint8_t* occ, int sms, cudaStream_t s);
-// Coarse bricks (edge 4 bricks) of an occupancy grid of nb^3 bricks: (nb+3)/4 per axis.
-cudaError_t launch_occupancy_coarse(const uint8_t* occ, int nb, uint8_t* coarse, int sms, cudaStream_t s);
+// Occupancy of one grid of edge R (<= 2048): bricks of 8^3 voxels, and coarse
+// bricks of 4^3 bricks where coarse is not null ((bricks + 3) / 4 per axis).
+// rows: occ_row_words(R) words of scratch.
+struct OccJob {
+    const float* src;   // the grid (launch_scan_levels), unused by launch_scan_grid
+    int R;
+    uint4* rows;
+    uint8_t* occ;
+    uint8_t* coarse;
+};
+constexpr int kMaxOccJobs = kOccMips;
+inline size_t occ_row_words(int R) { return (size_t)R * R * ((R + 1023) / 1024); }
+constexpr size_t kMipOccRows = 65536 + 16384 + 4096 + 1024 + 256;   // occ_row_words of mips 0..kOccMips-1
+// One pass over a density grid: its occupancy, the index bounds of its
+// nonzero voxels stats[0..5] = {min x, y, z, max x, y, z} (must start at
+// {R, R, R, -1, -1, -1}) and the bits of its majorant stats[6] (must start at
+// 1e-5's).
+cudaError_t launch_scan_grid(const float* d, const OccJob& job, int* stats, int sms, cudaStream_t s);
+cudaError_t launch_scan_grid(const __half* d, const OccJob& job, int* stats, int sms, cudaStream_t s);
+// Occupancy of several fp32 levels at once (count <= kMaxOccJobs).
+cudaError_t launch_scan_levels(const OccJob* jobs, int count, int sms, cudaStream_t s);
 // VolumeDev::pad_pair from the padded mips and TR levels (kPadLevelFloats pairs).
 cudaError_t launch_pair_padded(const float* mips_pad, const float* trs_pad, float2* out, cudaStream_t s);
 // VolumeDev::mip_tr from the pyramid and the TR levels (mip_tr_offset(5) pairs).
@@ -30,10 +45,6 @@ cudaError_t launch_interleave_mip_tr(const float* mips, const float* trs, float2
 // of edge 8, 4, 2; clamp: TR-level addressing, else border (density mips).
 cudaError_t launch_pad_levels(const float* l8, const float* l4, const float* l2, bool clamp, float* out,
                               cudaStream_t s);
-// Index bounds of the nonzero voxels: out6 = {min x, min y, min z, max x,
-// max y, max z}, which must start at {R, R, R, -1, -1, -1}.
-cudaError_t launch_nonzero_bounds(const float* d, int R, int* out6, int sms, cudaStream_t s);
-cudaError_t launch_nonzero_bounds(const __half* d, int R, int* out6, int sms, cudaStream_t s);
 // Copies of mips 1..8 with a border of zeros (kTrPadFloats floats), which the
 // TR levels are marched through.
 cudaError_t launch_pad_pyramid(const float* mips, float* mips_tr, int sms, cudaStream_t s);

@@ -8,6 +8,7 @@
 // texture + surface references (core/volume.cu:1322-1400, 1535-1696).  Here
 // every resource is a plain z-fastest fp32 array in HBM produced by one
 // kernel launch per level, on the volume's stream.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -88,37 +89,50 @@ MRP_D float cpu_fetch(const T* __restrict__ d, int res, int x, int y, int z) {
     if (x < 0 || y < 0 || z < 0 || x >= res || y >= res || z >= res) return 0.0f;
     return fmaxf(0.0f, ldg_f(d + ((size_t)x * res + y) * res + z));
 }
+// res = 1 << lg (256 >> m, or 512 and 1024 on the way down to 256): one
+// thread per texel, k fastest.  The source coordinate of an index is the same
+// for all three axes, so a block works the (double) coordinates of the res
+// indices out once; per texel that leaves the eight loads and the lerps.
+// DRAM bound where the source is the grid: 512^3 -> 256^3 takes 95 us (5.7 TB/s), and all nine
+// levels 133 us against 281 with the coordinates worked out per texel.
+constexpr int kResampleThreads = 256, kResampleMax = 1024;
 template <class T>
-__global__ void k_resample(float* __restrict__ out, int res, const T* __restrict__ src, int src_res) {
-    size_t n = (size_t)res * res * res;
-    float sr = (float)src_res;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        int k = (int)(i % res), j = (int)((i / res) % res), q = (int)(i / ((size_t)res * res));
-        float u = (float)(((double)q + 0.5) / res), v = (float)(((double)j + 0.5) / res),
-              w = (float)(((double)k + 0.5) / res);
-        float px = fs(fm(u, sr), 0.5f), py = fs(fm(v, sr), 0.5f), pz = fs(fm(w, sr), 0.5f);
-        int x = (int)floorf(px), y = (int)floorf(py), z = (int)floorf(pz);
-        float wx = fs(px, (float)x), wy = fs(py, (float)y), wz = fs(pz, (float)z);
-        float a = lerp(lerp(cpu_fetch(src, src_res, x, y, z), cpu_fetch(src, src_res, x, y, z + 1), wz),
-                       lerp(cpu_fetch(src, src_res, x, y + 1, z), cpu_fetch(src, src_res, x, y + 1, z + 1), wz), wy);
-        float b = lerp(lerp(cpu_fetch(src, src_res, x + 1, y, z), cpu_fetch(src, src_res, x + 1, y, z + 1), wz),
-                       lerp(cpu_fetch(src, src_res, x + 1, y + 1, z), cpu_fetch(src, src_res, x + 1, y + 1, z + 1), wz), wy);
+__global__ void __launch_bounds__(kResampleThreads) k_resample(float* __restrict__ out, int lg, const T* __restrict__ src,
+                                                               int src_res) {
+    __shared__ int at[kResampleMax];
+    __shared__ float wt[kResampleMax];
+    const int res = 1 << lg;
+    const float sr = (float)src_res;
+    for (int q = threadIdx.x; q < res; q += kResampleThreads) {
+        const float u = (float)(((double)q + 0.5) / res);
+        const float px = fs(fm(u, sr), 0.5f);
+        const int x = (int)floorf(px);
+        at[q] = x;
+        wt[q] = fs(px, (float)x);
+    }
+    __syncthreads();
+    const int n = 1 << (3 * lg);
+    const size_t sx = (size_t)src_res * src_res, sy = src_res;
+    for (int i = blockIdx.x * kResampleThreads + threadIdx.x; i < n; i += gridDim.x * kResampleThreads) {
+        const int k = i & (res - 1), j = (i >> lg) & (res - 1), q = i >> (2 * lg);
+        const int x = at[q], y = at[j], z = at[k];
+        const float wx = wt[q], wy = wt[j], wz = wt[k];
+        float t[8];
+        if ((unsigned)x < (unsigned)(src_res - 1) && (unsigned)y < (unsigned)(src_res - 1) &&
+            (unsigned)z < (unsigned)(src_res - 1)) {
+            const T* p = src + x * sx + y * sy + z;
+            t[0] = ldg_f(p); t[1] = ldg_f(p + 1); t[2] = ldg_f(p + sy); t[3] = ldg_f(p + sy + 1);
+            t[4] = ldg_f(p + sx); t[5] = ldg_f(p + sx + 1); t[6] = ldg_f(p + sx + sy); t[7] = ldg_f(p + sx + sy + 1);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) t[c] = fmaxf(0.0f, t[c]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) t[c] = cpu_fetch(src, src_res, x + (c >> 2), y + ((c >> 1) & 1), z + (c & 1));
+        }
+        const float a = lerp(lerp(t[0], t[1], wz), lerp(t[2], t[3], wz), wy);
+        const float b = lerp(lerp(t[4], t[5], wz), lerp(t[6], t[7], wz), wy);
         out[i] = lerp(a, b, wx);
     }
-}
-
-// ---------------------------------------------------------------------------
-// max density (the delta-tracking majorant), floored at the reference's
-// default 1e-5 (core/volume.hpp:104).  Densities are compared as int bits,
-// which orders non-negative floats; negative (SDF) values never win.
-// ---------------------------------------------------------------------------
-template <class T>
-__global__ void k_max_density(const T* __restrict__ d, size_t n, int* __restrict__ out_bits) {
-    float m = 0.00001f;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        m = fmaxf(m, ldg_f(d + i));
-    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out_bits, __float_as_int(m));
 }
 
 // Mip level L and TR level L - 1 side by side per texel, L = 1..4
@@ -162,82 +176,146 @@ __global__ void k_pad_levels(const float* __restrict__ l8, const float* __restri
     }
 }
 
-// One warp per grid row (x, y): the lanes scan z, the warp keeps the bounds
-// of the nonzero voxels it saw and adds them with six atomics at the end.
-template <class T>
-__global__ void k_nonzero_bounds(const T* __restrict__ d, int R, int* __restrict__ out6) {
-    const int lane = threadIdx.x & 31;
-    const long long warps = (long long)gridDim.x * (blockDim.x / 32);
-    int lo[3] = {R, R, R}, hi[3] = {-1, -1, -1};
-    for (long long row = blockIdx.x * (long long)(blockDim.x / 32) + threadIdx.x / 32; row < (long long)R * R;
-         row += warps) {
-        const T* p = d + row * R;
-        int zlo = R, zhi = -1;
-        for (int z = lane; z < R; z += 32)
-            if (ldg_f(p + z) != 0.0f) { zlo = min(zlo, z); zhi = max(zhi, z); }
-        zlo = __reduce_min_sync(0xffffffffu, zlo);
-        zhi = __reduce_max_sync(0xffffffffu, zhi);
-        if (zhi >= 0) {
-            const int x = (int)(row / R), y = (int)(row % R);
-            lo[0] = min(lo[0], x); hi[0] = max(hi[0], x);
-            lo[1] = min(lo[1], y); hi[1] = max(hi[1], y);
-            lo[2] = min(lo[2], zlo); hi[2] = max(hi[2], zhi);
-        }
-    }
-    if (lane == 0 && hi[0] >= 0) {
-        for (int a = 0; a < 3; ++a) {
-            atomicMin(out6 + a, lo[a]);
-            atomicMax(out6 + 3 + a, hi[a]);
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
+// One pass over a grid for everything Update derives from single voxels: the
+// majorant, the bounds of the nonzero voxels, and per row (x, y) which bricks
+// along z the row's nonzero voxels occupy.
+//
+// Majorant: max density floored at the reference's default 1e-5
+// (core/volume.hpp:104).  Densities are compared as int bits, which orders
+// non-negative floats; negative (SDF) values never win.
+//
 // Occupancy bricks for exact empty-space skipping in the first-hit march.
-// Brick b covers voxels [b*B, b*B + B) per axis.  A trilinear fetch whose
-// base voxel lies in brick b reads voxels base..base+1, i.e. at most one
-// voxel past the brick; the brick is marked occupied when any voxel in
-// [b*B - 1, b*B + B + 1] holds a non-zero value, one voxel more on each
-// side than the fetch needs, so that a base voxel found from a coordinate
-// that may be off by less than one voxel still picks a brick whose apron
-// holds the whole footprint.  A zero brick therefore guarantees Density() ==
-// 0 exactly for every sample whose base voxel is in it or within one voxel
-// of it (border texels are 0 by addressing).
+// Brick b covers voxels [8b, 8b + 8) per axis.  A trilinear fetch whose base
+// voxel lies in brick b reads voxels base..base+1, i.e. at most one voxel
+// past the brick; the brick is marked occupied when any voxel in
+// [8b - 1, 8b + 9] holds a non-zero value, one voxel more on each side than
+// the fetch needs, so that a base voxel found from a coordinate that may be
+// off by less than one voxel still picks a brick whose apron holds the whole
+// footprint.  A zero brick therefore guarantees Density() == 0 exactly for
+// every sample whose base voxel is in it or within one voxel of it (border
+// texels are 0 by addressing).
+//
+// DRAM bound: each voxel is read once (k_scan_rows), then the rows' masks,
+// a 32nd of the grid at most, are combined over 11 x 11 rows per brick column
+// (k_occ_bricks).  512^3 fp32 and the five mips: 160 us (the grid alone
+// 118 us, 4.6 TB/s) against 1.94 ms when the majorant, the bounds and each
+// brick's 11^3 voxels were read by kernels of their own.
 // ---------------------------------------------------------------------------
+constexpr int kScanThreads = 256, kScanBlocks = 6;   // resident blocks per SM: one wave
+constexpr int kSegVoxels = 1024;   // voxels of a row that a warp masks at a time
+struct ScanJobs {
+    OccJob job[kMaxOccJobs];
+};
+// One warp per row; lane l keeps the 32-bit mask of voxels 32 l .. 32 l + 31
+// of each segment, widens it by the aprons' voxels, and the warp leaves four
+// words per segment: bit l of word b is brick 4 l + b of the segment.
+// stats (or null): the bounds {min x, y, z, max x, y, z}, then the majorant's bits.
 template <class T>
-__global__ void k_occupancy(const T* __restrict__ d, int R, int shift, int nb, uint8_t* __restrict__ occ) {
-    int total = nb * nb * nb;
-    for (int b = blockIdx.x; b < total; b += gridDim.x) {
-        int bz = b % nb, by = (b / nb) % nb, bx = b / (nb * nb);
-        int B = 1 << shift;
-        int x0 = bx * B - 1, y0 = by * B - 1, z0 = bz * B - 1;
-        int span = B + 3;
-        int any = 0;
-        for (int t = threadIdx.x; t < span * span * span && !any; t += blockDim.x) {
-            int z = z0 + t % span, y = y0 + (t / span) % span, x = x0 + t / (span * span);
-            if ((unsigned)x < (unsigned)R && (unsigned)y < (unsigned)R && (unsigned)z < (unsigned)R)
-                any |= ldg_f(d + ((size_t)x * R + y) * R + z) != 0.0f;
+__global__ void __launch_bounds__(kScanThreads, kScanBlocks) k_scan_rows(const T* __restrict__ only, ScanJobs jobs,
+                                                            int* __restrict__ stats) {
+    const OccJob J = jobs.job[blockIdx.y];
+    const T* __restrict__ d = only ? only : reinterpret_cast<const T*>(J.src);
+    const int R = J.R, lane = threadIdx.x & 31;
+    const int warps = gridDim.x * (kScanThreads / 32);
+    const int segs = (R + kSegVoxels - 1) / kSegVoxels;   // 1 or 2 (R <= 2048)
+    int lo[3] = {R, R, R}, hi[3] = {-1, -1, -1};
+    float top = 0.00001f;
+    for (int row = blockIdx.x * (kScanThreads / 32) + threadIdx.x / 32; row < R * R; row += warps) {
+        const T* p = d + (size_t)row * R;
+        uint32_t m[2] = {0u, 0u};
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            if (s >= segs) break;
+            const int nw = min((R - s * kSegVoxels + 31) / 32, 32);
+            for (int c0 = 0; c0 < nw; c0 += 16) {   // sixteen loads in flight per lane
+                float v[16];
+#pragma unroll
+                for (int c = 0; c < 16; ++c) {
+                    const int z = s * kSegVoxels + 32 * (c0 + c) + lane;
+                    v[c] = z < R ? ldg_f(p + z) : 0.0f;
+                }
+#pragma unroll
+                for (int c = 0; c < 16; ++c) {
+                    top = fmaxf(top, v[c]);
+                    const uint32_t b = __ballot_sync(0xffffffffu, v[c] != 0.0f);
+                    if (lane == c0 + c) m[s] = b;
+                }
+            }
         }
-        any = __syncthreads_or(any);
-        if (threadIdx.x == 0) occ[b] = any ? 1 : 0;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            if (s >= segs) break;
+            uint32_t up = __shfl_up_sync(0xffffffffu, m[s], 1), dn = __shfl_down_sync(0xffffffffu, m[s], 1);
+            const uint32_t last0 = __shfl_sync(0xffffffffu, m[0], 31), first1 = __shfl_sync(0xffffffffu, m[1], 0);
+            if (lane == 0) up = s ? last0 : 0u;
+            if (lane == 31) dn = s ? 0u : first1;
+            const uint32_t w = m[s] | (m[s] << 1) | (up >> 31) | (m[s] >> 1) | (dn << 31) | (m[s] >> 2) | (dn << 30);
+            uint4 o;
+            o.x = __ballot_sync(0xffffffffu, (w & 0x000000ffu) != 0u);
+            o.y = __ballot_sync(0xffffffffu, (w & 0x0000ff00u) != 0u);
+            o.z = __ballot_sync(0xffffffffu, (w & 0x00ff0000u) != 0u);
+            o.w = __ballot_sync(0xffffffffu, (w & 0xff000000u) != 0u);
+            if (lane == 0) J.rows[row * segs + s] = o;
+            const uint32_t any = __ballot_sync(0xffffffffu, m[s] != 0u);
+            if (stats && any) {
+                const int f = __ffs(any) - 1, l = 31 - __clz(any);
+                const uint32_t mf = __shfl_sync(0xffffffffu, m[s], f), ml = __shfl_sync(0xffffffffu, m[s], l);
+                const int x = row / R, y = row % R, z0 = s * kSegVoxels;
+                lo[0] = min(lo[0], x); hi[0] = max(hi[0], x);
+                lo[1] = min(lo[1], y); hi[1] = max(hi[1], y);
+                lo[2] = min(lo[2], z0 + 32 * f + __ffs(mf) - 1); hi[2] = max(hi[2], z0 + 32 * l + 31 - __clz(ml));
+            }
+        }
+    }
+    if (!stats) return;
+    for (int o = 16; o; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if (lane == 0) {
+        atomicMax(stats + 6, __float_as_int(top));
+        if (hi[0] >= 0)
+            for (int a = 0; a < 3; ++a) {
+                atomicMin(stats + a, lo[a]);
+                atomicMax(stats + 3 + a, hi[a]);
+            }
     }
 }
-
-// Coarse bricks of 4^3 occupancy bricks (edge 4B): coarse brick C is empty
-// when the 64 bricks 4C..4C+3 per axis are.  Their aprons together cover
-// voxels [4CB - 1, 4CB + 4B + 1], the coarse brick's own apron, so a zero
-// coarse brick carries the same guarantee as a zero brick, over its span.
-__global__ void k_occupancy_coarse(const uint8_t* __restrict__ occ, int nb, int nc, uint8_t* __restrict__ out) {
-    const int total = nc * nc * nc;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < total; c += gridDim.x * blockDim.x) {
-        const int cz = c % nc, cy = (c / nc) % nc, cx = c / (nc * nc);
-        int any = 0;
-        for (int k = 0; k < 64 && !any; ++k) {
-            const int x = 4 * cx + k / 16, y = 4 * cy + (k / 4) % 4, z = 4 * cz + k % 4;
-            if (x < nb && y < nb && z < nb) any = occ[(x * nb + y) * nb + z];
+// One block per 4 x 4 brick columns, one column a warp: the column's bricks
+// from the masks of its 11 x 11 rows, and of the block's sixteen columns the
+// coarse bricks (4^3 bricks each: coarse brick C is empty when the 64 bricks
+// 4C..4C+3 per axis are; their aprons together are the coarse brick's own
+// apron, so a zero coarse brick carries the same guarantee over its span).
+__global__ void __launch_bounds__(512) k_occ_bricks(ScanJobs jobs) {
+    const OccJob J = jobs.job[blockIdx.y];
+    const int R = J.R, nb = (R + 7) >> 3, nc = (nb + 3) >> 2, segs = (R + kSegVoxels - 1) / kSegVoxels;
+    if ((int)blockIdx.x >= nc * nc) return;
+    __shared__ uint32_t coarse[64];
+    if (threadIdx.x < 64) coarse[threadIdx.x] = 0u;
+    __syncthreads();
+    const int cx = blockIdx.x / nc, cy = blockIdx.x % nc, warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+    const int bx = 4 * cx + warp / 4, by = 4 * cy + warp % 4;
+    if (bx < nb && by < nb) {
+        for (int s = 0; s < segs; ++s) {
+            uint4 o = make_uint4(0u, 0u, 0u, 0u);
+            for (int t = lane; t < 121; t += 32) {
+                const int x = 8 * bx - 1 + t / 11, y = 8 * by - 1 + t % 11;
+                if ((unsigned)x < (unsigned)R && (unsigned)y < (unsigned)R) {
+                    const uint4 r = J.rows[(x * R + y) * segs + s];
+                    o.x |= r.x; o.y |= r.y; o.z |= r.z; o.w |= r.w;
+                }
+            }
+            o.x = __reduce_or_sync(0xffffffffu, o.x); o.y = __reduce_or_sync(0xffffffffu, o.y);
+            o.z = __reduce_or_sync(0xffffffffu, o.z); o.w = __reduce_or_sync(0xffffffffu, o.w);
+            const uint32_t b[4] = {(o.x >> lane) & 1u, (o.y >> lane) & 1u, (o.z >> lane) & 1u, (o.w >> lane) & 1u};
+            const int bz = s * (kSegVoxels / 8) + 4 * lane;
+            uint8_t* dst = J.occ + (bx * nb + by) * nb;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (bz + q < nb) dst[bz + q] = (uint8_t)b[q];
+            if (b[0] | b[1] | b[2] | b[3]) coarse[s * 32 + lane] = 1u;
         }
-        out[c] = any ? 1 : 0;
     }
+    __syncthreads();
+    if (J.coarse && (int)threadIdx.x < nc) J.coarse[(cx * nc + cy) * nc + threadIdx.x] = (uint8_t)coarse[threadIdx.x];
 }
 
 // ---------------------------------------------------------------------------
@@ -662,21 +740,19 @@ cudaError_t launch_widen(const __half* in, size_t n, float* out, int sms, cudaSt
     k_widen<<<grid_for(n, 256, sms), 256, 0, s>>>(in, n, out);
     return cudaGetLastError();
 }
-cudaError_t launch_resample(float* out, int res, const float* src, int src_res, int sms, cudaStream_t s) {
-    k_resample<float><<<grid_for((size_t)res * res * res, 256, sms), 256, 0, s>>>(out, res, src, src_res);
+template <class T>
+static cudaError_t resample_t(float* out, int res, const T* src, int src_res, int sms, cudaStream_t s) {
+    int lg = 0;
+    while ((1 << lg) < res) ++lg;
+    if ((1 << lg) != res || res > kResampleMax) return cudaErrorInvalidValue;
+    k_resample<T><<<grid_for((size_t)res * res * res, kResampleThreads, sms), kResampleThreads, 0, s>>>(out, lg, src, src_res);
     return cudaGetLastError();
+}
+cudaError_t launch_resample(float* out, int res, const float* src, int src_res, int sms, cudaStream_t s) {
+    return resample_t(out, res, src, src_res, sms, s);
 }
 cudaError_t launch_resample(float* out, int res, const __half* src, int src_res, int sms, cudaStream_t s) {
-    k_resample<__half><<<grid_for((size_t)res * res * res, 256, sms), 256, 0, s>>>(out, res, src, src_res);
-    return cudaGetLastError();
-}
-cudaError_t launch_max_density(const float* d, size_t n, int* out_bits, int sms, cudaStream_t s) {
-    k_max_density<float><<<grid_for(n, 256, sms), 256, 0, s>>>(d, n, out_bits);
-    return cudaGetLastError();
-}
-cudaError_t launch_max_density(const __half* d, size_t n, int* out_bits, int sms, cudaStream_t s) {
-    k_max_density<__half><<<grid_for(n, 256, sms), 256, 0, s>>>(d, n, out_bits);
-    return cudaGetLastError();
+    return resample_t(out, res, src, src_res, sms, s);
 }
 cudaError_t launch_interleave_mip_tr(const float* mips, const float* trs, float2* out, int sms, cudaStream_t s) {
     k_interleave_mip_tr<<<sms * 8, 256, 0, s>>>(mips, trs, out);
@@ -691,34 +767,37 @@ cudaError_t launch_pad_levels(const float* l8, const float* l4, const float* l2,
     k_pad_levels<<<dim3(1, 3), 256, 0, s>>>(l8, l4, l2, clamp ? 1 : 0, out);
     return cudaGetLastError();
 }
-template <class T>
-static cudaError_t nonzero_bounds_t(const T* d, int R, int* out6, int sms, cudaStream_t s) {
-    long long rows = (long long)R * R;
-    int blocks = (int)((rows + 7) / 8 < sms * 16 ? (rows + 7) / 8 : sms * 16);
-    k_nonzero_bounds<T><<<blocks, 256, 0, s>>>(d, R, out6);
-    return cudaGetLastError();
-}
-cudaError_t launch_nonzero_bounds(const float* d, int R, int* out6, int sms, cudaStream_t s) {
-    return nonzero_bounds_t(d, R, out6, sms, s);
-}
-cudaError_t launch_nonzero_bounds(const __half* d, int R, int* out6, int sms, cudaStream_t s) {
-    return nonzero_bounds_t(d, R, out6, sms, s);
+static unsigned coarse_columns(int R) {   // blocks of k_occ_bricks
+    const unsigned nc = (unsigned)(((R + 7) >> 3) + 3) >> 2;
+    return nc * nc;
 }
 template <class T>
-static cudaError_t occupancy_t(const T* d, int R, int shift, int nb, uint8_t* occ, int sms, cudaStream_t s) {
-    int total = nb * nb * nb;
-    k_occupancy<T><<<total < sms * 16 ? total : sms * 16, 256, 0, s>>>(d, R, shift, nb, occ);
+static cudaError_t scan_grid_t(const T* d, const OccJob& job, int* stats, int sms, cudaStream_t s) {
+    ScanJobs J{};
+    J.job[0] = job;
+    const int rows = job.R * job.R, need = (rows + kScanThreads / 32 - 1) / (kScanThreads / 32);
+    k_scan_rows<T><<<std::min(need, sms * kScanBlocks), kScanThreads, 0, s>>>(d, J, stats);
+    k_occ_bricks<<<coarse_columns(job.R), 512, 0, s>>>(J);
     return cudaGetLastError();
 }
-cudaError_t launch_occupancy(const float* d, int R, int shift, int nb, uint8_t* occ, int sms, cudaStream_t s) {
-    return occupancy_t(d, R, shift, nb, occ, sms, s);
+cudaError_t launch_scan_grid(const float* d, const OccJob& job, int* stats, int sms, cudaStream_t s) {
+    return scan_grid_t(d, job, stats, sms, s);
 }
-cudaError_t launch_occupancy(const __half* d, int R, int shift, int nb, uint8_t* occ, int sms, cudaStream_t s) {
-    return occupancy_t(d, R, shift, nb, occ, sms, s);
+cudaError_t launch_scan_grid(const __half* d, const OccJob& job, int* stats, int sms, cudaStream_t s) {
+    return scan_grid_t(d, job, stats, sms, s);
 }
-cudaError_t launch_occupancy_coarse(const uint8_t* occ, int nb, uint8_t* coarse, int sms, cudaStream_t s) {
-    const int nc = (nb + 3) / 4, total = nc * nc * nc;
-    k_occupancy_coarse<<<grid_for((size_t)total, 128, sms), 128, 0, s>>>(occ, nb, nc, coarse);
+cudaError_t launch_scan_levels(const OccJob* job, int count, int sms, cudaStream_t s) {
+    if (count < 1 || count > kMaxOccJobs) return cudaErrorInvalidValue;
+    ScanJobs J{};
+    int need = 0;
+    unsigned columns = 0;
+    for (int i = 0; i < count; ++i) {
+        J.job[i] = job[i];
+        need = std::max(need, (job[i].R * job[i].R + kScanThreads / 32 - 1) / (kScanThreads / 32));
+        columns = std::max(columns, coarse_columns(job[i].R));
+    }
+    k_scan_rows<float><<<dim3(std::min(need, sms * kScanBlocks), count), kScanThreads, 0, s>>>(nullptr, J, nullptr);
+    k_occ_bricks<<<dim3(columns, count), 512, 0, s>>>(J);
     return cudaGetLastError();
 }
 cudaError_t launch_pad_pyramid(const float* mips, float* mips_tr, int sms, cudaStream_t s) {

@@ -86,3 +86,54 @@ def test_tr_levels(light, R, lo, hi):
     got = np.concatenate([v.read(M.api.RES_TR, m) for m in range(8)])
     ref = O.tr_mips(mips, 48.0, np.array(light, np.float32))
     np.testing.assert_allclose(got, ref, rtol=2e-6, atol=1e-7)
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16"])
+@pytest.mark.parametrize("R", [2, 7, 8, 9, 31, 33, 64, 70, 129, 1030])
+def test_scan(R, storage):
+    """Occupancy bricks and majorant at grid edges around the bricks' and the
+    row masks' sizes (8, 32 and 1024 voxels), from voxels at corners, at brick
+    and mask borders and inside: a brick is set exactly when a nonzero voxel
+    lies in [8 b - 1, 8 b + 9] per axis; a negative voxel and a NaN count as
+    nonzero and never as the majorant."""
+    import torch
+
+    import mrpnn_b200 as M
+    M.init()
+    if R > 1024 and storage == "fp32":
+        pytest.skip("one storage type is enough for the long rows")
+    rng = np.random.default_rng(R)
+    at = {(0, 0, 0), (R - 1, R - 1, R - 1), (R // 2, 0, R - 1), (min(7, R - 1), min(8, R - 1), min(9, R - 1)),
+          (0, R - 1, min(31, R - 1)), (0, R // 3, min(32, R - 1)), (R - 1, R // 3, min(1023, R - 1)),
+          (R // 3, 1, min(1024, R - 1))} | {tuple(rng.integers(0, R, 3)) for _ in range(6)}
+    d = torch.zeros((R, R, R), device="cuda")
+    vals = [-0.5, float("nan")] + [0.25 + 0.125 * k for k in range(len(at))]
+    nb = (R + 7) // 8
+    want = np.zeros((nb, nb, nb), np.uint8)
+    top = 1e-5
+    for (x, y, z), val in zip(sorted(at), vals):
+        d[x, y, z] = val
+        top = max(top, val) if val == val else top
+        r = [[b for b in range(nb) if 8 * b - 1 <= c <= 8 * b + 9] for c in (x, y, z)]
+        want[np.ix_(*r)] = 1
+    v = M.VolumeRender(R, storage=storage)
+    torch.cuda.synchronize()
+    v.set_data(d)
+    v.Update(process_mips=R <= 129)
+    np.testing.assert_array_equal(v.read(M.api.RES_OCCUPANCY).reshape(nb, nb, nb), want)
+    assert v.max_density == np.float32(top)
+
+
+@pytest.mark.parametrize("R", [2, 3, 100, 255, 257, 300])
+def test_pyramid_levels(R):
+    """The pyramid of grids below, at and above 256 and of two voxels,
+    negative voxels among them: bit-exact against the oracle."""
+    import mrpnn_b200 as M
+    M.init()
+    data = np.random.default_rng(R).uniform(-0.2, 1.0, R ** 3).astype(np.float32)
+    v = M.VolumeRender(R)
+    v.set_data(data)
+    v.Update()
+    ref = O.split_levels(O.build_pyramid(data, R), O.mip_sizes())
+    for m in range(9):
+        np.testing.assert_array_equal(v.read(M.api.RES_MIP, m), ref[m].ravel(), err_msg=f"mip {m}")
