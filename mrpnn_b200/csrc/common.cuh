@@ -618,6 +618,15 @@ MRP_D void flush_tally(unsigned long long* c, const Tally& t) {
     atomicAdd(c + 3, (unsigned long long)t.events);
 }
 
+// The running mean of a pixel over launches (RenderCamera, core/volume.cu:224-227).
+MRP_D void running_mean(float4* accum, int pix, int mean_k, float4 res) {
+    res.x = fmaxf(0.0f, res.x); res.y = fmaxf(0.0f, res.y); res.z = fmaxf(0.0f, res.z); res.w = fmaxf(0.0f, res.w);
+    // result = lerp(result, res, 1/(1+frameNum)) (core/volume.cu:226-227)
+    float rate = fd(1.0f, (float)(1 + mean_k));
+    float4 a = mean_k == 0 ? make_float4(0, 0, 0, 0) : accum[pix];
+    accum[pix] = make_float4(lerp(a.x, res.x, rate), lerp(a.y, res.y, rate), lerp(a.z, res.z, rate), lerp(a.w, res.w, rate));
+}
+
 // ---------------------------------------------------------------------------
 // Packed MLP weight layout (fp32, one buffer).  Per SE block: the gate MLP
 // 8->8 (no bias) and 8->3 (no bias), then the three branch layers w->w with
@@ -645,13 +654,4 @@ constexpr int lxb(int k) { return kLXk + k * 272 + 256; }
 constexpr int kLX12W = kLXk + 12 * 272, kLX12B = kLX12W + 16;
 constexpr int kWeightCount = kLX12B + 1;
 static_assert(kWeightCount == 49673, "packed weight count must match core/NNWeight.cuh");
-// The device copy appends two transposed copies for the FP32 network:
-// LC1W as [128][64] and LSEFin1W as [75][16] (16-byte aligned rows).
-constexpr int kLC1T = (kWeightCount + 3) / 4 * 4;
-constexpr int kFin1T = kLC1T + 8192;
-constexpr int kWeightCountDev = kFin1T + 1200;
-static_assert(kLC1T % 4 == 0 && kFin1T % 4 == 0 && kLC0W % 4 == 0 && kLC2W % 4 == 0 && kLXW % 4 == 0 &&
-                  kMainFinalOff % 4 == 0 && kDiOff % 4 == 0 && kLXk % 4 == 0,
-              "rows read as float4 start on 16-byte boundaries");
-
 }  // namespace mrp

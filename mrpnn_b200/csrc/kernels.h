@@ -76,6 +76,10 @@ cudaError_t launch_lut_dirs(const float* lut, float* out, cudaStream_t s);
 // features: [n][576] (X_Val, X_Val_Sub, X_Val_Hg), gamma [n]
 cudaError_t launch_gather(const VolumeDev& v, const float* pos, const float* bases, const float* light, float g,
                           float alpha, int n, float* feat, float* gamma, cudaStream_t s);
+// mlp_fp32.cu: the FP32 network's device weights (fp32_weight_floats()) and
+// constants from the packed ones (host, common.cuh)
+size_t fp32_weight_floats();
+cudaError_t fp32_prepare_weights(const float* packed, float* d_out);
 cudaError_t launch_mlp_fp32(const float* weights, const float* feat, const float* gamma, float g, const float sr[3],
                             int n, float* out3, cudaStream_t s);
 cudaError_t launch_first_hit(const VolumeDev& v, const float* ori, const float* dir, float alpha, float pass_rate, int n,
