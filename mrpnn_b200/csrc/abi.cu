@@ -283,23 +283,28 @@ mrp_status mrp_volume_create_ex(int res, mrp_storage storage, mrp_volume** out) 
     size_t n = (size_t)res * res * res;
     v->occ_res = (res + (1 << v->occ_shift) - 1) >> v->occ_shift;
     v->occ2_res = (v->occ_res + 3) / 4;
-    size_t nocc = (size_t)v->occ_res * v->occ_res * v->occ_res;
+    // the small buffers lie behind larger ones: an allocation and its free
+    // cost about half a millisecond each
+    const size_t nocc = (size_t)v->occ_res * v->occ_res * v->occ_res,
+                 nocc2 = (size_t)v->occ2_res * v->occ2_res * v->occ2_res,
+                 nrow = std::max(occ_row_words(res), kMipOccRows);
     if ((storage == MRP_STORAGE_FP16 ? (e = mrp::dev_malloc(&v->density_h, n * sizeof(__half)))
                                      : (e = mrp::dev_malloc(&v->density, n * sizeof(float)))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->mips, kMipFloats * sizeof(float))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->trs, kTrFloats * sizeof(float))) != cudaSuccess ||
+        (e = mrp::dev_malloc(&v->mips, (kMipFloats + kTrPadFloats + kPadLevelFloats) * sizeof(float))) != cudaSuccess ||
+        (e = mrp::dev_malloc(&v->trs, (kTrFloats + kPadLevelFloats) * sizeof(float))) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->lut, kLutAlloc * sizeof(float))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->occ, nocc)) != cudaSuccess || (e = mrp::dev_malloc(&v->mip_occ, kMipOccBytes)) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->occ2, (size_t)v->occ2_res * v->occ2_res * v->occ2_res)) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->d_stats, 7 * sizeof(int))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->occ_rows, std::max(occ_row_words(res), kMipOccRows) * sizeof(uint4))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->mips_tr, kTrPadFloats * sizeof(float))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->mips_pad, kPadLevelFloats * sizeof(float))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->trs_pad, kPadLevelFloats * sizeof(float))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->mip_tr, mip_tr_offset(5) * sizeof(float2))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->pad_pair, kPadLevelFloats * sizeof(float2))) != cudaSuccess)
+        (e = mrp::dev_malloc(&v->occ_rows, nrow * sizeof(uint4) + 32 + kMipOccBytes + nocc + nocc2)) != cudaSuccess ||
+        (e = mrp::dev_malloc(&v->mip_tr, (mip_tr_offset(5) + kPadLevelFloats) * sizeof(float2))) != cudaSuccess)
         return cleanup(fail(e == cudaErrorMemoryAllocation ? MRP_ERR_OOM : MRP_ERR_CUDA, "volume allocation: %s",
                             cudaGetErrorString(e)));
+    v->mips_tr = v->mips + kMipFloats;
+    v->mips_pad = v->mips_tr + kTrPadFloats;
+    v->trs_pad = v->trs + kTrFloats;
+    v->pad_pair = v->mip_tr + mip_tr_offset(5);
+    v->d_stats = reinterpret_cast<int*>(v->occ_rows + nrow);
+    v->mip_occ = reinterpret_cast<uint8_t*>(v->d_stats) + 32;
+    v->occ = v->mip_occ + kMipOccBytes;
+    v->occ2 = v->occ + nocc;
     if (v->density_h) cudaMemsetAsync(v->density_h, 0, n * sizeof(__half), v->stream);
     else cudaMemsetAsync(v->density, 0, n * sizeof(float), v->stream);
     *out = v;
@@ -315,7 +320,7 @@ mrp_status mrp_volume_destroy(mrp_volume* v) {
     if (v->stream_copy) cudaStreamSynchronize(v->stream_copy);
     mrp::dev_free(v->accum_alt);
     mrp::dev_free(v->density); mrp::dev_free(v->density_h); mrp::dev_free(v->mips); mrp::dev_free(v->trs); mrp::dev_free(v->lut); mrp::dev_free(v->baked);
-    mrp::dev_free(v->occ); mrp::dev_free(v->occ2); mrp::dev_free(v->mip_occ); mrp::dev_free(v->d_stats); mrp::dev_free(v->occ_rows); mrp::dev_free(v->mips_tr); mrp::dev_free(v->mips_pad); mrp::dev_free(v->trs_pad); mrp::dev_free(v->mip_tr); mrp::dev_free(v->pad_pair); mrp::dev_free(v->accum); mrp::dev_free(v->sum3); mrp::dev_free(v->first_pos);
+    mrp::dev_free(v->occ_rows); mrp::dev_free(v->mip_tr); mrp::dev_free(v->accum); mrp::dev_free(v->sum3); mrp::dev_free(v->first_pos);
     mrp::dev_free(v->counter);
     mrp::dev_free(v->hdri);
     drop_density_texture(v);
