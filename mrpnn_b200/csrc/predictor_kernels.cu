@@ -833,8 +833,8 @@ cudaError_t launch_hit(const VolumeDev& v, const ViewDev& view, HitRecords rec, 
 // ---------------------------------------------------------------------------
 // Tile gather of the tile network (GatherData -> GatherSamples ->
 // NNGatherSamples, core/volume.cu:257-282; core/render.cuh:199-397, 464-485,
-// 1006-1142; SetupInputData2, core/radiancePredict.cu:487-553): one thread
-// per 8 x 8-pixel tile, 773 floats: X_Val[192], X_Val_Hg[192], X_Val_Sub[192],
+// 1006-1142; SetupInputData2, core/radiancePredict.cu:487-553): per 8 x
+// 8-pixel tile 773 floats: X_Val[192], X_Val_Hg[192], X_Val_Sub[192],
 // 5 angle / depth-gradient terms, 192 t-grid values.  nl = {-log 0.76,
 // -log 0.75, -log 0.25} from the host's logf.
 // ---------------------------------------------------------------------------
@@ -879,7 +879,13 @@ MRP_D bool check_exit(float S, float lastS, float dt, float t, TauState& st, flo
     return false;
 }
 
-// DeterminateEstimatedHit(alpha, pos, dir, dis) -> float4 (core/render.cuh:298-397)
+// DeterminateEstimatedHit(alpha, pos, dir, dis) -> float4 (core/render.cuh:298-397).
+// A step that reads 0 (and no transition from density pending) only advances
+// t by half a voxel, so the march skips such steps exactly as the first-hit
+// march does (estimated_hit): up to the box of nonzero voxels, through empty
+// bricks, and past the box's far side, where it ends with what the t > dis
+// test gives.
+template <class DT>
 MRP_D void estimated_hit_ts(const VolumeDev& v, float alpha, f3 pos, f3 dir, float dis, const float nl[3],
                             float ts[4]) {
     float smax = fm(v.max_density, alpha);
@@ -889,16 +895,44 @@ MRP_D void estimated_hit_ts(const VolumeDev& v, float alpha, f3 pos, f3 dir, flo
     float rf = (float)v.res;
     float t_step = fd(1.0f, rf);
     if (fm(smax, t_step) > nl[0]) t_step = fd(nl[0], smax);
+    const float half = fd(0.5f, rf);
+    const bool pow2 = (v.res & (v.res - 1)) == 0;
+    const MarchRay mr = march_ray(v, pos, dir);
     TauState st{0.0f, nl[1], true};
     int loop = 0;
-    float last = 0.0f;
+    float last = 0.0f, t_exit = 3.0e38f;
+    if (v.has_bounds && v.occ) {
+        float t0 = 0.0f, t1 = dis;
+        const float o[3] = {pos.x, pos.y, pos.z}, dd[3] = {dir.x, dir.y, dir.z};
+        const float lo[3] = {v.nz_lo.x, v.nz_lo.y, v.nz_lo.z}, hi[3] = {v.nz_hi.x, v.nz_hi.y, v.nz_hi.z};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            if (dd[a] == 0.0f) {
+                if (o[a] < lo[a] || o[a] > hi[a]) t0 = 3.0e38f;
+            } else {
+                const float ta = (lo[a] - o[a]) / dd[a], tb = (hi[a] - o[a]) / dd[a];
+                t0 = fmaxf(t0, fminf(ta, tb));
+                t1 = fminf(t1, fmaxf(ta, tb));
+            }
+        }
+        const float t_enter = t0 > t1 ? 3.0e38f : t0;
+        t_exit = t0 > t1 ? 0.0f : t1;
+        if (pow2) replay_empty(t, loop, 2.0f * rf, half, dis, t_enter, 10000);
+        while (loop < 10000 && t <= dis && t < t_enter) {
+            ++loop;
+            t = fa(t, half);
+        }
+    }
     while (loop++ < 10000) {
-        if (t > dis) {
+        // past the box: only empty steps are left, and fewer than the
+        // bound allows (each advances t by half a voxel)
+        if (t > dis || (t > t_exit && !(last > 0.0f) && (float)(10000 - loop) > (dis - t) * (2.0f * rf) + 2.0f)) {
             if (st.first) ts[0] = last_non_empty_t;
             else ts[1] = last_non_empty_t;
             break;
         }
-        float d = density(v, add(pos, mul(dir, t)));
+        float t_brick = -1.0f;
+        const float d = v.occ ? density_skip<DT>(v, mr, t, nullptr, &t_brick) : density_as<DT>(v, add(pos, mul(dir, t)));
         if (d > 0) {
             float S = fm(d, alpha);
             if (check_exit(S, last, t_step, t, st, ts, nl[2])) break;
@@ -915,8 +949,13 @@ MRP_D void estimated_hit_ts(const VolumeDev& v, float alpha, f3 pos, f3 dir, flo
                     last_non_empty_t = t;
                 }
             }
-            t = fa(t, fmaxf(fm(-d, 1.0f), fd(0.5f, rf)));
+            t = fa(t, fmaxf(fm(-d, 1.0f), half));
             last = 0.0f;
+        }
+        if (pow2 && t_brick >= 0.0f) replay_empty(t, loop, 2.0f * rf, half, fminf(t_brick, dis), 3.0e38f, 10000);
+        while (t <= t_brick && t <= dis && loop < 10000) {
+            ++loop;
+            t = fa(t, half);
         }
     }
     if (ts[2] == FLT_MAX) ts[2] = 0.0f;
@@ -925,42 +964,15 @@ MRP_D void estimated_hit_ts(const VolumeDev& v, float alpha, f3 pos, f3 dir, flo
 }
 
 // GetSampleT (core/render.cuh:464-485)
+template <class DT>
 MRP_D void sample_t(const VolumeDev& v, f3 ori, f3 dir, float alpha, const float nl[3], float ts[4]) {
     float dis = ray_box_offset(ori, dir);
     if (dis < 0) { ts[0] = ts[1] = ts[2] = ts[3] = 0.0f; return; }
     f3 sp = add(ori, mul(dir, dis));
     float md = ray_box_distance(sp, dir);
-    estimated_hit_ts(v, alpha, sp, dir, md, nl, ts);
+    estimated_hit_ts<DT>(v, alpha, sp, dir, md, nl, ts);
     if (ts[0] > 0) { ts[0] = fa(ts[0], dis); ts[2] = fa(ts[2], dis); }
     if (ts[1] > 0) ts[1] = fa(ts[1], dis);
-}
-
-struct TileAcc {
-    float minx, miny, maxx, maxy;
-    f3 avg;
-};
-
-// PrepareRay (core/render.cuh:1006-1040)
-MRP_D void prepare_ray(const VolumeDev& v, float ox, float oy, f3 dir, f3 ro, f3 uo, f3 ori, float alpha,
-                       const float nl[3], bool p25, int gid, float* tg, TileAcc& acc, float& hd, float& vd,
-                       float ray[4]) {
-    f3 sd = normalize(add(add(dir, mul(ro, ox)), mul(uo, oy)));
-    float ts[4];
-    sample_t(v, ori, sd, alpha, nl, ts);
-    ray[0] = sd.x; ray[1] = sd.y; ray[2] = sd.z; ray[3] = p25 ? ts[1] : ts[0];
-    const float rn = fd(1.0f, 3.0f);
-    float min_t = fm(ts[2], rn), max_t = fm(fmaxf(ts[0], ts[1]), rn);
-    tg[gid] = fm(fa(min_t, max_t), 0.5f);
-    tg[gid + 1] = fs(max_t, min_t);
-    tg[gid / 2 + 128] = ts[3];
-    if (ray[3] != 0) {
-        acc.minx = fminf(acc.minx, ox); acc.miny = fminf(acc.miny, oy);
-        acc.maxx = fmaxf(acc.maxx, ox); acc.maxy = fmaxf(acc.maxy, oy);
-        acc.avg = add(acc.avg, ts[1] > 0 ? mul(sd, 2.0f) : sd);
-        float sum_t = fa(ts[0], ts[1]);
-        hd = fa(hd, sum_t);
-        vd = fa(vd, sum_t);
-    }
 }
 
 struct TileView {
@@ -971,10 +983,23 @@ struct TileView {
     float nl[3];
 };
 
-__global__ void __launch_bounds__(64) k_gather_tiles(VolumeDev v, TileView T, float* __restrict__ out) {
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= T.W * T.H) return;
-    int i = idx / T.W, j = idx % T.W;
+// One block of 64 threads per tile: a thread marches one of the tile's 64 rays
+// (PrepareRay, core/render.cuh:1006-1040: sample `sid`'s base ray and its
+// three neighbours), the sums over the rays run in the reference's order on
+// one thread per component, and the 192 stencil points are spread over the
+// block.  Bound by the marches (lanes of a warp end apart).  128 x 128 tiles
+// of a 256^3 cloud: 13.9 ms with one thread per tile, 0.64 ms.
+constexpr int kTileThreads = 64;
+template <class DT>
+__global__ void __launch_bounds__(kTileThreads) k_gather_tiles(const __grid_constant__ VolumeDev v,
+                                                               const __grid_constant__ TileView T,
+                                                               float* __restrict__ out) {
+    __shared__ float ray[64][4];      // direction, t of the ray's threshold (0: none)
+    __shared__ float ray_t[64][2];    // ts[0], ts[1]
+    __shared__ float samples[16][4], total[5];
+    __shared__ float box[2][4];       // per warp: min x, min y, max x, max y of the rays that hit
+    const int idx = blockIdx.x, tid = threadIdx.x;
+    const int i = idx / T.W, j = idx % T.W;
     float* ob = out + (size_t)idx * 773;
     float u = fs(1.0f, fd(fa(fa((float)j, fd((float)T.px, 8.0f)), 0.5f), (float)T.W));
     float w = fs(1.0f, fd(fa(fa((float)i, fd((float)T.py, 8.0f)), 0.5f), (float)T.H));
@@ -983,76 +1008,120 @@ __global__ void __launch_bounds__(64) k_gather_tiles(VolumeDev v, TileView T, fl
     const float rw = fm((float)T.W, 4.0f), rh = fm((float)T.H, 4.0f);
     f3 ro = mk3(fd(-T.right.x, rw), fd(-T.right.y, rw), fd(-T.right.z, rw));
     f3 uo = mk3(fd(-T.up.x, rh), fd(-T.up.y, rh), fd(-T.up.z, rh));
-    float samples[16][4];
-    TileAcc acc{FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, mk3(0, 0, 0)};
-    float hor = 0.0f, vert = 0.0f;
-    float* tg = ob + 192 * 3 + 5;
-    if (idx == 0) ob[0] = fm(ob[0], 1.00001f);
-    for (int y = -3, sid = 0, gid = 0, cb = 0; y <= 3; y += 2, cb = (cb + 1) & 1, gid += 16)
-        for (int x = -3; x <= 3; x += 2, sid++, gid += 4) {
-            bool p25 = ((sid + cb) & 1) != 0;
-            float h_ = 0.0f, v_ = 0.0f;
-            float r[4], c[4];
-            prepare_ray(v, (float)x - 0.5f, (float)y - 0.5f, dir, ro, uo, T.ori, T.alpha, T.nl, p25, gid, tg, acc, h_,
-                        v_, r);
-#pragma unroll 1
-            for (int q = 0; q < 3; ++q) {
-                float ox = q == 1 ? -0.5f : 0.5f, oy = q == 0 ? -0.5f : 0.5f;
-                int go = q == 0 ? 2 : q == 1 ? 16 : 18;
-                prepare_ray(v, (float)x + ox, (float)y + oy, dir, ro, uo, T.ori, T.alpha, T.nl, p25, gid + go, tg, acc,
-                            h_, v_, c);
-                if ((c[3] != 0 && ((c[3] < r[3]) != p25)) || r[3] == 0)
-                    for (int k = 0; k < 4; ++k) r[k] = c[k];
-            }
-            hor = fa(hor, x > 0 ? h_ : -h_);
-            vert = fa(vert, y > 0 ? v_ : -v_);
-            int fill = sid / 2 + (p25 ? 8 : 0);
-            for (int k = 0; k < 4; ++k) samples[fill][k] = r[k];
+    {
+        // sample sid at (x, y) in {-3, -1, 1, 3}^2, its ray q at (+-0.5, +-0.5)
+        // around it; t-grid place: 4 floats a sample, 16 more a row
+        const int sid = tid >> 2, q = tid & 3;
+        const int x = -3 + 2 * (sid & 3), y = -3 + 2 * (sid >> 2), cb = (sid >> 2) & 1;
+        const bool p25 = ((sid + cb) & 1) != 0;
+        const float ox = (float)x + (q & 1 ? 0.5f : -0.5f), oy = (float)y + (q & 2 ? 0.5f : -0.5f);
+        const int gid = 4 * sid + 16 * (sid >> 2) + (q & 1 ? 2 : 0) + (q & 2 ? 16 : 0);
+        const f3 sd = normalize(add(add(dir, mul(ro, ox)), mul(uo, oy)));
+        float ts[4];
+        sample_t<DT>(v, T.ori, sd, T.alpha, T.nl, ts);
+        const float rt = p25 ? ts[1] : ts[0];
+        ray[tid][0] = sd.x; ray[tid][1] = sd.y; ray[tid][2] = sd.z; ray[tid][3] = rt;
+        ray_t[tid][0] = ts[0]; ray_t[tid][1] = ts[1];
+        const float rn = fd(1.0f, 3.0f);
+        const float min_t = fm(ts[2], rn), max_t = fm(fmaxf(ts[0], ts[1]), rn);
+        float* tg = ob + 192 * 3 + 5;
+        tg[gid] = fm(fa(min_t, max_t), 0.5f);
+        tg[gid + 1] = fs(max_t, min_t);
+        tg[gid / 2 + 128] = ts[3];
+        const bool in = rt != 0;
+        float b[4] = {in ? ox : FLT_MAX, in ? oy : FLT_MAX, in ? ox : -FLT_MAX, in ? oy : -FLT_MAX};
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            b[0] = fminf(b[0], __shfl_xor_sync(0xffffffffu, b[0], o));
+            b[1] = fminf(b[1], __shfl_xor_sync(0xffffffffu, b[1], o));
+            b[2] = fmaxf(b[2], __shfl_xor_sync(0xffffffffu, b[2], o));
+            b[3] = fmaxf(b[3], __shfl_xor_sync(0xffffffffu, b[3], o));
         }
-    if (idx == 0) ob[0] = fm(ob[0], 1.00001f);
-    if (acc.minx == FLT_MAX) { ob[0] = -1000.0f; return; }
+        if ((tid & 31) == 0)
+            for (int k = 0; k < 4; ++k) box[tid >> 5][k] = b[k];
+    }
+    __syncthreads();
+    const float bx0 = fminf(box[0][0], box[1][0]), by0 = fminf(box[0][1], box[1][1]);
+    const float bx1 = fmaxf(box[0][2], box[1][2]), by1 = fmaxf(box[0][3], box[1][3]);
+    if (bx0 == FLT_MAX) {   // all 64 rays miss
+        if (tid == 0) ob[0] = -1000.0f;
+        return;
+    }
+    // (the tile's first value starts at 0, which the reference's multiplies
+    // of tile 0 by 1.00001 before this point leave as it is)
+    if (tid < 3) {          // component tid of the mean direction
+        float a = 0.0f;
+        for (int k = 0; k < 64; ++k)
+            if (ray[k][3] != 0) a = fa(a, ray_t[k][1] > 0 ? fm(ray[k][tid], 2.0f) : ray[k][tid]);
+        total[tid] = a;
+    } else if (tid >= 32 && tid < 34) {   // depth gradients: horizontal, vertical
+        float a = 0.0f;
+        for (int s = 0; s < 16; ++s) {
+            float h = 0.0f;
+            for (int k = 4 * s; k < 4 * s + 4; ++k)
+                if (ray[k][3] != 0) h = fa(h, fa(ray_t[k][0], ray_t[k][1]));
+            a = fa(a, (tid == 32 ? (s & 3) >= 2 : (s >> 2) >= 2) ? h : -h);
+        }
+        total[3 + (tid - 32)] = a;
+    } else if (tid >= 40 && tid < 56) {   // the ray that stands for a sample
+        const int s = tid - 40;
+        const bool p25 = ((s + ((s >> 2) & 1)) & 1) != 0;
+        int best = 4 * s;
+        for (int k = 4 * s + 1; k < 4 * s + 4; ++k) {
+            const float c = ray[k][3], r = ray[best][3];
+            if ((c != 0 && ((c < r) != p25)) || r == 0) best = k;
+        }
+        const int fill = s / 2 + (p25 ? 8 : 0);
+        for (int k = 0; k < 4; ++k) samples[fill][k] = ray[best][k];
+    }
+    __syncthreads();
     Stream st(kPixelStream, (uint32_t)idx, 0, (uint32_t)T.frame, T.seed);
     f3 X, Y, Z, LX, LY, LZ;
-    basis(acc.avg, 0.0f, st, &X, &Y, &Z);
+    basis(mk3(total[0], total[1], total[2]), 0.0f, st, &X, &Y, &Z);
     basis(T.L, 0.0f, st, &LX, &LY, &LZ);
-    float minx = fs(acc.minx, 0.5f), miny = fs(acc.miny, 0.5f), maxx = fa(acc.maxx, 0.5f), maxy = fa(acc.maxy, 0.5f);
-    f3 blc = normalize(add(add(dir, mul(ro, minx)), mul(uo, miny)));
-    f3 rc = normalize(add(dir, mul(ro, maxx))), uc = normalize(add(dir, mul(uo, maxy)));
-    auto cl = [](float x) { return fmaxf(-1.0f, fminf(1.0f, x)); };
-    float* go = ob + 192 * 3;
-    go[0] = acosf(cl(dot(X, T.L)));
-    float gbl = acosf(cl(dot(blc, T.L)));
-    go[1] = fs(acosf(cl(dot(rc, T.L))), gbl);
-    go[2] = fs(acosf(cl(dot(uc, T.L))), gbl);
-    go[3] = hor;
-    go[4] = vert;
-    // SetupInputData2: X_Val [0, 192), X_Val_Hg [192, 384), X_Val_Sub [384, 576)
-    for (int k = 0; k < 16; ++k) {
-        const float* sm = samples[k];
-        if (sm[3] != 0) {
-            f3 sd = mk3(sm[0], sm[1], sm[2]);
-            f3 sp = add(T.ori, mul(sd, sm[3]));
-            float d = tex3<false>(mip_level(v, 0), 256, sp);
-            ob[k] = logf(fa(1.0f, fm(fm(T.alpha, d), 0.015625f)));
-            ob[192 + k] = logf(fa(hg(dot(sd, T.L), T.g), 1.0f));
-            ob[384 + k] = shadow_tr(v, sp, T.L, 0);
-        } else {
-            ob[k] = 0.0f; ob[192 + k] = 0.0f; ob[384 + k] = 0.0f;
-        }
+    if (tid == 0) {
+        float minx = fs(bx0, 0.5f), miny = fs(by0, 0.5f), maxx = fa(bx1, 0.5f), maxy = fa(by1, 0.5f);
+        f3 blc = normalize(add(add(dir, mul(ro, minx)), mul(uo, miny)));
+        f3 rc = normalize(add(dir, mul(ro, maxx))), uc = normalize(add(dir, mul(uo, maxy)));
+        auto cl = [](float x) { return fmaxf(-1.0f, fminf(1.0f, x)); };
+        float* go = ob + 192 * 3;
+        go[0] = acosf(cl(dot(X, T.L)));
+        float gbl = acosf(cl(dot(blc, T.L)));
+        go[1] = fs(acosf(cl(dot(rc, T.L))), gbl);
+        go[2] = fs(acosf(cl(dot(uc, T.L))), gbl);
+        go[3] = total[3];
+        go[4] = total[4];
     }
-    int sid = 0;
-    for (int k = 16; k < 192; ++k) {
-        while (samples[sid][3] == 0) sid = (sid + 1) & 0xf;
-        const float* sm = samples[sid];
-        sid = (sid + 1) & 0xf;
-        PixelFrame pf{add(T.ori, mul(mk3(sm[0], sm[1], sm[2]), sm[3])), X, Y, Z, T.L, T.L, T.g, T.alpha};
-        float fdv, fsv, fhv;
-        gather_sample(v, pf, k, &fdv, &fsv, &fhv);
+    // the samples that have a hit, in order: point k >= 16 takes them in turn
+    uint32_t have = 0;
+#pragma unroll
+    for (int s = 0; s < 16; ++s) have |= (uint32_t)(samples[s][3] != 0) << s;
+    const int n = __popc(have);
+    // SetupInputData2: X_Val [0, 192), X_Val_Hg [192, 384), X_Val_Sub [384, 576)
+    for (int k = tid; k < 192; k += kTileThreads) {
+        float fdv = 0.0f, fsv = 0.0f, fhv = 0.0f;
+        if (k < 16) {
+            const float* sm = samples[k];
+            if (sm[3] != 0) {
+                f3 sd = mk3(sm[0], sm[1], sm[2]);
+                f3 sp = add(T.ori, mul(sd, sm[3]));
+                float d = tex3<false>(mip_level(v, 0), 256, sp);
+                fdv = logf(fa(1.0f, fm(fm(T.alpha, d), 0.015625f)));
+                fhv = logf(fa(hg(dot(sd, T.L), T.g), 1.0f));
+                fsv = shadow_tr(v, sp, T.L, 0);
+            }
+        } else {
+            uint32_t m = have;
+            for (int q = (k - 16) % n; q; --q) m &= m - 1;
+            const float* sm = samples[__ffs(m) - 1];
+            PixelFrame pf{add(T.ori, mul(mk3(sm[0], sm[1], sm[2]), sm[3])), X, Y, Z, T.L, T.L, T.g, T.alpha};
+            gather_sample(v, pf, k, &fdv, &fsv, &fhv);
+        }
+        if (idx == 0 && k == 0) fdv = fm(fdv, 1.00001f);   // the reference's debug multiply of tile 0
         ob[k] = fdv;
         ob[192 + k] = fhv;
         ob[384 + k] = fsv;
     }
-    if (idx == 0) ob[0] = fm(ob[0], 1.00001f);
 }
 
 cudaError_t launch_gather_tiles(const VolumeDev& v, const ViewDev& view, int px, int py, const float nl[3], float* out,
@@ -1061,7 +1130,8 @@ cudaError_t launch_gather_tiles(const VolumeDev& v, const ViewDev& view, int px,
     if (n <= 0) return cudaSuccess;
     TileView T{view.width, view.height, px, py, view.frame, view.seed, view.ori, view.up, view.right,
                view.light_dir, view.alpha, view.g, {nl[0], nl[1], nl[2]}};
-    k_gather_tiles<<<(n + 63) / 64, 64, 0, s>>>(v, T, out);
+    if (v.density_h) k_gather_tiles<__half><<<n, kTileThreads, 0, s>>>(v, T, out);
+    else k_gather_tiles<float><<<n, kTileThreads, 0, s>>>(v, T, out);
     return cudaGetLastError();
 }
 
