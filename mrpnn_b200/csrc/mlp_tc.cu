@@ -3,15 +3,23 @@
 //
 // Layout of the work.  A persistent kernel with one CTA per SM holds every
 // layer's weights in shared memory as UMMA operand images (K-major, no
-// swizzle: 8-row x 16-byte core matrices).  Two groups of 128 threads each
-// own one 128-pixel tile at a time; thread t of a group owns pixel row t of
-// its tile and TMEM lane t.  Per layer step the group writes its A rows
-// (activations, rounded to BF16 or quantised to FP8-E4M3) to shared memory,
-// one elected thread issues tcgen05.mma into the group's TMEM columns and
-// commits to an mbarrier, and every thread reads its row of the FP32
-// accumulator back with tcgen05.ld for the epilogue (bias, ReLU, residuals,
-// gates), all in FP32 on the CUDA cores.  The SE gate MLPs, pooling, the
-// LSEFin gate and the last 16->1 layer stay in FP32.
+// swizzle: 8-row x 16-byte core matrices).  Three groups of 128 threads (two
+// for coloured albedos) each own one 128-pixel tile at a time; thread t of a
+// group owns pixel row t of its tile and TMEM lane t.  Per layer step the
+// group writes its A rows (activations, rounded to BF16 or quantised to
+// FP8-E4M3) to shared memory, one elected thread issues tcgen05.mma into the
+// group's TMEM columns and commits to an mbarrier, and every thread reads its
+// row of the FP32 accumulator back with tcgen05.ld for the epilogue (bias,
+// ReLU, residuals, gates), all in FP32 on the CUDA cores.  The SE gate MLPs,
+// pooling, the LSEFin gate and the last 16->1 layer stay in FP32.
+//
+// What bounds it: the latency of each tile's chain of dependent steps, so the
+// tiles in flight on an SM decide.  Three instead of two need a group's state
+// in 160 instead of 256 TMEM columns (residuals where the accumulators go,
+// comb where LC0's accumulator goes) and a thread's in 168 registers instead
+// of 248 (LC0..LX rows made 32 values at a time); the element-wise work in
+// register pairs (f32x2) takes 13 % of the instructions away.  BF16 network of
+// a 1920 x 1080 frame (966 K hits): 1.44 -> 1.10 ms, the same bits.
 //
 // Layers (58): per SE block three branch layers w x w (main widths 8, 8, 16,
 // 16, 16, 32, 32, 32; direct-illumination 4 x 8), the three final 32x32 and
@@ -65,8 +73,10 @@ __host__ __device__ constexpr int scale_off(int i) {
 constexpr int kScaleCount = scale_off(kLayers);
 // The fp32 constants the CUDA-core parts read, packed for shared memory:
 // FP8 weight scales, layer biases (both indexed by scale_off), the 12 SE gate
-// MLPs (8x8 + 3x8 each), LSEFin1 / LSEFin2, LGGS and the 16 -> 1 head.
-constexpr int kAuxScale = 0, kAuxBias = kScaleCount, kAuxSE = 2 * kScaleCount, kAuxLSE1 = kAuxSE + 12 * 88,
+// MLPs (input-major: 8 x 8, then 8 x 3 padded to 8 x 4), LSEFin1 / LSEFin2,
+// LGGS and the 16 -> 1 head.
+constexpr int kAuxSEBlock = 96;
+constexpr int kAuxScale = 0, kAuxBias = kScaleCount, kAuxSE = 2 * kScaleCount, kAuxLSE1 = kAuxSE + 12 * kAuxSEBlock,
               kAuxLSE2 = kAuxLSE1 + 1200, kAuxLGGSW = kAuxLSE2 + 96, kAuxLGGSB = kAuxLGGSW + 24,
               kAuxLX12W = kAuxLGGSB + 8, kAuxLX12B = kAuxLX12W + 16, kAuxCount = (kAuxLX12B + 1 + 3) / 4 * 4;
 // fp32 weight / bias of layer i in the packed fp32 layout (common.cuh)
@@ -80,7 +90,7 @@ __host__ __device__ constexpr int layer_w32(int i) {
 __host__ __device__ constexpr int layer_b32(int i) { return layer_w32(i) + layer_n(i) * layer_k(i); }
 static_assert(layer_b32(kLC0) == kLC0B && layer_b32(kLX0 + 11) == lxb(11), "layer table");
 static_assert(image_bytes(2) <= 110 * 1024, "BF16 weight image must fit shared memory");
-static_assert(kAuxBias % 4 == 0 && kAuxSE % 4 == 0 && kAuxLSE1 % 4 == 0 && kAuxLSE2 % 4 == 0 && 88 % 4 == 0,
+static_assert(kAuxBias % 4 == 0 && kAuxSE % 4 == 0 && kAuxLSE1 % 4 == 0 && kAuxLSE2 % 4 == 0 && kAuxSEBlock % 4 == 0,
               "constants read as float4 start on 16-byte boundaries");
 
 // Byte offset of element (row m, k) in a K-major no-swizzle operand tile of
@@ -150,7 +160,11 @@ cudaError_t tc_prepare_weights(const float* w32, TcWeights& w) {
         for (int r = 0; r < layer_n(i); ++r) aux[kAuxBias + scale_off(i) + r] = w32[layer_b32(i) + r];
     for (int b = 0; b < 12; ++b) {
         const float* src = w32 + (b < 8 ? mblk_off(b) : di_block_off(b - 8));
-        std::memcpy(&aux[kAuxSE + 88 * b], src, 88 * sizeof(float));
+        float* dst = &aux[kAuxSE + kAuxSEBlock * b];
+        for (int j = 0; j < 8; ++j) {
+            for (int o = 0; o < 8; ++o) dst[8 * j + o] = src[8 * o + j];
+            for (int o = 0; o < 3; ++o) dst[64 + 4 * j + o] = src[64 + 8 * o + j];
+        }
     }
     // LSEFin1 [16][75] (out, in) stored input-major [75][16]
     for (int o = 0; o < 16; ++o)
@@ -198,8 +212,14 @@ void tc_free_scratch(TcScratch& s) {
 // table (instead of one template instance per layer).
 // ---------------------------------------------------------------------------
 constexpr int kGroupThreads = 128;
-constexpr int kGroups = 2;
-constexpr int kTmemColsPerGroup = 256;
+constexpr int kTmemCols = 512;
+// Groups of a block (tiles in flight on an SM) and their share of tensor
+// memory: three where the pixels' albedo is grey, two where it is not, whose
+// tail runs once per channel and so keeps comb beside LC0's accumulator.
+template <bool COL> constexpr int kGroups = COL ? 2 : 3;
+template <bool COL> constexpr int kTmemColsPerGroup = COL ? 256 : 160;
+static_assert(kGroups<false> * kTmemColsPerGroup<false> <= kTmemCols && kGroups<true> * kTmemColsPerGroup<true> <= kTmemCols,
+              "tensor memory columns");
 constexpr uint32_t kWaitLimit = 1u << 22;   // polls before an MMA round is declared lost
 constexpr int kABytes = 128 * 128 * 2;      // one group's A buffer (largest: 128 x 128 BF16)
 
@@ -324,16 +344,24 @@ __device__ __forceinline__ float write_row(uint32_t a_s, int off, int row, const
     return s;
 }
 
-// Reads N (<= 128) accumulator columns of this thread's row.
-template <int N>
-__device__ __forceinline__ void read_cols(const Group& G, int col, float* out) {
+// Values [32 p, 32 p + 32) of this thread's A row of N (a multiple of 32).
+template <int EB, int N>
+MRP_D void store_part(const Group& G, int p, const float (&v)[32], float inv) {
+    constexpr int E = 16 / EB;
 #pragma unroll
-    for (int c = 0; c < (N + 15) / 16; ++c) {
-        float v[16];
-        tc::tmem_ld16(G.tmem + col + 16 * c, v);
+    for (int c = 0; c < 32 / E; ++c) {
+        uint32_t w[4];
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (16 * c + i < N) out[16 * c + i] = v[i];
+        for (int q = 0; q < 4; ++q) {
+            if (EB == 2) {
+                w[q] = tc::pack_bf16(v[8 * c + 2 * q], v[8 * c + 2 * q + 1]);
+            } else {
+                const int i = 16 * c + 4 * q;
+                w[q] = (uint32_t)tc::pack_e4m3(v[i] * inv, v[i + 1] * inv) |
+                       ((uint32_t)tc::pack_e4m3(v[i + 2] * inv, v[i + 3] * inv) << 16);
+            }
+        }
+        tc::st_shared_v4(G.a_s + (uint32_t)op_off(G.t, 32 * p + c * E, N, EB), w[0], w[1], w[2], w[3]);
     }
 }
 
@@ -358,24 +386,45 @@ MRP_D float lds1(const float* p) {
     return v;
 }
 
+// Two IEEE operations at once on register pairs (element-wise work is what
+// the threads of a row spend their instructions on).
+typedef unsigned long long u64;
+MRP_D u64 pk(float lo, float hi) {
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+MRP_D void upk(u64 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+MRP_D u64 fma2(u64 a, u64 b, u64 c) { u64 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+MRP_D u64 add2(u64 a, u64 b) { u64 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+MRP_D u64 mul2(u64 a, u64 b) { u64 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+MRP_D void add_to(float& a0, float& a1, float b0, float b1) { upk(add2(pk(a0, a1), pk(b0, b1)), a0, a1); }
+// a = x * g + a
+MRP_D void fma_to(float& a0, float& a1, float x0, float x1, u64 g) { upk(fma2(pk(x0, x1), g, pk(a0, a1)), a0, a1); }
+
 // Biases and scales start on 16-float boundaries (scale_off), so they are
-// read four at a time.
-template <int EB, int N>
+// read four at a time.  OFF: first output of the part at hand.
+template <int EB, int N, int OFF = 0>
 MRP_D void bias_relu(float* d, int L, float rs, const float* aux) {
     static_assert(N % 4 == 0, "layer widths are multiples of 4");
-    const int ab = c_layer_desc[L].abias, so = c_layer_desc[L].soff;
+    const int ab = c_layer_desc[L].abias + OFF, so = c_layer_desc[L].soff + OFF;
 #pragma unroll
     for (int q = 0; q < N / 4; ++q) {
         const float4 b = lds4(aux + ab + 4 * q);
-        float4 sc = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        u64 lo = pk(d[4 * q], d[4 * q + 1]), hi = pk(d[4 * q + 2], d[4 * q + 3]);
         if (EB == 1) {
             const float4 w = lds4(aux + kAuxScale + so + 4 * q);
-            sc = make_float4(rs * w.x, rs * w.y, rs * w.z, rs * w.w);
+            const u64 r2 = pk(rs, rs);
+            lo = fma2(lo, mul2(r2, pk(w.x, w.y)), pk(b.x, b.y));
+            hi = fma2(hi, mul2(r2, pk(w.z, w.w)), pk(b.z, b.w));
+        } else {
+            lo = add2(lo, pk(b.x, b.y));
+            hi = add2(hi, pk(b.z, b.w));
         }
-        d[4 * q] = fmaxf(fmaf(d[4 * q], sc.x, b.x), 0.0f);
-        d[4 * q + 1] = fmaxf(fmaf(d[4 * q + 1], sc.y, b.y), 0.0f);
-        d[4 * q + 2] = fmaxf(fmaf(d[4 * q + 2], sc.z, b.z), 0.0f);
-        d[4 * q + 3] = fmaxf(fmaf(d[4 * q + 3], sc.w, b.w), 0.0f);
+        upk(lo, d[4 * q], d[4 * q + 1]);
+        upk(hi, d[4 * q + 2], d[4 * q + 3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[4 * q + i] = fmaxf(d[4 * q + i], 0.0f);
     }
 }
 // n consecutive constants (16-byte aligned, n a multiple of 4) into registers.
@@ -412,14 +461,19 @@ struct TileFeatures {          // FP16 pairs of the staged predictor's tiled lay
     }
 };
 
-// Per-row state that lives in TMEM between blocks (columns of the group's
-// 256; the MMA accumulators use 0..95 (main blocks, finals), 128..175 (DI
-// blocks), 176..223 (DI finals)): the LSEFin1 partial sums and the residual
-// of the main (3 x 32) and direct-illumination (3 x 8) chains.  Keeping them
-// out of registers leaves the per-block routines without a stack frame for
-// them.
-constexpr int kColHf = 96, kColPrevMain = 160, kColPrevDi = 232;
-
+// Per-row state that lives in TMEM between blocks.  Of a group's columns the
+// main chain has 0..95, 32 a channel, the direct-illumination chain
+// 112..159, 16 a channel: a channel's residual lies where the MMAs put its
+// accumulator, since it has gone into the A row before the MMA that
+// overwrites it is issued.  96..111 hold the LSEFin1 partial sums.  In the
+// tail of a grey albedo comb lies in 0..119 until LC0's accumulator (0..127)
+// takes its place, the LSEFin1 sums in 128..143 and the residual pairs' state
+// in 144..159; of a coloured one comb lies in 136..255, the sums are put into
+// 96..111 again before each channel, and the pairs' state follows them there.
+constexpr int kColHf = 96, kColDi = 112;
+template <bool COL> constexpr int kColComb = COL ? 136 : 0;
+template <bool COL> constexpr int kColHfTail = COL ? 96 : 128;
+template <bool COL> constexpr int kColA16 = COL ? 96 : 144;
 template <int N>
 MRP_D void tmem_get(const Group& G, int col, float* out) {
     if constexpr (N == 8) {
@@ -457,34 +511,32 @@ MRP_D void tmem_put(const Group& G, int col, const float* v) {
     }
 }
 
-struct BlockDesc { int w, from, widen, has_prev, l0, dcol, se_off, pid, pcol, pstride; };
+struct BlockDesc { int w, from, widen, has_prev, l0, col, stride, se_off, pid; };
 __constant__ BlockDesc c_blocks[12] = {
-    {8, 0, 0, 0, 0, 0, kAuxSE + 88 * 0, 0, kColPrevMain, 32},      {8, 8, 1, 1, 3, 0, kAuxSE + 88 * 1, 3, kColPrevMain, 32},
-    {16, 16, 0, 1, 6, 0, kAuxSE + 88 * 2, 6, kColPrevMain, 32},    {16, 32, 0, 1, 9, 0, kAuxSE + 88 * 3, 9, kColPrevMain, 32},
-    {16, 48, 1, 1, 12, 0, kAuxSE + 88 * 4, 12, kColPrevMain, 32},  {32, 64, 0, 1, 15, 0, kAuxSE + 88 * 5, 15, kColPrevMain, 32},
-    {32, 96, 0, 1, 18, 0, kAuxSE + 88 * 6, 18, kColPrevMain, 32},  {32, 128, 0, 1, 21, 0, kAuxSE + 88 * 7, 21, kColPrevMain, 32},
-    {8, 160, 0, 0, 27, 128, kAuxSE + 88 * 8, 24, kColPrevDi, 8}, {8, 168, 0, 1, 30, 128, kAuxSE + 88 * 9, 27, kColPrevDi, 8},
-    {8, 176, 0, 1, 33, 128, kAuxSE + 88 * 10, 30, kColPrevDi, 8}, {8, 184, 0, 1, 36, 128, kAuxSE + 88 * 11, 33, kColPrevDi, 8},
+    {8, 0, 0, 0, 0, 0, 32, kAuxSE + kAuxSEBlock * 0, 0},      {8, 8, 1, 1, 3, 0, 32, kAuxSE + kAuxSEBlock * 1, 3},
+    {16, 16, 0, 1, 6, 0, 32, kAuxSE + kAuxSEBlock * 2, 6},    {16, 32, 0, 1, 9, 0, 32, kAuxSE + kAuxSEBlock * 3, 9},
+    {16, 48, 1, 1, 12, 0, 32, kAuxSE + kAuxSEBlock * 4, 12},  {32, 64, 0, 1, 15, 0, 32, kAuxSE + kAuxSEBlock * 5, 15},
+    {32, 96, 0, 1, 18, 0, 32, kAuxSE + kAuxSEBlock * 6, 18},  {32, 128, 0, 1, 21, 0, 32, kAuxSE + kAuxSEBlock * 7, 21},
+    {8, 160, 0, 0, 27, kColDi, 16, kAuxSE + kAuxSEBlock * 8, 24}, {8, 168, 0, 1, 30, kColDi, 16, kAuxSE + kAuxSEBlock * 9, 27},
+    {8, 176, 0, 1, 33, kColDi, 16, kAuxSE + kAuxSEBlock * 10, 30}, {8, 184, 0, 1, 36, kColDi, 16, kAuxSE + kAuxSEBlock * 11, 33},
 };
 
 // One SE block over the three channels (SE / SERES + ADD3 / REP3,
 // core/radiancePredict.cu:240-294): gate from the slice pools, branch layers
-// l0..l0+2 on the tensor cores (D at dcol, dcol+stride, dcol+2*stride), then
-// prev <- relu(D + b) + slice (ADD3) or concat(relu(D + b), slice) (REP3).
+// l0..l0+2 on the tensor cores (accumulators at col, stride columns a channel
+// on), then prev <- relu(D + b) + slice (ADD3) or concat(relu(D + b), slice)
+// (REP3), left where the accumulator was.
 template <int EB, int W, class Src>
 __device__ __noinline__ int tc_block(const Group G, int st, const Src src, const float* aux, int b, float g,
                                      float gamma) {
     const BlockDesc bd = c_blocks[b];
-    const int from = bd.from, widen = bd.widen, has_prev = bd.has_prev, l0 = bd.l0, dcol = bd.dcol,
-              se_off = bd.se_off, pid = bd.pid, pcol = bd.pcol, pstride = bd.pstride;
     constexpr int KP = pad_to(W, EB == 2 ? 16 : 32);
     constexpr int SUB = 128 * KP * EB;   // bytes of one branch's A sub-tile
-    constexpr int DSTR = W <= 16 ? 16 : 32;
     float xs[3][W];                      // the block's feature slice, loaded once
     float p8[8];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        src.template load<W>(c, from, xs[c]);
+        src.template load<W>(c, bd.from, xs[c]);
         float s = 0.0f, m = -10000.0f;
 #pragma unroll
         for (int i = 0; i < W; ++i) { s += xs[c][i]; m = fmaxf(m, xs[c][i]); }
@@ -494,74 +546,82 @@ __device__ __noinline__ int tc_block(const Group G, int st, const Src src, const
     p8[6] = g;
     p8[7] = gamma;
     // LSEFin1 (75 -> 16) accumulated block by block in TMEM: pool[pid + c] =
-    // avg, pool[36 + pid + c] = max
+    // avg, pool[36 + pid + c] = max; LSEFin1 is stored input-major (the 16
+    // weights of input j at kAuxLSE1 + 16 j), outputs in pairs
     {
         float hf[16];
         tmem_get<16>(G, kColHf, hf);
-        // (LSEFin1 is stored input-major: the 16 weights of input j at
-        // kAuxLSE1 + 16 j; per output the same sequence of FMAs as o-major)
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            float wa[16], wm[16];
-            aux_row<16>(aux, kAuxLSE1 + 16 * (pid + c), wa);
-            aux_row<16>(aux, kAuxLSE1 + 16 * (36 + pid + c), wm);
+            const u64 av = pk(p8[c], p8[c]), mx = pk(p8[3 + c], p8[3 + c]);
 #pragma unroll
-            for (int o = 0; o < 16; ++o) {
-                hf[o] = fmaf(wa[o], p8[c], hf[o]);
-                hf[o] = fmaf(wm[o], p8[3 + c], hf[o]);
+            for (int q = 0; q < 4; ++q) {
+                const float4 wa = lds4(aux + kAuxLSE1 + 16 * (bd.pid + c) + 4 * q);
+                const float4 wm = lds4(aux + kAuxLSE1 + 16 * (36 + bd.pid + c) + 4 * q);
+                fma_to(hf[4 * q], hf[4 * q + 1], wa.x, wa.y, av);
+                fma_to(hf[4 * q + 2], hf[4 * q + 3], wa.z, wa.w, av);
+                fma_to(hf[4 * q], hf[4 * q + 1], wm.x, wm.y, mx);
+                fma_to(hf[4 * q + 2], hf[4 * q + 3], wm.z, wm.w, mx);
             }
         }
         tmem_put<16>(G, kColHf, hf);
     }
-    float h[8], gate[3];
+    u64 gate[3];
+    {
+        float h[8], a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-    for (int o = 0; o < 8; ++o) {
-        float w[8];
-        aux_row<8>(aux, se_off + o * 8, w);
-        float a = 0.0f;
+        for (int o = 0; o < 8; ++o) h[o] = 0.0f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) a = fmaf(p8[j], w[j], a);
-        h[o] = fmaxf(a, 0.0f);
-    }
+        for (int j = 0; j < 8; ++j) {
+            const float4 u = lds4(aux + bd.se_off + 8 * j), v = lds4(aux + bd.se_off + 8 * j + 4);
+            const u64 p = pk(p8[j], p8[j]);
+            fma_to(h[0], h[1], u.x, u.y, p);
+            fma_to(h[2], h[3], u.z, u.w, p);
+            fma_to(h[4], h[5], v.x, v.y, p);
+            fma_to(h[6], h[7], v.z, v.w, p);
+        }
 #pragma unroll
-    for (int o = 0; o < 3; ++o) {
-        float w[8];
-        aux_row<8>(aux, se_off + 64 + o * 8, w);
-        float a = 0.0f;
+        for (int j = 0; j < 8; ++j) {
+            const float4 u = lds4(aux + bd.se_off + 64 + 4 * j);
+            h[j] = fmaxf(h[j], 0.0f);
+            fma_to(a[0], a[1], u.x, u.y, pk(h[j], h[j]));
+            a[2] = fmaf(h[j], u.z, a[2]);
+        }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) a = fmaf(h[j], w[j], a);
-        gate[o] = sigmoid_d(a);
+        for (int o = 0; o < 3; ++o) {
+            const float q = sigmoid_d(a[o]);
+            gate[o] = pk(q, q);
+        }
     }
     float rs[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         float in[W];
-        if (has_prev) {
-            float pv[W];
-            tmem_get<W>(G, pcol + c * pstride, pv);
+        if (bd.has_prev) {
+            tmem_get<W>(G, bd.col + c * bd.stride, in);
 #pragma unroll
-            for (int i = 0; i < W; ++i) in[i] = fmaf(xs[c][i], gate[c], pv[i]);
+            for (int i = 0; i < W; i += 2) fma_to(in[i], in[i + 1], xs[c][i], xs[c][i + 1], gate[c]);
         } else {
 #pragma unroll
-            for (int i = 0; i < W; ++i) in[i] = xs[c][i] * gate[c];
+            for (int i = 0; i < W; i += 2) upk(mul2(pk(xs[c][i], xs[c][i + 1]), gate[c]), in[i], in[i + 1]);
         }
         rs[c] = write_row<EB, W, KP>(G.a_s, c * SUB, G.t, in);
     }
-    st = mma_round<EB>(G, st, 3, l0, SUB, dcol, DSTR);
+    st = mma_round<EB>(G, st, 3, bd.l0, SUB, bd.col, bd.stride);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         float d[W];
-        read_cols<W>(G, dcol + c * DSTR, d);
-        bias_relu<EB, W>(d, l0 + c, rs[c], aux);
-        if (widen) {
+        tmem_get<W>(G, bd.col + c * bd.stride, d);
+        bias_relu<EB, W>(d, bd.l0 + c, rs[c], aux);
+        if (bd.widen) {
             float nv[2 * W];
 #pragma unroll
             for (int o = 0; o < W; ++o) { nv[o] = d[o]; nv[W + o] = xs[c][o]; }
-            tmem_put<2 * W>(G, pcol + c * pstride, nv);
+            tmem_put<2 * W>(G, bd.col + c * bd.stride, nv);
         } else {
 #pragma unroll
-            for (int o = 0; o < W; ++o) d[o] = d[o] + xs[c][o];
-            tmem_put<W>(G, pcol + c * pstride, d);
+            for (int o = 0; o < W; o += 2) add_to(d[o], d[o + 1], xs[c][o], xs[c][o + 1]);
+            tmem_put<W>(G, bd.col + c * bd.stride, d);
         }
     }
     tc::tmem_wait_st();
@@ -570,98 +630,141 @@ __device__ __noinline__ int tc_block(const Group G, int st, const Src src, const
 
 // Residual pair k of the tail: a += relu(LX(2k+1) relu(LX(2k) a + b) + b),
 // a (16 values) kept in TMEM columns kColA16.
-constexpr int kColA16 = 96;
-template <int EB>
+template <int EB, bool COL>
 __device__ __noinline__ int tc_residual_pair(const Group G, int st, const float* aux, int k) {
     constexpr int KP = EB == 2 ? 16 : 32;
     const int La = kLX0 + 2 * k, Lb = La + 1;
     float a16[16];
-    tmem_get<16>(G, kColA16, a16);
+    tmem_get<16>(G, kColA16<COL>, a16);
     float r0 = write_row<EB, 16, KP>(G.a_s, 0, G.t, a16);
     st = mma_round<EB>(G, st, 1, La, 0, 64, 0);
     float u[16];
-    read_cols<16>(G, 64, u);
+    tmem_get<16>(G, 64, u);
     bias_relu<EB, 16>(u, La, r0, aux);
     float r1 = write_row<EB, 16, KP>(G.a_s, 0, G.t, u);
     st = mma_round<EB>(G, st, 1, Lb, 0, 80, 0);
     float z[16];
-    read_cols<16>(G, 80, z);
+    tmem_get<16>(G, 80, z);
     bias_relu<EB, 16>(z, Lb, r1, aux);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) a16[i] += z[i];
-    tmem_put<16>(G, kColA16, a16);
+    for (int i = 0; i < 16; i += 2) add_to(a16[i], a16[i + 1], z[i], z[i + 1]);
+    tmem_put<16>(G, kColA16<COL>, a16);
     tc::tmem_wait_st();
     return st;
 }
 
+// An A row of N values that come in parts of 32: get(part, v) makes part
+// `part`.  FP8 rows take two passes, the first for the row's scale, so the
+// row is never held whole.
+template <int EB, int N, class F>
+MRP_D float write_parts(const Group& G, F get) {
+    float v[32];
+    if (EB == 2) {
+#pragma unroll
+        for (int p = 0; p < N / 32; ++p) {
+            get(p, v);
+            store_part<EB, N>(G, p, v, 1.0f);
+        }
+        return 1.0f;
+    }
+    float amax = 0.0f;
+#pragma unroll
+    for (int p = 0; p < N / 32; ++p) {
+        get(p, v);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    }
+    const float s = amax > 0.0f ? amax * (1.0f / 448.0f) : 1.0f, inv = 1.0f / s;
+#pragma unroll
+    for (int p = 0; p < N / 32; ++p) {
+        get(p, v);
+        store_part<EB, N>(G, p, v, inv);
+    }
+    return s;
+}
+
 // The tail of one albedo channel (core/radiancePredict.cu:375-419): LSEFin
 // gate, LC0 over [comb * gate, LGGS], LC1, LC2, LX, six residual pairs and
-// the 16 -> 1 head.  comb comes from TMEM (kColComb); the accumulators use
-// columns 0..127 only, so comb survives for the next channel.
-constexpr int kColComb = 136;
+// the 16 -> 1 head.  comb (kColComb) and the LSEFin1 sums (kColHfTail) come
+// from TMEM.
 struct TailOut { float p; int st; };
-// hf (the LSEFin1 partial sums) is read from TMEM columns kColHf first thing.
-template <int EB>
+template <int EB, bool COL>
 __device__ __noinline__ TailOut tc_tail(const Group G, int st, const float* aux, float g, float gamma, float s4) {
-    float h[16], gf[6];
-    tmem_get<16>(G, kColHf, h);
+    float gf[6];
+    {
+        float h[16];
+        tmem_get<16>(G, kColHfTail<COL>, h);
 #pragma unroll
-    for (int o = 0; o < 16; ++o) {
-        float a = h[o];
-        a = fmaf(lds1(aux + kAuxLSE1 + 16 * 72 + o), g, a);
-        a = fmaf(lds1(aux + kAuxLSE1 + 16 * 73 + o), gamma, a);
-        a = fmaf(lds1(aux + kAuxLSE1 + 16 * 74 + o), s4, a);
-        h[o] = fmaxf(a, 0.0f);
-    }
+        for (int o = 0; o < 16; ++o) {
+            float a = h[o];
+            a = fmaf(lds1(aux + kAuxLSE1 + 16 * 72 + o), g, a);
+            a = fmaf(lds1(aux + kAuxLSE1 + 16 * 73 + o), gamma, a);
+            a = fmaf(lds1(aux + kAuxLSE1 + 16 * 74 + o), s4, a);
+            h[o] = fmaxf(a, 0.0f);
+        }
 #pragma unroll
-    for (int o = 0; o < 6; ++o) {
-        float w[16];
-        aux_row<16>(aux, kAuxLSE2 + o * 16, w);
-        float a = 0.0f;
+        for (int o = 0; o < 6; ++o) {
+            float w[16];
+            aux_row<16>(aux, kAuxLSE2 + o * 16, w);
+            float a = 0.0f;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) a = fmaf(h[j], w[j], a);
-        gf[o] = sigmoid_d(a);
+            for (int j = 0; j < 16; ++j) a = fmaf(h[j], w[j], a);
+            gf[o] = sigmoid_d(a);
+        }
     }
     // LC0's A row: [comb * gate segment, LGGS (3 -> 8)]
-    float x[128];
-    tmem_get<32>(G, kColComb, x);
-    tmem_get<32>(G, kColComb + 32, x + 32);
-    tmem_get<32>(G, kColComb + 64, x + 64);
-    tmem_get<8>(G, kColComb + 96, x + 96);
-    tmem_get<8>(G, kColComb + 104, x + 104);
-    tmem_get<8>(G, kColComb + 112, x + 112);
+    float r = write_parts<EB, 128>(G, [&](int p, float (&v)[32]) {
+        if (p < 3) {
+            tmem_get<32>(G, kColComb<COL> + 32 * p, v);
+            const u64 q = pk(gf[p], gf[p]);
 #pragma unroll
-    for (int i = 0; i < 120; ++i) x[i] = x[i] * gf[i < 96 ? i / 32 : 3 + (i - 96) / 8];
+            for (int i = 0; i < 32; i += 2) upk(mul2(pk(v[i], v[i + 1]), q), v[i], v[i + 1]);
+        } else {
+            float e[24];
+            tmem_get<16>(G, kColComb<COL> + 96, e);
+            tmem_get<8>(G, kColComb<COL> + 112, e + 16);
 #pragma unroll
-    for (int o = 0; o < 8; ++o) {
-        float a = 0.0f;
-        a = fmaf(g, lds1(aux + kAuxLGGSW + o * 3), a);
-        a = fmaf(gamma, lds1(aux + kAuxLGGSW + o * 3 + 1), a);
-        a = fmaf(s4, lds1(aux + kAuxLGGSW + o * 3 + 2), a);
-        x[120 + o] = fmaxf(a + lds1(aux + kAuxLGGSB + o), 0.0f);
-    }
-    float r = write_row<EB, 128, kpad(kLC0, EB)>(G.a_s, 0, G.t, x);
+            for (int i = 0; i < 24; ++i) v[i] = e[i] * gf[3 + i / 8];
+#pragma unroll
+            for (int o = 0; o < 8; ++o) {
+                float a = 0.0f;
+                a = fmaf(g, lds1(aux + kAuxLGGSW + o * 3), a);
+                a = fmaf(gamma, lds1(aux + kAuxLGGSW + o * 3 + 1), a);
+                a = fmaf(s4, lds1(aux + kAuxLGGSW + o * 3 + 2), a);
+                v[24 + o] = fmaxf(a + lds1(aux + kAuxLGGSB + o), 0.0f);
+            }
+        }
+    });
     st = mma_round<EB>(G, st, 1, kLC0, 0, 0, 0);
-    read_cols<128>(G, 0, x);
-    bias_relu<EB, 128>(x, kLC0, r, aux);
-    r = write_row<EB, 128, kpad(kLC1, EB)>(G.a_s, 0, G.t, x);
+    float rn = write_parts<EB, 128>(G, [&](int p, float (&v)[32]) {
+        tmem_get<32>(G, 32 * p, v);
+        if (p == 0) bias_relu<EB, 32, 0>(v, kLC0, r, aux);
+        else if (p == 1) bias_relu<EB, 32, 32>(v, kLC0, r, aux);
+        else if (p == 2) bias_relu<EB, 32, 64>(v, kLC0, r, aux);
+        else bias_relu<EB, 32, 96>(v, kLC0, r, aux);
+    });
     st = mma_round<EB>(G, st, 1, kLC1, 0, 0, 0);
-    read_cols<64>(G, 0, x);
-    bias_relu<EB, 64>(x, kLC1, r, aux);
-    r = write_row<EB, 64, kpad(kLC2, EB)>(G.a_s, 0, G.t, x);
+    r = rn;
+    rn = write_parts<EB, 64>(G, [&](int p, float (&v)[32]) {
+        tmem_get<32>(G, 32 * p, v);
+        if (p == 0) bias_relu<EB, 32, 0>(v, kLC1, r, aux);
+        else bias_relu<EB, 32, 32>(v, kLC1, r, aux);
+    });
     st = mma_round<EB>(G, st, 1, kLC2, 0, 0, 0);
-    read_cols<32>(G, 0, x);
-    bias_relu<EB, 32>(x, kLC2, r, aux);
-    r = write_row<EB, 32, kpad(kLX, EB)>(G.a_s, 0, G.t, x);
+    r = rn;
+    rn = write_parts<EB, 32>(G, [&](int, float (&v)[32]) {
+        tmem_get<32>(G, 0, v);
+        bias_relu<EB, 32>(v, kLC2, r, aux);
+    });
     st = mma_round<EB>(G, st, 1, kLX, 0, 32, 0);
     float a16[16];
-    read_cols<16>(G, 32, a16);
-    bias_relu<EB, 16>(a16, kLX, r, aux);
-    tmem_put<16>(G, kColA16, a16);
+    tmem_get<16>(G, 32, a16);
+    bias_relu<EB, 16>(a16, kLX, rn, aux);
+    tmem_put<16>(G, kColA16<COL>, a16);
     tc::tmem_wait_st();
 #pragma unroll 1
-    for (int k = 0; k < 6; ++k) st = tc_residual_pair<EB>(G, st, aux, k);
-    tmem_get<16>(G, kColA16, a16);
+    for (int k = 0; k < 6; ++k) st = tc_residual_pair<EB, COL>(G, st, aux, k);
+    tmem_get<16>(G, kColA16<COL>, a16);
     float a = 0.0f;
 #pragma unroll
     for (int j = 0; j < 16; ++j) a = fmaf(a16[j], lds1(aux + kAuxLX12W + j), a);
@@ -677,7 +780,7 @@ MRP_D int run_block(const Group& G, int st, const Src& src, const float* aux, in
     return tc_block<EB, 32>(G, st, src, aux, b, g, gamma);
 }
 
-template <int EB, class Src>
+template <int EB, bool COL, class Src>
 MRP_D int tc_network(const Group& G, int st, const Src& src, const float* aux,
                       float gamma, float g, f3 sr, float out[3]) {
     {
@@ -687,7 +790,7 @@ MRP_D int tc_network(const Group& G, int st, const Src& src, const float* aux,
         tmem_put<16>(G, kColHf, z);
         tc::tmem_wait_st();
     }
-    // main branch, X[0:160]; the three 32x32 finals leave comb[0:96) in TMEM columns 0..95
+    // main branch, X[0:160], and its three 32x32 finals
 #pragma unroll 1
     for (int b = 0; b < 8; ++b) st = run_block<EB>(G, st, src, aux, b, g, gamma);
     float rs_main[3];
@@ -696,12 +799,12 @@ MRP_D int tc_network(const Group& G, int st, const Src& src, const float* aux,
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             float pv[32];
-            tmem_get<32>(G, kColPrevMain + 32 * c, pv);
+            tmem_get<32>(G, 32 * c, pv);
             rs_main[c] = write_row<EB, 32, KP>(G.a_s, c * SUB, G.t, pv);
         }
         st = mma_round<EB>(G, st, 3, kL81, SUB, 0, 32);
     }
-    // direct-illumination branch, X[160:192]; the 8x8 finals at columns 176..223
+    // direct-illumination branch, X[160:192], and its 8x8 finals
 #pragma unroll 1
     for (int b = 8; b < 12; ++b) st = run_block<EB>(G, st, src, aux, b, g, gamma);
     float rs_di[3];
@@ -710,46 +813,51 @@ MRP_D int tc_network(const Group& G, int st, const Src& src, const float* aux,
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             float pv[8];
-            tmem_get<8>(G, kColPrevDi + 8 * c, pv);
+            tmem_get<8>(G, kColDi + 16 * c, pv);
             rs_di[c] = write_row<EB, 8, KP>(G.a_s, c * SUB, G.t, pv);
         }
-        st = mma_round<EB>(G, st, 3, kLD41, SUB, 176, 16);
+        st = mma_round<EB>(G, st, 3, kLD41, SUB, kColDi, 16);
     }
+    // comb[120] = relu(finals + b): the direct-illumination part behind the
+    // main one, once it and the LSEFin1 sums have been read
     float hf[16];
-    tmem_get<16>(G, kColHf, hf);   // before LC0's accumulator covers columns 0..127
-    // comb[120] = relu(finals + b) -> TMEM columns kColComb..+119: the DI
-    // finals (176..223) first, then the main ones (0..95) -- the main comb
-    // lands on 136..231, over DI columns already read.
+    {
+        float e[3][8];
+        tmem_get<16>(G, kColHf, hf);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        float e[8];
-        read_cols<8>(G, 176 + 16 * c, e);
-        bias_relu<EB, 8>(e, kLD41 + c, rs_di[c], aux);
-        tmem_put<8>(G, kColComb + 96 + 8 * c, e);
+        for (int c = 0; c < 3; ++c) tmem_get<8>(G, kColDi + 16 * c, e[c]);
+        tmem_put<16>(G, kColHfTail<COL>, hf);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            bias_relu<EB, 8>(e[c], kLD41 + c, rs_di[c], aux);
+            tmem_put<8>(G, kColComb<COL> + 96 + 8 * c, e[c]);
+        }
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         float m[32];
-        read_cols<32>(G, 32 * c, m);
+        tmem_get<32>(G, 32 * c, m);
         bias_relu<EB, 32>(m, kL81 + c, rs_main[c], aux);
-        tmem_put<32>(G, kColComb + 32 * c, m);
+        tmem_put<32>(G, kColComb<COL> + 32 * c, m);
     }
     tc::tmem_wait_st();
     // tail, once per distinct albedo channel (core/radiancePredict.cu:375-419)
-    float srv[3] = {sr.x, sr.y, sr.z}, P[3];
+    const float srv[3] = {sr.x, sr.y, sr.z};
+    float P[3];
 #pragma unroll
-    for (int ch = 0; ch < 3; ++ch) {
+    for (int ch = 0; ch < (COL ? 3 : 1); ++ch) {
         if (ch == 1 && srv[1] == srv[0]) { P[1] = P[0]; continue; }
         if (ch == 2 && srv[2] == srv[0]) { P[2] = P[0]; continue; }
         if (ch == 2 && srv[2] == srv[1]) { P[2] = P[1]; continue; }
-        if (ch > 0) {   // the previous tail's accumulators covered kColHf
-            tmem_put<16>(G, kColHf, hf);
+        if (ch > 0) {   // the previous tail's accumulators covered the sums
+            tmem_put<16>(G, kColHfTail<COL>, hf);
             tc::tmem_wait_st();
         }
-        TailOut t = tc_tail<EB>(G, st, aux, g, gamma, powf(srv[ch], 4.0f));
+        TailOut t = tc_tail<EB, COL>(G, st, aux, g, gamma, powf(srv[ch], 4.0f));
         st = t.st;
         P[ch] = t.p;
     }
+    if (!COL) P[1] = P[2] = P[0];
 #pragma unroll
     for (int c = 0; c < 3; ++c) out[c] = fmaxf(expf(P[c]) - 1.0f, 0.0f) * powf(srv[c], 4.0f);
     return st;
@@ -777,16 +885,16 @@ struct TcArgs {
     TcSegment seg0;
 };
 
-template <int EB, bool STAGED>
-__global__ void __launch_bounds__(kGroups * kGroupThreads, 1) k_mlp_tc(const __grid_constant__ TcArgs A) {
+template <int EB, bool STAGED, bool COL>
+__global__ void __launch_bounds__(kGroups<COL> * kGroupThreads, 1) k_mlp_tc(const __grid_constant__ TcArgs A) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const int wbytes = (A.wimg_bytes + 1023) & ~1023;
     uint8_t* wimg = smem;
     uint8_t* abuf = smem + wbytes;
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(abuf + kGroups * kABytes);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + kGroups);
+    uint64_t* mbar = reinterpret_cast<uint64_t*>(abuf + kGroups<COL> * kABytes);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + kGroups<COL>);
     int* tile_slot = reinterpret_cast<int*>(tslot + 1);
-    int* seg_start = tile_slot + kGroups;   // staged: first tile of each segment, [nseg + 1]
+    int* seg_start = tile_slot + kGroups<COL>;   // staged: first tile of each segment, [nseg + 1]
     float* aux_s = reinterpret_cast<float*>(seg_start + kTcMaxSegments + 1 + 3);   // 16-byte aligned below
     const TcSegment* segs = A.segs ? A.segs : &A.seg0;
     const int nseg = A.segs ? A.nseg : 1;
@@ -799,10 +907,10 @@ __global__ void __launch_bounds__(kGroups * kGroupThreads, 1) k_mlp_tc(const __g
     for (int i = tid * 4; i < kAuxCount; i += blockDim.x * 4)
         *reinterpret_cast<float4*>(aux_s + i) = __ldg(reinterpret_cast<const float4*>(A.aux + i));
     if (warp == 0) {
-        tc::tmem_alloc(tslot, kGroups * kTmemColsPerGroup);
+        tc::tmem_alloc(tslot, kTmemCols);
         tc::tmem_relinquish();
     }
-    if (tid < kGroups) tc::mbar_init(mbar + tid, 1);
+    if (tid < kGroups<COL>) tc::mbar_init(mbar + tid, 1);
     if (STAGED && tid == 32) {
         int acc = 0;
         for (int q = 0; q < nseg; ++q) {
@@ -823,13 +931,17 @@ __global__ void __launch_bounds__(kGroups * kGroupThreads, 1) k_mlp_tc(const __g
     G.a_s = tc::smem_addr(abuf + G.g * kABytes);
     G.wimg_s = tc::smem_addr(wimg);
     G.mbar_s = tc::smem_addr(mbar + G.g);
-    G.tmem = tbase + (uint32_t)(G.g * kTmemColsPerGroup) + ((uint32_t)(32 * ((tid / 32) % 4)) << 16);
+    G.tmem = tbase + (uint32_t)(G.g * kTmemColsPerGroup<COL>) + ((uint32_t)(32 * ((tid / 32) % 4)) << 16);
     G.err = A.err;
     int st = 0;
 
     const int total_tiles = STAGED ? seg_start[nseg] : (A.n + 127) / 128;
-    for (;;) {
-        if (G.t == 0) tile_slot[G.g] = atomicAdd(A.tile_counter, 1);
+    // the first tiles go round the blocks (few tiles: each its own SM), the
+    // rest to whichever group is free
+    for (bool first = true;; first = false) {
+        if (G.t == 0)
+            tile_slot[G.g] = first ? G.g * (int)gridDim.x + (int)blockIdx.x
+                                   : kGroups<COL> * (int)gridDim.x + atomicAdd(A.tile_counter, 1);
         group_bar(G.g);
         int tile = tile_slot[G.g];
         group_bar(G.g);
@@ -848,7 +960,7 @@ __global__ void __launch_bounds__(kGroups * kGroupThreads, 1) k_mlp_tc(const __g
             const size_t cap = S->rec_cap;
             float gamma = valid ? S->rec_f[15 * cap + r] : 0.0f;
             TileFeatures src{reinterpret_cast<const __half2*>(S->feat) + (size_t)(r >> 5) * 288 * 32 + (r & 31), valid};
-            st = tc_network<EB>(G, st, src, aux_s, gamma, S->g, S->sr, o);
+            st = tc_network<EB, COL>(G, st, src, aux_s, gamma, S->g, S->sr, o);
             if (valid && !(st & kStFailed)) {
                 int pix = S->rec_pix[r];
                 f3 hit = mk3(S->rec_f[r], S->rec_f[cap + r], S->rec_f[2 * cap + r]);
@@ -866,7 +978,7 @@ __global__ void __launch_bounds__(kGroups * kGroupThreads, 1) k_mlp_tc(const __g
             const bool valid = r < A.n;
             float gamma = valid ? A.gamma[r] : 0.0f;
             RowFeatures src{A.feat + (size_t)r * 576, valid};
-            st = tc_network<EB>(G, st, src, aux_s, gamma, A.g, A.sr, o);
+            st = tc_network<EB, COL>(G, st, src, aux_s, gamma, A.g, A.sr, o);
             if (valid && !(st & kStFailed)) {
                 A.out3[3 * (size_t)r] = o[0];
                 A.out3[3 * (size_t)r + 1] = o[1];
@@ -878,24 +990,30 @@ __global__ void __launch_bounds__(kGroups * kGroupThreads, 1) k_mlp_tc(const __g
     __syncthreads();
     if (warp == 0) {
         tc::fence_after_sync();
-        tc::tmem_dealloc(tbase, kGroups * kTmemColsPerGroup);
+        tc::tmem_dealloc(tbase, kTmemCols);
     }
 }
 
-static size_t tc_smem_bytes(int eb) {
-    return (size_t)((image_bytes(eb) + 1023) & ~1023) + kGroups * kABytes + kGroups * 8 + 16 +
+static size_t tc_smem_bytes(int eb, int groups) {
+    return (size_t)((image_bytes(eb) + 1023) & ~1023) + groups * kABytes + groups * 8 + 16 +
            (kTcMaxSegments + 1 + 3) * sizeof(int) + 16 + kAuxCount * sizeof(float);
 }
 
-template <int EB, bool STAGED>
+template <int EB, bool STAGED, bool COL>
 static cudaError_t launch_tc(TcArgs& a, int sms, cudaStream_t s) {
-    size_t smem = tc_smem_bytes(EB);
-    cudaError_t e = cudaFuncSetAttribute(k_mlp_tc<EB, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    size_t smem = tc_smem_bytes(EB, kGroups<COL>);
+    cudaError_t e = cudaFuncSetAttribute(k_mlp_tc<EB, STAGED, COL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(a.tile_counter, 0, sizeof(int), s)) != cudaSuccess) return e;
-    k_mlp_tc<EB, STAGED><<<sms, kGroups * kGroupThreads, smem, s>>>(a);
+    k_mlp_tc<EB, STAGED, COL><<<sms, kGroups<COL> * kGroupThreads, smem, s>>>(a);
     return cudaGetLastError();
 }
+template <bool STAGED>
+static cudaError_t launch_tc(TcArgs& a, bool fp8, bool coloured, int sms, cudaStream_t s) {
+    if (coloured) return fp8 ? launch_tc<1, STAGED, true>(a, sms, s) : launch_tc<2, STAGED, true>(a, sms, s);
+    return fp8 ? launch_tc<1, STAGED, false>(a, sms, s) : launch_tc<2, STAGED, false>(a, sms, s);
+}
+static bool is_coloured(f3 sr) { return !(sr.x == sr.y && sr.x == sr.z); }
 
 static TcArgs base_args(const TcWeights& w, bool fp8) {
     TcArgs a{};
@@ -917,7 +1035,7 @@ cudaError_t tc_launch_mlp(const TcWeights& w, bool fp8, const float* feat, const
     a.g = g;
     a.sr = mk3(sr[0], sr[1], sr[2]);
     a.out3 = out3;
-    return fp8 ? launch_tc<1, false>(a, sms, s) : launch_tc<2, false>(a, sms, s);
+    return launch_tc<false>(a, fp8, is_coloured(a.sr), sms, s);
 }
 
 cudaError_t tc_launch_mlp_at(const TcWeights& w, bool fp8, const float* feat, const float* gamma, float g,
@@ -935,7 +1053,7 @@ cudaError_t tc_launch_mlp_at(const TcWeights& w, bool fp8, const float* feat, co
     a.out3 = out3;
     cudaError_t e = cudaMemsetAsync(err, 0, sizeof(int), s);
     if (e != cudaSuccess) return e;
-    return fp8 ? launch_tc<1, false>(a, sms, s) : launch_tc<2, false>(a, sms, s);
+    return launch_tc<false>(a, fp8, is_coloured(a.sr), sms, s);
 }
 
 TcSegment tc_segment(const VolumeDev& v, const ViewDev& view, const HitRecords& rec, const float* feat,
@@ -966,19 +1084,21 @@ cudaError_t tc_launch_mlp_rec(const TcWeights& w, bool fp8, const VolumeDev& v, 
     a.segs = nullptr;
     a.nseg = 1;
     a.seg0 = tc_segment(v, view, rec, feat, accum);
-    return fp8 ? launch_tc<1, true>(a, sms, s) : launch_tc<2, true>(a, sms, s);
+    return launch_tc<true>(a, fp8, is_coloured(a.seg0.sr), sms, s);
 }
 
-cudaError_t tc_launch_mlp_segments(const TcWeights& w, bool fp8, const TcSegment* d_segs, int nseg,
-                                   const TcScratch& sc, int sms, cudaStream_t s) {
-    if (!w.ready || !w.d_fp32 || !sc.d || !d_segs) return cudaErrorNotReady;
+cudaError_t tc_launch_mlp_segments(const TcWeights& w, bool fp8, const TcSegment* d_segs, const TcSegment* h_segs,
+                                   int nseg, const TcScratch& sc, int sms, cudaStream_t s) {
+    if (!w.ready || !w.d_fp32 || !sc.d || !d_segs || !h_segs) return cudaErrorNotReady;
     if (nseg < 1 || nseg > kTcMaxSegments) return cudaErrorInvalidValue;
     TcArgs a = base_args(w, fp8);
     a.tile_counter = sc.d;
     a.err = sc.d + 1;
     a.segs = d_segs;
     a.nseg = nseg;
-    return fp8 ? launch_tc<1, true>(a, sms, s) : launch_tc<2, true>(a, sms, s);
+    bool coloured = false;
+    for (int q = 0; q < nseg; ++q) coloured = coloured || is_coloured(h_segs[q].sr);
+    return launch_tc<true>(a, fp8, coloured, sms, s);
 }
 
 // ---------------------------------------------------------------------------

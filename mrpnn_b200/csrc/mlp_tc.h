@@ -56,9 +56,10 @@ cudaError_t tc_launch_mlp_rec(const TcWeights& w, bool fp8, const VolumeDev& v, 
                               const HitRecords& rec, const float* feat, float4* accum, const TcScratch& sc, int sms,
                               cudaStream_t s);
 // The network over several requests' records in one persistent launch:
-// d_segs[0, nseg) in device memory (nseg <= kTcMaxSegments).
-cudaError_t tc_launch_mlp_segments(const TcWeights& w, bool fp8, const TcSegment* d_segs, int nseg,
-                                   const TcScratch& sc, int sms, cudaStream_t s);
+// d_segs[0, nseg) in device memory (nseg <= kTcMaxSegments), h_segs the same
+// on the host.
+cudaError_t tc_launch_mlp_segments(const TcWeights& w, bool fp8, const TcSegment* d_segs, const TcSegment* h_segs,
+                                   int nseg, const TcScratch& sc, int sms, cudaStream_t s);
 
 // Self-test: D[128][n] = A[128][k] * B[n][k]^T with operands rounded to BF16
 // (or E4M3), k a multiple of 16 (32), n a multiple of 16 up to 128.

@@ -82,7 +82,7 @@ mrp_status mrp_render_views(mrp_volume* v, const mrp_view* views, int n, float* 
     if (tc) {
         CU(cudaMemcpyAsync(B.d_segs, segs.data(), n * sizeof(TcSegment), cudaMemcpyHostToDevice, v->stream));
         CU(cudaMemsetAsync(v->tc.d + 1, 0, sizeof(int), v->stream));
-        CU(tc_launch_mlp_segments(g.tc, v->params.precision == MRP_FP8, B.d_segs, n, v->tc, g.sms, v->stream));
+        CU(tc_launch_mlp_segments(g.tc, v->params.precision == MRP_FP8, B.d_segs, segs.data(), n, v->tc, g.sms, v->stream));
     }
     CU(cudaEventRecord(v->ev_stage[1], v->stream));
     for (int i = 0; i < n; ++i) {

@@ -434,7 +434,7 @@ bool mrp_server::launch_network() {
     cudaError_t e;
     if ((e = cudaMemcpyAsync(d_segs, h_segs, n * sizeof(TcSegment), cudaMemcpyHostToDevice, net)) != cudaSuccess ||
         (e = cudaMemsetAsync(sc.d + 1, 0, sizeof(int), net)) != cudaSuccess ||
-        (e = tc_launch_mlp_segments(g.tc, cfg.precision == MRP_FP8, d_segs, n, sc, g.sms, net)) != cudaSuccess ||
+        (e = tc_launch_mlp_segments(g.tc, cfg.precision == MRP_FP8, d_segs, h_segs, n, sc, g.sms, net)) != cudaSuccess ||
         (e = cudaMemcpyAsync(h_err, sc.d + 1, sizeof(int), cudaMemcpyDeviceToHost, net)) != cudaSuccess ||
         (e = cudaEventRecord(ev_net, net)) != cudaSuccess) {
         for (int i : batch) {
