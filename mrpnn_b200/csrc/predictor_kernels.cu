@@ -43,6 +43,8 @@ constexpr int kStencilRuns[12][3] = {{0, 0, 8},     {1, 8, 16},    {2, 16, 32}, 
 __constant__ int c_stencil_runs[12][3] = {{0, 0, 8},     {1, 8, 16},    {2, 16, 32},   {3, 32, 48},
                                           {4, 48, 64},   {5, 64, 96},   {6, 96, 128},  {7, 128, 160},
                                           {0, 160, 168}, {1, 168, 176}, {2, 176, 184}, {3, 184, 192}};
+// The runs in six parts of 32 points each: first run of part p, and the end.
+__constant__ int c_stencil_parts[7] = {0, 3, 5, 6, 7, 8, 12};
 cudaError_t set_stencil_tables(const StencilTables& t) {
     cudaError_t e;
     // the staged gather is compiled for the runs of kStencilRuns
@@ -476,21 +478,21 @@ MRP_D void gather_point_fast(const VolumeDev& v, const PixelFrame& f, const RunL
     }
     *fs_ = tr;
 }
-// All 192 points, run by run (GetSamples23_'s layout: layers 0..7 over the
+// The points of runs [first_run, end_run) (0, 12: all 192), run by run (GetSamples23_'s layout: layers 0..7 over the
 // 160 rotated directions, then layers 0..3 on the light ray), into a tiled
 // feature layout: fp32 (record r, channel c, sample i at word
 // ((r / 32) * 576 + c * 192 + i) * 32 + r % 32), or FP16 pairs (samples 2k,
 // 2k + 1 of channel c as one half2 at word ((r / 32) * 288 + c * 96 + k) * 32
 // + r % 32).  Either way a warp of 32 records writes 128 contiguous bytes.
 template <bool FP16>
-MRP_D void gather_all_fast(const VolumeDev& v, const PixelFrame& f, float* feat, int r) {
+MRP_D void gather_all_fast(const VolumeDev& v, const PixelFrame& f, float* feat, int r, int first_run, int end_run) {
     float* out = feat + (size_t)(r >> 5) * 576 * 32 + (r & 31);
     __half2* out2 = reinterpret_cast<__half2*>(feat) + (size_t)(r >> 5) * 288 * 32 + (r & 31);
     float pa = 0.0f, pb = 0.0f, pc = 0.0f;   // the even sample of a pair
     const HgFast H = FP16 ? hg_fast(v, f) : HgFast{mk3(0, 0, 0), 0.0f, 0.0f, nullptr};
     const f3 iLX = inv(f.LX);
 #pragma unroll 1
-    for (int run = 0; run < 12; ++run) {
+    for (int run = first_run; run < end_run; ++run) {
         const int layer = c_stencil_runs[run][0], from = c_stencil_runs[run][1], to = c_stencil_runs[run][2];
         const int tl = layer > 1 ? layer - 1 : 0;
         // edge <= 8 (mips 5..7, TR levels 4..6): most footprints touch the
@@ -597,13 +599,13 @@ MRP_D void gather_point_tex(const VolumeDev& v, const PixelFrame& f, const TexRu
         *fh_ = __logf(fmaf(a, b, 1.0f));
     }
 }
-MRP_D void gather_all_tex(const VolumeDev& v, const PixelFrame& f, float* feat, int r) {
+MRP_D void gather_all_tex(const VolumeDev& v, const PixelFrame& f, float* feat, int r, int first_run, int end_run) {
     __half2* out2 = reinterpret_cast<__half2*>(feat) + (size_t)(r >> 5) * 288 * 32 + (r & 31);
     float pa = 0.0f, pb = 0.0f, pc = 0.0f;   // the even sample of a pair
     const HgFast H = hg_fast(v, f);
     const f3 iLX = inv(f.LX);
 #pragma unroll 1
-    for (int run = 0; run < 12; ++run) {
+    for (int run = first_run; run < end_run; ++run) {
         const int layer = c_stencil_runs[run][0], from = c_stencil_runs[run][1], to = c_stencil_runs[run][2];
         const float n = (float)(256 >> layer);
         const TexRun R = layer == 0 ? TexRun{v.gmip0_tex, v.gtr0_tex, 0.0f, 0.0f, false, from >= 160}
@@ -762,8 +764,13 @@ __global__ void __launch_bounds__(128) k_gather_rec(VolumeDev v, ViewDev w, HitR
     int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= *rec.count) return;
     PixelFrame pf = record_frame(rec, r, normalize(w.light_dir), w.g, w.alpha);
-    if (TEX) gather_all_tex(v, pf, feat, r);
-    else gather_all_fast<FP16>(v, pf, feat, r);
+    int first_run = 0, end_run = 12;
+    if (gridDim.y > 1) {   // one of the six parts of the stencil
+        first_run = c_stencil_parts[blockIdx.y];
+        end_run = c_stencil_parts[blockIdx.y + 1];
+    }
+    if (TEX) gather_all_tex(v, pf, feat, r, first_run, end_run);
+    else gather_all_fast<FP16>(v, pf, feat, r, first_run, end_run);
 }
 
 // Per-pixel intermediates for the debug entry point: aux [npix][20] = hit
@@ -1139,9 +1146,17 @@ cudaError_t launch_gather_rec(const VolumeDev& v, const ViewDev& view, HitRecord
                               cudaStream_t s) {
     int n = view.width * view.height;
     if (n <= 0) return cudaSuccess;
-    if (fp16 && v.glut_tex) k_gather_rec<true, true><<<(n + 127) / 128, 128, 0, s>>>(v, view, rec, feat);
-    else if (fp16) k_gather_rec<true><<<(n + 127) / 128, 128, 0, s>>>(v, view, rec, feat);
-    else k_gather_rec<false><<<(n + 127) / 128, 128, 0, s>>>(v, view, rec, feat);
+    // A record's 192 points in series take 100 us (texture form; 170 us the
+    // FP32 form) however few records there are; six threads a record, 32
+    // points each, take 28 us (53 us) for small frames and still 239 against
+    // 249 us at 724^2 pixels.  At 1024^2 (half of them hits) the records fill
+    // the SMs by themselves: 465 against 444 us for the texture form, while
+    // the FP32 form, waiting for its loads, still gains (961 against 978 us).
+    const bool parts = !fp16 || n <= 600000;
+    const dim3 grid((n + 127) / 128, parts ? 6 : 1);
+    if (fp16 && v.glut_tex) k_gather_rec<true, true><<<grid, 128, 0, s>>>(v, view, rec, feat);
+    else if (fp16) k_gather_rec<true><<<grid, 128, 0, s>>>(v, view, rec, feat);
+    else k_gather_rec<false><<<grid, 128, 0, s>>>(v, view, rec, feat);
     return cudaGetLastError();
 }
 cudaError_t launch_debug_scatter(HitRecords rec, const float* feat, bool fp16, int npix, float* aux, float* feat_out,
