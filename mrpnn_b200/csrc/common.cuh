@@ -90,16 +90,27 @@ MRP_D f3 sample_hg(float e0, float e1, f3 v, float g) {
     }
     float phi = (float)(2.0 * 3.14159265359 * (double)e1);
     float sint = fsq(fmaxf(0.0f, fs(1.0f, fm(cost, cost))));
-    f3 v2 = fabsf(v.z) > 0.70710678118654757 ? normalize(cross(v, mk3(0, 1, 0))) : normalize(cross(v, mk3(0, 0, 1)));
-    f3 v3 = cross(v2, v);
-    return add(add(mul(v3, fm(sint, cosf(phi))), mul(v2, fm(sint, sinf(phi)))), mul(v, cost));
+    // normalize(cross(v, y)) = (-v.z, 0, v.x) / l or normalize(cross(v, z)) =
+    // (v.y, -v.x, 0) / l: the products with the axis' zeros and ones are
+    // exact, so the two components carry all of it
+    const bool up = fabsf(v.z) > 0.70710678118654757;
+    float a = up ? -v.z : v.y, b = up ? v.x : -v.x;
+    const float l = fsq(fa(fm(a, a), fm(b, b)));
+    a = fd(a, l);
+    b = fd(b, l);
+    const f3 v2 = up ? mk3(a, 0.0f, b) : mk3(a, b, 0.0f), v3 = cross(v2, v);
+    float sn, cs;
+    sincosf(phi, &sn, &cs);
+    return add(add(mul(v3, fm(sint, cs)), mul(v2, fm(sint, sn))), mul(v, cost));
 }
 // UniformSampleSphere (core/vector.cu:195-208)
 MRP_D f3 uniform_sphere(float ex, float ey) {
     float phi = fm(fm(2.0f, 3.14159265359f), ex);
     float cost = fs(1.0f, fm(2.0f, ey));
     float sint = fsq(fs(1.0f, fm(cost, cost)));
-    return {fm(sint, cosf(phi)), fm(sint, sinf(phi)), cost};
+    float sn, cs;
+    sincosf(phi, &sn, &cs);
+    return {fm(sint, cs), fm(sint, sn), cost};
 }
 
 // ---------------------------------------------------------------------------

@@ -14,32 +14,55 @@
 // next flight) of every lane that has collided.  Collided lanes wait until
 // kScatterBatch of them are pending (or no lane can step), so the long
 // collision branch runs with many lanes at once instead of with the one or
-// two that collide in a given step.  A lane whose sample ends takes the next
-// item from a global counter at once (one atomic per warp for all lanes
-// that need work).  Every sample has its own Philox stream (sub = sample
-// index) and its arithmetic is CalculateRadiance's, in the reference's order,
-// so results do not depend on which lane ran it or when.  The free-flight
-// step (distance and accept test) uses the fast log and division that the
-// reference's -use_fast_math build compiles to (CMakeLists.txt:184); the
-// rest is in IEEE float.  Per-sample radiance is fp32, accumulated per pixel
-// in FP64.
+// two that collide in a given step; ended lanes likewise wait until
+// kRefillBatch of them deposit their samples and take the next items from a
+// global counter (one atomic per warp).  Every sample has its own Philox
+// stream (sub = sample index) and its arithmetic is CalculateRadiance's, in
+// the reference's order, so results do not depend on which lane ran it or
+// when.  The free-flight step (distance and accept test) uses the fast log
+// and division that the reference's -use_fast_math build compiles to
+// (CMakeLists.txt:184); the rest is in IEEE float.  Per-sample radiance is
+// fp32, accumulated per pixel in FP64.
+//
+// Bound by instructions, most of them issued for part of a warp.  256^2, 16
+// spp, <= 256 bounces, 128^3 cloud (1 M samples, 52 M steps, 6.5 M
+// collisions): 2.37 ms when ended lanes were refilled one by one and each
+// lane ran Philox as its own four draws ended (10.7 of 32 lanes active);
+// 1.60 ms with refills in batches, draws in windows (LaneStream) and a
+// shorter sample_hg.
 #include "kernels.h"
 #include "tracing.cuh"
 
 namespace mrp {
 
 namespace {
-constexpr int kScatterBatch = 8;
+constexpr int kTraceThreads = 128;
+constexpr int kTraceBlocks = 7;   // resident per SM (72 registers; eight at 64: 1.61, six: 1.57, seven: 1.55 ms)
+constexpr int kScatterBatch = 7, kRefillBatch = 12;   // 8 and 8: 1.59, 7 and 8: 1.56, 7 and 16 (eight blocks): 1.70 ms
 
-// The sample's kPixelStream: the state of Stream(kPixelStream, pix, k,
-// frame, seed) without its constant fields (same draws).
+// A lane's window of its sample's kPixelStream (the uniforms of Stream(
+// kPixelStream, pix, k, frame, seed)): every use takes two of them, and up to
+// four pairs wait in shared memory, two of them made by one Philox block.
+// Lanes stand at different places of their streams, so a block made for each
+// lane as it runs dry would run for half of the lanes at nearly every step;
+// here all lanes with room make one whenever one is empty.
 struct LaneStream {
-    uint32_t n, blk[4];
-    MRP_D float next(uint32_t pix, uint32_t k, uint32_t frame, uint32_t seed) {
-        if ((n & 3) == 0) philox(n >> 2, k, frame, kPixelStream, pix, seed ^ (kPixelStream * 0x9E3779B9u), blk);
-        uint32_t x = (n & 2) ? ((n & 1) ? blk[3] : blk[2]) : ((n & 1) ? blk[1] : blk[0]);
-        ++n;
-        return u01(x);
+    uint2* win;        // pair p of this lane at win[(p & 3) * kTraceThreads]
+    uint32_t used, made;   // pairs
+    MRP_D void start() { used = made = 0; }
+    MRP_D bool empty() const { return used == made; }
+    MRP_D bool room() const { return made - used <= 2; }
+    MRP_D void make(uint32_t pix, uint32_t k, uint32_t frame, uint32_t seed) {
+        uint32_t b[4];
+        philox(made >> 1, k, frame, kPixelStream, pix, seed ^ (kPixelStream * 0x9E3779B9u), b);
+        win[(made & 3) * kTraceThreads] = make_uint2(b[0], b[1]);
+        win[((made + 1) & 3) * kTraceThreads] = make_uint2(b[2], b[3]);
+        made += 2;
+    }
+    MRP_D float2 next() {
+        const uint2 x = win[(used & 3) * kTraceThreads];
+        ++used;
+        return make_float2(u01(x.x), u01(x.y));
     }
 };
 
@@ -70,7 +93,7 @@ MRP_D void deposit(double* __restrict__ sum3, double* __restrict__ sumsq3, int* 
 }  // namespace
 
 template <bool COUNT, class DT, bool TEX = false, bool ENV = false>
-__global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ VolumeDev v,
+__global__ void __launch_bounds__(kTraceThreads, kTraceBlocks) k_trace(const __grid_constant__ VolumeDev v,
                                                const __grid_constant__ ViewDev w, double* __restrict__ sum3,
                                                double* __restrict__ sumsq3, int* __restrict__ first_pos,
                                                unsigned long long* __restrict__ counter) {
@@ -80,26 +103,36 @@ __global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ Volume
     const float smax = fm(v.max_density, w.alpha);
     const uint32_t frame = (uint32_t)w.frame, seed = w.seed;
     const unsigned lane = threadIdx.x & 31, lt_mask = (1u << lane) - 1u;
+    __shared__ uint2 windows[4 * kTraceThreads];
     Tally tally;
     // the lane's sample: pixel, index, stream, vertex, direction, throughput,
     // radiance, bounce, free-flight distance / limit / iteration
     bool live = false, dry = false, hit = false;
+    int ended = 0;   // the lane's last sample waits to be deposited: 1 out of bounces, 2 left the box
     int pix = 0, k = 0, b = 0, loop = 0;
     uint32_t nee_n = 0;
-    LaneStream st{0, {0, 0, 0, 0}};
+    LaneStream st{windows + threadIdx.x, 0, 0};
     f3 p = mk3(0, 0, 0), rd = p, csr = p, res = p;
     float t = 0.0f, md = 0.0f;
     for (;;) {
-        // refill: every lane without a sample takes the next item (rays that
-        // miss the box are resolved to the sky here and refilled again)
-        for (;;) {
-            const unsigned need = __ballot_sync(0xffffffffu, !live && !dry);
-            if (!need) break;
+        // refill: lanes without a sample take the next items, once enough of
+        // them wait or nobody else has work (a sample takes about fifty
+        // steps, so without waiting this long branch would run for one or two
+        // lanes at almost every other step)
+        const unsigned need = __ballot_sync(0xffffffffu, !live && !dry);
+        const unsigned busy = __ballot_sync(0xffffffffu, live);
+        if (need && (__popc(need) >= kRefillBatch || !busy)) {
             const int leader = __ffs(need) - 1;
             unsigned long long base = 0;
             if ((int)lane == leader) base = atomicAdd(counter, (unsigned long long)__popc(need));
             base = __shfl_sync(0xffffffffu, base, leader);
             if (!live && !dry) {
+                if (ended) {   // (deposited here, with the others that wait, not one lane at a time)
+                    if (ended == 2)
+                        res = add(res, mul(ENV ? sky_map(v.hdri, v.hdri_w, v.hdri_h, v.env_exp, rd) : v.sky, csr));
+                    deposit(sum3, sumsq3, first_pos, pix, k, res, true);
+                    ended = 0;
+                }
                 const unsigned long long item = base + __popc(need & lt_mask);
                 if (item >= total) {
                     dry = true;
@@ -124,7 +157,7 @@ __global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ Volume
                         if (w.multi_scatter < 1) {
                             deposit(sum3, sumsq3, first_pos, pix, k, mk3(0, 0, 0), true);
                         } else {
-                            st.n = 0;
+                            st.start();
                             nee_n = 0;
                             res = mk3(0, 0, 0);
                             p = add(ori, mul(dir, dis));
@@ -144,39 +177,42 @@ __global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ Volume
         }
         const unsigned pend = __ballot_sync(0xffffffffu, live && hit);
         const unsigned fly = __ballot_sync(0xffffffffu, live && !hit);
-        if (!(pend | fly)) break;
+        if (!(pend | fly)) {
+            if (__ballot_sync(0xffffffffu, !dry)) continue;   // (rays that missed the box)
+            break;
+        }
+        if (__any_sync(0xffffffffu, live && st.empty())) {
+            if (live && st.room()) st.make(pix, k, frame, seed);
+        }
         if (fly && __popc(pend) < kScatterBatch) {
             if (!live || hit) continue;
             // one iteration of DeterminateNextVertex's loop (while (loop++ < 10000))
             if (loop >= 10000) { hit = true; continue; }
             ++loop;
-            float rk = st.next(pix, k, frame, seed);
+            const float2 rk = st.next();
             // the free-flight step in the reference's build arithmetic
             // (-use_fast_math: __logf, __fdividef), 10 % of the frame
             // against IEEE log and division; decisions stay per sample
-            t = t - __fdividef(__logf(1.0f - rk), smax);
+            t = t - __fdividef(__logf(1.0f - rk.x), smax);
             if (t > md) {   // left the box: sky radiance, the sample ends
-                res = add(res, mul(ENV ? sky_map(v.hdri, v.hdri_w, v.hdri_h, v.env_exp, rd) : v.sky, csr));
-                deposit(sum3, sumsq3, first_pos, pix, k, res, true);
+                ended = 2;
                 live = false;
                 continue;
             }
-            rk = st.next(pix, k, frame, seed);
             const f3 q = add(p, mul(rd, t));
             // the texture unit's filter (tracer_filter 1), as the reference's
             // Density(): tex3D(uv.z, uv.y, uv.x) with uv = pos + 0.5
             float d = TEX ? tex3D<float>(v.dens_tex, q.z + 0.5f, q.y + 0.5f, q.x + 0.5f) : density_t<DT>(v, q);
             if (COUNT) tally.fetches++;
             float S = d * w.alpha;
-            hit = __fdividef(S, smax) > rk;
+            hit = __fdividef(S, smax) > rk.y;
             if (!hit && d < 0) t = fs(t, d);
             continue;
         }
         if (!live || !hit) continue;
         // real collision: phase sampling, NEE, next flight
-        float e1 = st.next(pix, k, frame, seed);
-        float e0 = st.next(pix, k, frame, seed);
-        f3 nd = sample_hg(e0, e1, rd, w.g);
+        const float2 e = st.next();   // (first draw e1, second e0)
+        f3 nd = sample_hg(e.y, e.x, rd, w.g);
         p = add(mul(rd, t), p);
         csr = mul(csr, v.scatter_rate);
         float ph = hg(dot(rd, L), w.g);
@@ -190,7 +226,7 @@ __global__ void __launch_bounds__(128, 8) k_trace(const __grid_constant__ Volume
         rd = nd;
         hit = false;
         if (++b >= w.multi_scatter) {
-            deposit(sum3, sumsq3, first_pos, pix, k, res, true);
+            ended = 1;
             live = false;
         } else {
             md = ray_box_distance(p, rd);
@@ -307,7 +343,7 @@ cudaError_t launch_fill_int(int* p, int n, int value, cudaStream_t s) {
 template <class DT>
 static void launch_trace_dt(const VolumeDev& v, const ViewDev& view, double* sum3, double* sumsq3, int* first_pos,
                             unsigned long long* counter, int sms, cudaStream_t s) {
-    const dim3 grid(sms * 8), block(128);
+    const dim3 grid(sms * kTraceBlocks), block(kTraceThreads);
     if (view.counters) k_trace<true, DT><<<grid, block, 0, s>>>(v, view, sum3, sumsq3, first_pos, counter);
     else if (v.dens_tex && v.hdri) k_trace<false, DT, true, true><<<grid, block, 0, s>>>(v, view, sum3, sumsq3, first_pos, counter);
     else if (v.dens_tex) k_trace<false, DT, true, false><<<grid, block, 0, s>>>(v, view, sum3, sumsq3, first_pos, counter);
