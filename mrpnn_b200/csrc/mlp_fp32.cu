@@ -11,13 +11,16 @@
 // before this one) spent its time waiting for those weights (5.69 ms).  Here
 // a block of eight warps takes a tile of 64 pixels (32 for few pixels):
 // activations [row][pixel] and the weights of the layer at hand in shared
-// memory; a thread makes 8 pixels x up to 4 outputs in registers, a warp 64
-// pixels x 16 outputs, so one input row costs a warp three 16-byte loads a
-// lane for 32 multiply-adds, which are issued as 16 paired ones
-// (fma.rn.f32x2: two IEEE fused multiply-adds).  509 K hits: 2.02 ms, shared-
-// memory wavefronts at 73 % of their peak (a 16-byte load costs a warp four);
-// tiles of 128 pixels with a thread's features loaded where they are used:
-// 3.03 ms.  200 003 feature sets in rows: 3.25 -> 0.93 ms.
+// memory; a thread makes 8 pixels x 4 outputs of a wide layer in registers, 4
+// pixels x up to 4 outputs of a narrow one, and issues its multiply-adds in
+// pairs (fma.rn.f32x2: two IEEE fused multiply-adds).  A shared-memory load
+// costs a warp one wavefront per float a lane gets, whatever the lanes share,
+// so floats loaded per multiply-add decide (12 for 32 in the wide layers).
+// 509 K hits: 1.86 ms; 2.02 with 8 pixels a thread in the narrow layers too;
+// 1.98 with four warps of 8 x 8 a thread (two warps a scheduler do not hide
+// the latencies, and coloured albedos take 1.17 instead of 0.98 ms per 100
+// 001 sets); 3.03 with 128 pixels a tile and features loaded where they are
+// used.  200 003 sets in rows: 3.25 -> 0.87 ms.
 //
 // Weights stream through two 8 KB stages in 28 chunks (laid out input-major
 // on the host) and the SE blocks' feature slices through two 24 KB regions,
@@ -35,7 +38,7 @@ namespace mrp {
 
 namespace {
 
-constexpr int kThreads = 256, kWarps = 8;
+constexpr int kThreads = 256;   // eight warps
 constexpr int kChunk = 2048;   // floats of a stage
 enum Chunk { kCGate = 0, kCFin1 = 1, kCHead = 2, kCB2 = 3, kCB4 = 4, kCB5 = 5, kCFinal = 11, kCLC0 = 13, kCLC1 = 21,
              kCLC2 = 25, kCRes0 = 26, kCRes1 = 27, kChunks = 28 };
@@ -156,7 +159,10 @@ MRP_D void stv(float* p, const Vec<N>& r) {
     else *p = r.v[0];
 }
 
-// The layer phases: H groups of four pixels, lane l's at 32 h + 4 (l % 8).
+// The layer phases.  Wide layers: a thread has H groups of four pixels, lane
+// l's at 32 h + 4 (l % 8), and outputs by l / 8 (of four).  Narrow layers:
+// one group of four pixels, at 4 (l % (8 H)), and outputs by l / (8 H) (of
+// 4 / H), twice as many for H = 2: fewer floats loaded per multiply-add.
 template <int H>
 struct Px { float v[4 * H]; };
 template <int H>
@@ -258,10 +264,11 @@ struct TiledSource {   // the staged predictor's tiled layout (launch_gather_rec
         }
     }
     // NO samples from row o of a channel's region for a thread's pixels
-    template <int H, int NO>
-    static MRP_D void region(const float* reg, int o, int pg, Px<H> (&x)[NO]) {
+    // (G: the thread's groups of four pixels, H or 1)
+    template <int H, int G, int NO>
+    static MRP_D void region(const float* reg, int o, int pg, Px<G> (&x)[NO]) {
 #pragma unroll
-        for (int n = 0; n < NO; ++n) x[n] = ldp<H>(reg + (o + n) * 32 * H, pg);
+        for (int n = 0; n < NO; ++n) x[n] = ldp<G>(reg + (o + n) * 32 * H, pg);
     }
 };
 // [n][576], a pixel's features in a row; region: [pixel slot][32 samples] in
@@ -313,12 +320,12 @@ struct RowSource {
             }
         }
     }
-    template <int H, int NO>
-    static MRP_D void region(const float* reg, int o, int pg, Px<H> (&x)[NO]) {   // o a multiple of NO
+    template <int H, int G, int NO>
+    static MRP_D void region(const float* reg, int o, int pg, Px<G> (&x)[NO]) {   // o a multiple of NO
 #pragma unroll
-        for (int p = 0; p < 4 * H; ++p) {
+        for (int p = 0; p < 4 * G; ++p) {
             const int s = (p & 3) * 8 * H + (p >> 2) * 8 + pg;
-            const float* d = reg + s * 32 + ((o >> 2) ^ pg) * 4 + (o & 3);
+            const float* d = reg + s * 32 + ((o >> 2) ^ (pg & 7)) * 4 + (o & 3);
             if constexpr (NO == 4) { const float4 q = *reinterpret_cast<const float4*>(d); x[0].v[p] = q.x; x[1].v[p] = q.y; x[2].v[p] = q.z; x[3].v[p] = q.w; }
             else if constexpr (NO == 2) { const float2 q = *reinterpret_cast<const float2*>(d); x[0].v[p] = q.x; x[1].v[p] = q.y; }
             else x[0].v[p] = *d;
@@ -449,47 +456,46 @@ struct Net {
     }
     // Main block b, channel c: layer, then the next block's inputs in place:
     // out = relu(acc) (+ slice, or beside it when the block widens), next
-    // input = next slice * next gate + out.  This warp: outputs half * W / 2
-    // on, lane group og a quarter of them.
+    // input = next slice * next gate + out.  This warp: outputs half * W / 2 on.
     template <int W, bool WIDEN>
-    MRP_D void main_block(const float* w, int b, int c, int half, int pg, int og) {
-        constexpr int NO = W / 8;
-        const int o = half * (W / 2) + og * NO;
-        Acc<H, NO> acc;
+    MRP_D void main_block(const float* w, int b, int c, int half, int lane) {   // W = 8, 16
+        constexpr int NO = W * H / 8;
+        const int pg = lane % (8 * H), o = half * (W / 2) + lane / (8 * H) * NO;
+        Acc<1, NO> acc;
         acc.bias(main_bias_at(b) + c * W + o);
         acc.template mul<W>(act(32 * c) + 4 * pg, T, w + c * W * W + o, W);
         group_sync(c);   // both halves have read the inputs
-        main_step<NO, W, WIDEN, false>(acc, b, c, o, pg);
+        main_step<1, NO, W, WIDEN, false>(acc, b, c, o, pg);
         group_sync(c);
     }
-    template <int NO, int W, bool WIDEN, bool LAST>
-    MRP_D void main_step(const Acc<H, NO>& acc, int b, int c, int o, int pg) {
-        Px<H> x[NO], y[NO], z[NO], g;
-        Source::template region<H, NO>(region(b, c), slice_row(b) + o, pg, x);
+    template <int G, int NO, int W, bool WIDEN, bool LAST>
+    MRP_D void main_step(const Acc<G, NO>& acc, int b, int c, int o, int pg) {
+        Px<G> x[NO], y[NO], z[NO], g;
+        Source::template region<H, G, NO>(region(b, c), slice_row(b) + o, pg, x);
         if (!LAST) {
-            Source::template region<H, NO>(region(b + 1, c), slice_row(b + 1) + o, pg, y);
-            if (WIDEN) Source::template region<H, NO>(region(b + 1, c), slice_row(b + 1) + W + o, pg, z);
-            g = ldp<H>(sm + L::kGates + (3 * (b + 1) + c) * T, pg);
+            Source::template region<H, G, NO>(region(b + 1, c), slice_row(b + 1) + o, pg, y);
+            if (WIDEN) Source::template region<H, G, NO>(region(b + 1, c), slice_row(b + 1) + W + o, pg, z);
+            g = ldp<G>(sm + L::kGates + (3 * (b + 1) + c) * T, pg);
         }
 #pragma unroll
         for (int n = 0; n < NO; ++n) {
-            Px<H> a = acc.out(n), e;
+            Px<G> a = acc.out(n), e;
 #pragma unroll
-            for (int p = 0; p < 4 * H; ++p) {
+            for (int p = 0; p < 4 * G; ++p) {
                 if (!WIDEN) a.v[p] = a.v[p] + x[n].v[p];
                 if (!LAST) a.v[p] = fmaf(y[n].v[p], g.v[p], a.v[p]);
                 if (WIDEN) e.v[p] = fmaf(z[n].v[p], g.v[p], x[n].v[p]);
             }
-            stp<H>(act(32 * c + o + n), pg, a);
-            if (WIDEN) stp<H>(act(32 * c + W + o + n), pg, e);
+            stp<G>(act(32 * c + o + n), pg, a);
+            if (WIDEN) stp<G>(act(32 * c + W + o + n), pg, e);
         }
     }
     // A layer of the direct-illumination chain (b = 4: the finals): two warps,
     // four of the eight outputs of every channel each; rows 96 + 8 c.
     template <bool LAST>
-    MRP_D void di_layer(const Source& src, int r0, const float* w, int b, int half, int pg, int og) {
-        const int o = 4 * half + og;
-        Acc<H, 1> acc[3];
+    MRP_D void di_layer(const Source& src, int r0, const float* w, int b, int half, int lane) {
+        const int pg = lane % (8 * H), o = 4 * half + lane / (8 * H) * H;
+        Acc<1, H> acc[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             acc[c].bias(kBDi + 24 * b + 8 * c + o);
@@ -498,19 +504,23 @@ struct Net {
         group_sync(3);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            Px<H> a = acc[c].out(0);
-            if (b < 4) {
-                const Px<H> x = src.template sample<H>(r0, pg, c * 192 + 160 + 8 * b + o);
+            Px<1> g;
+            if (b < 4 && !LAST) g = ldp<1>(sm + L::kGates + (3 * (9 + b) + c) * T, pg);
 #pragma unroll
-                for (int p = 0; p < 4 * H; ++p) a.v[p] = a.v[p] + x.v[p];
-                if (!LAST) {
-                    const Px<H> y = src.template sample<H>(r0, pg, c * 192 + 168 + 8 * b + o),
-                                g = ldp<H>(sm + L::kGates + (3 * (9 + b) + c) * T, pg);
+            for (int n = 0; n < H; ++n) {
+                Px<1> a = acc[c].out(n);
+                if (b < 4) {
+                    const Px<1> x = src.template sample<1>(r0, pg, c * 192 + 160 + 8 * b + o + n);
 #pragma unroll
-                    for (int p = 0; p < 4 * H; ++p) a.v[p] = fmaf(y.v[p], g.v[p], a.v[p]);
+                    for (int p = 0; p < 4; ++p) a.v[p] = a.v[p] + x.v[p];
+                    if (!LAST) {
+                        const Px<1> y = src.template sample<1>(r0, pg, c * 192 + 168 + 8 * b + o + n);
+#pragma unroll
+                        for (int p = 0; p < 4; ++p) a.v[p] = fmaf(y.v[p], g.v[p], a.v[p]);
+                    }
                 }
+                stp<1>(act(96 + 8 * c + o + n), pg, a);
             }
-            stp<H>(act(96 + 8 * c + o), pg, a);
         }
         group_sync(3);
     }
@@ -523,12 +533,12 @@ struct Net {
         const float* w = next(kCB2);
         if (main) {
             Px<H> x[1];
-            Source::template region<H, 1>(region(0, c), 4 * half + og, pg, x);
+            Source::template region<H, H, 1>(region(0, c), 4 * half + og, pg, x);
             gated(x[0], ldp<H>(sm + L::kGates + c * T, pg));
             stp<H>(act(32 * c + 4 * half + og), pg, x[0]);
             group_sync(c);
-            main_block<8, false>(w, 0, c, half, pg, og);
-            main_block<8, true>(w + 192, 1, c, half, pg, og);
+            main_block<8, false>(w, 0, c, half, lane);
+            main_block<8, true>(w + 192, 1, c, half, lane);
         } else {
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
@@ -537,23 +547,23 @@ struct Net {
                 stp<H>(act(96 + 8 * d + 4 * half + og), pg, x);
             }
             group_sync(3);
-            di_layer<false>(src, r0, w + kHeadDi, 0, half, pg, og);
+            di_layer<false>(src, r0, w + kHeadDi, 0, half, lane);
         }
         w = next(kCB4);
         if (main) {
-            main_block<16, false>(w, 2, c, half, pg, og);
+            main_block<16, false>(w, 2, c, half, lane);
             stage_next(src, r0, 5, c, half, lane);   // region 0: slice 2 was its last
-            main_block<16, false>(w + 768, 3, c, half, pg, og);
+            main_block<16, false>(w + 768, 3, c, half, lane);
         } else {
-            di_layer<false>(src, r0, w + kB2Di, 1, half, pg, og);
+            di_layer<false>(src, r0, w + kB2Di, 1, half, lane);
         }
         w = next(kCB5);
         if (main) {
-            main_block<16, true>(w, 4, c, half, pg, og);
+            main_block<16, true>(w, 4, c, half, lane);
             stage_next(src, r0, 6, c, half, lane);
         } else {
-            di_layer<false>(src, r0, w + kB4Di, 2, half, pg, og);
-            di_layer<true>(src, r0, w + kB4Di + 192, 3, half, pg, og);
+            di_layer<false>(src, r0, w + kB4Di, 2, half, lane);
+            di_layer<true>(src, r0, w + kB4Di + 192, 3, half, lane);
         }
         const int o = half * 16 + og * 4;
 #pragma unroll 1
@@ -565,18 +575,18 @@ struct Net {
                 acc.bias(main_bias_at(b) + c * 32 + o);
                 acc.template mul<16>(a, T, w + c * 512 + o, 32);
             } else if (b == 5) {
-                di_layer<true>(src, r0, w + kB5Di, 4, half, pg, og);
+                di_layer<true>(src, r0, w + kB5Di, 4, half, lane);
             }
             w = next(kCB5 + 2 * (b - 5) + 2);   // after the last: kCLC0
             if (main) {
                 acc.template mul<16>(a + 16 * T, T, w + c * 512 + o, 32);
                 group_sync(c);
                 if (b < 7) {
-                    main_step<4, 32, false, false>(acc, b, c, o, pg);
+                    main_step<H, 4, 32, false, false>(acc, b, c, o, pg);
                     group_sync(c);
                     if (b == 5) stage_next(src, r0, 7, c, half, lane);
                 } else if (b == 7) {
-                    main_step<4, 32, false, true>(acc, b, c, o, pg);
+                    main_step<H, 4, 32, false, true>(acc, b, c, o, pg);
                 } else {
                     store(acc, act(32 * c + o), pg);
                 }
@@ -584,10 +594,10 @@ struct Net {
         }
     }
     static_assert(kCFinal == kCB5 + 6 && kCLC0 == kCFinal + 2 && main_bias(7) + 96 == kBFinal, "chunk order");
-    template <int NO>
-    MRP_D void store(const Acc<H, NO>& acc, float* dst, int pg) const {
+    template <int G, int NO>
+    MRP_D void store(const Acc<G, NO>& acc, float* dst, int pg) const {
 #pragma unroll
-        for (int n = 0; n < NO; ++n) stp<H>(dst + n * T, pg, acc.out(n));
+        for (int n = 0; n < NO; ++n) stp<G>(dst + n * T, pg, acc.out(n));
     }
 
     // ---- pools, gates, LSEFin1 ---------------------------------------------
@@ -712,8 +722,8 @@ struct Net {
             for (int c = 0; c < 3; ++c) o[c] = fmaxf(expf(P[c]) - 1.0f, 0.0f) * powf(srv[c], 4.0f);
             sink.put(r, o);
         }
-        // (the next tile's pools overwrite activations that were last read
-        // before the hand-over of the tail's last chunk)
+        // (the next tile's pools overwrite rows 0..73, last read before the
+        // hand-over of the tail's last chunk)
     }
     // The tail of one albedo channel; thread t < T returns pixel t's output.
     MRP_D float tail(float s4, float g, const Vec<H>& gam, int warp, int lane, int after) {
@@ -774,78 +784,78 @@ struct Net {
             __syncthreads();
             store(acc, dst + (16 * warp + 4 * og) * T, pg);
         }
+        const int qg = lane % (8 * H), qo = lane / (8 * H);   // the narrow layers' pixels and outputs
         {
-            Acc<H, 2> acc;
-            acc.bias(kBLC1 + 8 * warp + 2 * og);
+            Acc<1, 2 * H> acc;
+            const int o = 8 * warp + 2 * H * qo;
+            acc.bias(kBLC1 + o);
 #pragma unroll 1
             for (int k = 0; k < 4; ++k) {
                 w = next(kCLC1 + k + 1);   // after the last: kCLC2
-                acc.template mul<32>(in + 32 * k * T, T, w + 8 * warp + 2 * og, 64);
+                acc.template mul<32>(dst + 4 * qg + 32 * k * T, T, w + o, 64);
             }
             __syncthreads();
-            store(acc, dst + (8 * warp + 2 * og) * T, pg);
+            store(acc, dst + o * T, qg);
         }
         {
-            Acc<H, 1> acc;
-            acc.bias(kBLC2 + 4 * warp + og);
+            Acc<1, H> acc;
+            const int o = 4 * warp + H * qo;
+            acc.bias(kBLC2 + o);
             w = next(kCRes0);
-            acc.template mul<64>(in, T, w + 4 * warp + og, 32);
+            acc.template mul<64>(dst + 4 * qg, T, w + o, 32);
             __syncthreads();
-            store(acc, dst + (4 * warp + og) * T, pg);
+            store(acc, dst + o * T, qg);
         }
-        // LX and the six residual pairs: one pixel a thread, in registers
+        // LX (rows 0..31 -> 96..111) and the six residual pairs (96..111 ->
+        // 112..127 -> 96..111): 32 pixels a warp, 4 pixels x 4 outputs a
+        // thread, whose own four sums stay in registers (rows that the next
+        // tile's pools, which other warps may have begun, leave alone)
         float P = 0.0f;
         w = next(kCRes1);
-        const bool mine = (int)threadIdx.x < T;
-        float a16[16];
+        const bool mine = warp < H;
+        float* col = dst + 32 * warp;   // this warp's pixels (mine)
+        Px<1> a[4];
         if (mine) {
-            u64 s[8];
+            Acc<1, 4> acc;
+            acc.bias(kBLX + 4 * og);
+            acc.template mul<32>(col + 4 * pg, T, w + 4 * og, 16);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) s[j] = pair(c_con[kBLX + 2 * j], c_con[kBLX + 2 * j + 1]);
-#pragma unroll
-            for (int k = 0; k < 32; ++k) {
-                const float x = dst[k * T + threadIdx.x];
-                dense16(s, pair(x, x), w + 16 * k);
+            for (int n = 0; n < 4; ++n) {
+                a[n] = acc.out(n);
+                stp<1>(col + (96 + 4 * og + n) * T, pg, a[n]);
             }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) { a16[2 * j] = relu(lo_of(s[j])); a16[2 * j + 1] = relu(hi_of(s[j])); }
+            __syncwarp();
 #pragma unroll 1
-            for (int k = 0; k < 3; ++k) residual(a16, w + 512 + 512 * k, kBRes + 32 * k);
+            for (int k = 0; k < 3; ++k) residual(a, col, w + 512 + 512 * k, kBRes + 32 * k, pg, og);
         }
         w = next(after);
         if (mine) {
 #pragma unroll 1
-            for (int k = 0; k < 3; ++k) residual(a16, w + 512 * k, kBRes + 96 + 32 * k);
-            float a = 0.0f;
+            for (int k = 0; k < 3; ++k) residual(a, col, w + 512 * k, kBRes + 96 + 32 * k, pg, og);
+            float p = 0.0f;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) a = fmaf(a16[j], c_con[kHeadW + j], a);
-            P = relu(a + c_con[kHeadB]);
+            for (int j = 0; j < 16; ++j) p = fmaf(col[(96 + j) * T + lane], c_con[kHeadW + j], p);
+            P = relu(p + c_con[kHeadB]);
         }
         return P;
     }
-    static MRP_D void dense16(u64 (&s)[8], u64 x, const float* w) {   // one input of a 16-output layer
+    static MRP_D void residual(Px<1> (&a)[4], float* col, const float* w, int b, int pg, int og) {
+        Acc<1, 4> y, z;
+        y.bias(b + 4 * og);
+        y.template mul<16>(col + 96 * T + 4 * pg, T, w + 4 * og, 16);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(w + 4 * j);
-            s[2 * j] = fma2(x, v.x, s[2 * j]);
-            s[2 * j + 1] = fma2(x, v.y, s[2 * j + 1]);
+        for (int n = 0; n < 4; ++n) stp<1>(col + (112 + 4 * og + n) * T, pg, y.out(n));
+        __syncwarp();
+        z.bias(b + 16 + 4 * og);
+        z.template mul<16>(col + 112 * T + 4 * pg, T, w + 256 + 4 * og, 16);
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const Px<1> o = z.out(n);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) a[n].v[p] += o.v[p];
+            stp<1>(col + (96 + 4 * og + n) * T, pg, a[n]);
         }
-    }
-    static MRP_D void layer16(const float (&in)[16], float (&out)[16], const float* w, int b) {
-        u64 s[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s[j] = pair(c_con[b + 2 * j], c_con[b + 2 * j + 1]);
-#pragma unroll
-        for (int k = 0; k < 16; ++k) dense16(s, pair(in[k], in[k]), w + 16 * k);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) { out[2 * j] = relu(lo_of(s[j])); out[2 * j + 1] = relu(hi_of(s[j])); }
-    }
-    static MRP_D void residual(float (&a)[16], const float* w, int b) {
-        float y[16], z[16];
-        layer16(a, y, w, b);
-        layer16(y, z, w + 256, b + 16);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) a[i] += z[i];
+        __syncwarp();
     }
 };
 
