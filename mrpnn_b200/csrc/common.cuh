@@ -28,6 +28,31 @@ MRP_D float fm(float a, float b) { return __fmul_rn(a, b); }
 MRP_D float fd(float a, float b) { return __fdiv_rn(a, b); }
 MRP_D float fsq(float a) { return __fsqrt_rn(a); }
 
+// Two IEEE operations at once on register pairs (f32x2): each half rounds as
+// the scalar operation does.
+typedef unsigned long long f32x2;
+MRP_D f32x2 pk2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+MRP_D void upk2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+MRP_D f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+MRP_D f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+MRP_D f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 struct f3 { float x, y, z; };
 MRP_HD f3 mk3(float x, float y, float z) { return {x, y, z}; }
 MRP_D f3 add(f3 a, f3 b) { return {fa(a.x, b.x), fa(a.y, b.y), fa(a.z, b.z)}; }
@@ -175,7 +200,12 @@ MRP_D float fetch_clamp(const float* __restrict__ g, int n, int x, int y, int z)
     return __ldg(g + ((size_t)x * n + y) * n + z);
 }
 // lerp with 1 - v computed once by the caller (same operations, same result).
-MRP_D float lerp_w(float a, float b, float v, float omv) { return fa(fm(a, omv), fm(b, v)); }
+MRP_D float lerp_w(float a, float b, float v, float omv) {
+    // (both products in one instruction, each rounded as fm rounds it)
+    float lo, hi;
+    upk2(mul2(pk2(a, b), pk2(omv, v)), lo, hi);
+    return fa(lo, hi);
+}
 // Trilinear fetch.  The eight texels come from per-axis clamped coordinates
 // (so every load is in bounds); border mode then zeroes the texels whose
 // unclamped coordinate lies outside [0, n).  Values and the order of the
@@ -225,6 +255,27 @@ MRP_D float tex3(const T* __restrict__ g, int n, f3 pos) {
 // and lerp arithmetic.  The march keeps the exact forms above -- its
 // accept / stop decisions must match the reference's float order.
 MRP_D float lerp_fast(float a, float b, float v) { return fmaf(v, b - a, a); }
+// the same of two values at once (a * -1 + b is b - a, rounded once)
+MRP_D f32x2 lerp_fast2(f32x2 a, f32x2 b, f32x2 v) { return fma2(v, fma2(a, pk2(-1.0f, -1.0f), b), a); }
+// Trilinear lerps of eight texels, the four along z and the two along y in pairs.
+MRP_D float lerps_fast(float t000, float t001, float t010, float t011, float t100, float t101, float t110, float t111,
+                       float wx, float wy, float wz) {
+    const f32x2 z2 = pk2(wz, wz);
+    const f32x2 c0 = lerp_fast2(pk2(t000, t100), pk2(t001, t101), z2), c1 = lerp_fast2(pk2(t010, t110), pk2(t011, t111), z2);
+    float a, b;
+    upk2(lerp_fast2(c0, c1, pk2(wy, wy)), a, b);
+    return lerp_fast(a, b, wx);
+}
+// Eight texel pairs: both channels at once.
+MRP_D void lerps_pair(const float2 (&t)[8], float wx, float wy, float wz, float* a, float* b) {
+    f32x2 q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = pk2(t[i].x, t[i].y);
+    const f32x2 x2 = pk2(wx, wx), y2 = pk2(wy, wy), z2 = pk2(wz, wz);
+    const f32x2 c00 = lerp_fast2(q[0], q[1], z2), c01 = lerp_fast2(q[2], q[3], z2);
+    const f32x2 c10 = lerp_fast2(q[4], q[5], z2), c11 = lerp_fast2(q[6], q[7], z2);
+    upk2(lerp_fast2(lerp_fast2(c00, c01, y2), lerp_fast2(c10, c11, y2), x2), *a, *b);
+}
 // n^3 must stay below 2^31 (the pyramid and TR levels: n <= 256): 32-bit
 // offsets.  Footprints inside the grid (the common case) skip the clamps and
 // the border selects.
@@ -248,9 +299,7 @@ MRP_D float tex3_padded(const float* __restrict__ g, int n, f3 pos) {
     const int PP = P * P;
     const float t000 = __ldg(b), t001 = __ldg(b + 1), t010 = __ldg(b + P), t011 = __ldg(b + P + 1);
     const float t100 = __ldg(b + PP), t101 = __ldg(b + PP + 1), t110 = __ldg(b + PP + P), t111 = __ldg(b + PP + P + 1);
-    const float c00 = lerp_fast(t000, t001, wz), c01 = lerp_fast(t010, t011, wz);
-    const float c10 = lerp_fast(t100, t101, wz), c11 = lerp_fast(t110, t111, wz);
-    return lerp_fast(lerp_fast(c00, c01, wy), lerp_fast(c10, c11, wy), wx);
+    return lerps_fast(t000, t001, t010, t011, t100, t101, t110, t111, wx, wy, wz);
 }
 
 // Two trilinear fetches at one position from texel pairs (mip_tr): the
@@ -267,18 +316,9 @@ MRP_D bool tex3_pair_interior(const float2* __restrict__ g, int n, f3 pos, float
     float wx = px - flx, wy = py - fly, wz = pz - flz;
     const int nn = n * n;
     const float2* q = g + (x * n + y) * n + z;
-    const float2 t000 = __ldg(q), t001 = __ldg(q + 1), t010 = __ldg(q + n), t011 = __ldg(q + n + 1);
-    const float2 t100 = __ldg(q + nn), t101 = __ldg(q + nn + 1), t110 = __ldg(q + nn + n), t111 = __ldg(q + nn + n + 1);
-    {
-        float c00 = lerp_fast(t000.x, t001.x, wz), c01 = lerp_fast(t010.x, t011.x, wz);
-        float c10 = lerp_fast(t100.x, t101.x, wz), c11 = lerp_fast(t110.x, t111.x, wz);
-        *a = lerp_fast(lerp_fast(c00, c01, wy), lerp_fast(c10, c11, wy), wx);
-    }
-    {
-        float c00 = lerp_fast(t000.y, t001.y, wz), c01 = lerp_fast(t010.y, t011.y, wz);
-        float c10 = lerp_fast(t100.y, t101.y, wz), c11 = lerp_fast(t110.y, t111.y, wz);
-        *b = lerp_fast(lerp_fast(c00, c01, wy), lerp_fast(c10, c11, wy), wx);
-    }
+    const float2 t[8] = {__ldg(q), __ldg(q + 1), __ldg(q + n), __ldg(q + n + 1),
+                         __ldg(q + nn), __ldg(q + nn + 1), __ldg(q + nn + n), __ldg(q + nn + n + 1)};
+    lerps_pair(t, wx, wy, wz, a, b);
     return true;
 }
 
@@ -295,18 +335,9 @@ MRP_D void tex3_padded_pair(const float2* __restrict__ g, int n, f3 pos, float* 
     const float wx = px - flx, wy = py - fly, wz = pz - flz;
     const float2* q = g + (x * P + y) * P + z;
     const int PP = P * P;
-    const float2 t000 = __ldg(q), t001 = __ldg(q + 1), t010 = __ldg(q + P), t011 = __ldg(q + P + 1);
-    const float2 t100 = __ldg(q + PP), t101 = __ldg(q + PP + 1), t110 = __ldg(q + PP + P), t111 = __ldg(q + PP + P + 1);
-    {
-        float c00 = lerp_fast(t000.x, t001.x, wz), c01 = lerp_fast(t010.x, t011.x, wz);
-        float c10 = lerp_fast(t100.x, t101.x, wz), c11 = lerp_fast(t110.x, t111.x, wz);
-        *a = lerp_fast(lerp_fast(c00, c01, wy), lerp_fast(c10, c11, wy), wx);
-    }
-    {
-        float c00 = lerp_fast(t000.y, t001.y, wz), c01 = lerp_fast(t010.y, t011.y, wz);
-        float c10 = lerp_fast(t100.y, t101.y, wz), c11 = lerp_fast(t110.y, t111.y, wz);
-        *b = lerp_fast(lerp_fast(c00, c01, wy), lerp_fast(c10, c11, wy), wx);
-    }
+    const float2 t[8] = {__ldg(q), __ldg(q + 1), __ldg(q + P), __ldg(q + P + 1),
+                         __ldg(q + PP), __ldg(q + PP + 1), __ldg(q + PP + P), __ldg(q + PP + P + 1)};
+    lerps_pair(t, wx, wy, wz, a, b);
 }
 
 // tex3_fast's footprints that touch the grid's edge: clamped texels, and
@@ -332,9 +363,7 @@ __device__ __noinline__ float tex3_edge(const float* __restrict__ g, int n, int 
         t100 = vx1 && vy0 && vz0 ? t100 : 0.0f; t101 = vx1 && vy0 && vz1 ? t101 : 0.0f;
         t110 = vx1 && vy1 && vz0 ? t110 : 0.0f; t111 = vx1 && vy1 && vz1 ? t111 : 0.0f;
     }
-    float c00 = lerp_fast(t000, t001, wz), c01 = lerp_fast(t010, t011, wz);
-    float c10 = lerp_fast(t100, t101, wz), c11 = lerp_fast(t110, t111, wz);
-    return lerp_fast(lerp_fast(c00, c01, wy), lerp_fast(c10, c11, wy), wx);
+    return lerps_fast(t000, t001, t010, t011, t100, t101, t110, t111, wx, wy, wz);
 }
 template <bool Clamp>
 MRP_D float tex3_fast(const float* __restrict__ g, int n, f3 pos) {
@@ -349,9 +378,7 @@ MRP_D float tex3_fast(const float* __restrict__ g, int n, f3 pos) {
     const float* b = g + (x * n + y) * n + z;
     const float t000 = __ldg(b), t001 = __ldg(b + 1), t010 = __ldg(b + n), t011 = __ldg(b + n + 1);
     const float t100 = __ldg(b + nn), t101 = __ldg(b + nn + 1), t110 = __ldg(b + nn + n), t111 = __ldg(b + nn + n + 1);
-    float c00 = lerp_fast(t000, t001, wz), c01 = lerp_fast(t010, t011, wz);
-    float c10 = lerp_fast(t100, t101, wz), c11 = lerp_fast(t110, t111, wz);
-    return lerp_fast(lerp_fast(c00, c01, wy), lerp_fast(c10, c11, wy), wx);
+    return lerps_fast(t000, t001, t010, t011, t100, t101, t110, t111, wx, wy, wz);
 }
 
 constexpr int kLut = 512;

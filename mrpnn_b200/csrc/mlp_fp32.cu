@@ -122,19 +122,8 @@ cudaError_t fp32_prepare_weights(const float* w, float* d_out) {
 
 namespace {
 
-typedef unsigned long long u64;
-MRP_D u64 pair(float lo, float hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-MRP_D float lo_of(u64 v) { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return a; }
-MRP_D float hi_of(u64 v) { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return b; }
-MRP_D u64 fma2(u64 a, u64 b, u64 c) {   // two IEEE fused multiply-adds
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
+MRP_D float lo_of(f32x2 v) { float a, b; upk2(v, a, b); return a; }
+MRP_D float hi_of(f32x2 v) { float a, b; upk2(v, a, b); return b; }
 MRP_D float relu(float a) { return a >= 0.0f ? a : 0.0f; }
 MRP_D float sigmoid_ref(float o) { return (float)(1.0 / (1.0 + (double)expf(-o))); }
 MRP_D void cp16(float* dst, const float* src, int bytes) {   // bytes: 16, or 0 for zeros
@@ -186,13 +175,13 @@ MRP_D void stp(float* row, int pg, const Px<H>& r) {
 // NO outputs of a thread's pixels, two pixels to a register pair.
 template <int H, int NO>
 struct Acc {
-    u64 a[NO][2 * H];
+    f32x2 a[NO][2 * H];
     MRP_D void bias(int at) {
 #pragma unroll
         for (int n = 0; n < NO; ++n) {
             const float b = c_con[at + n];
 #pragma unroll
-            for (int p = 0; p < 2 * H; ++p) a[n][p] = pair(b, b);
+            for (int p = 0; p < 2 * H; ++p) a[n][p] = pk2(b, b);
         }
     }
     MRP_D Px<H> out(int n) const {   // relu of output n
@@ -207,7 +196,7 @@ struct Acc {
     MRP_D void mul(const float* s, int T, const float* w, int R) {
 #pragma unroll 8
         for (int k = 0; k < K; ++k) {
-            u64 x[2 * H];
+            f32x2 x[2 * H];
 #pragma unroll
             for (int h = 0; h < H; ++h) {
                 const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(s + k * T + 32 * h);
@@ -219,7 +208,7 @@ struct Acc {
             else wk[0] = w[k * R];
 #pragma unroll
             for (int n = 0; n < NO; ++n) {
-                const u64 ww = pair(wk[n], wk[n]);
+                const f32x2 ww = pk2(wk[n], wk[n]);
 #pragma unroll
                 for (int p = 0; p < 2 * H; ++p) a[n][p] = fma2(x[p], ww, a[n][p]);
             }

@@ -386,21 +386,11 @@ MRP_D float lds1(const float* p) {
     return v;
 }
 
-// Two IEEE operations at once on register pairs (element-wise work is what
-// the threads of a row spend their instructions on).
-typedef unsigned long long u64;
-MRP_D u64 pk(float lo, float hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-MRP_D void upk(u64 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-MRP_D u64 fma2(u64 a, u64 b, u64 c) { u64 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
-MRP_D u64 add2(u64 a, u64 b) { u64 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-MRP_D u64 mul2(u64 a, u64 b) { u64 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-MRP_D void add_to(float& a0, float& a1, float b0, float b1) { upk(add2(pk(a0, a1), pk(b0, b1)), a0, a1); }
+// Element-wise work, which is what the threads of a row spend their
+// instructions on, runs in register pairs.
+MRP_D void add_to(float& a0, float& a1, float b0, float b1) { upk2(add2(pk2(a0, a1), pk2(b0, b1)), a0, a1); }
 // a = x * g + a
-MRP_D void fma_to(float& a0, float& a1, float x0, float x1, u64 g) { upk(fma2(pk(x0, x1), g, pk(a0, a1)), a0, a1); }
+MRP_D void fma_to(float& a0, float& a1, float x0, float x1, f32x2 g) { upk2(fma2(pk2(x0, x1), g, pk2(a0, a1)), a0, a1); }
 
 // Biases and scales start on 16-float boundaries (scale_off), so they are
 // read four at a time.  OFF: first output of the part at hand.
@@ -411,18 +401,18 @@ MRP_D void bias_relu(float* d, int L, float rs, const float* aux) {
 #pragma unroll
     for (int q = 0; q < N / 4; ++q) {
         const float4 b = lds4(aux + ab + 4 * q);
-        u64 lo = pk(d[4 * q], d[4 * q + 1]), hi = pk(d[4 * q + 2], d[4 * q + 3]);
+        f32x2 lo = pk2(d[4 * q], d[4 * q + 1]), hi = pk2(d[4 * q + 2], d[4 * q + 3]);
         if (EB == 1) {
             const float4 w = lds4(aux + kAuxScale + so + 4 * q);
-            const u64 r2 = pk(rs, rs);
-            lo = fma2(lo, mul2(r2, pk(w.x, w.y)), pk(b.x, b.y));
-            hi = fma2(hi, mul2(r2, pk(w.z, w.w)), pk(b.z, b.w));
+            const f32x2 r2 = pk2(rs, rs);
+            lo = fma2(lo, mul2(r2, pk2(w.x, w.y)), pk2(b.x, b.y));
+            hi = fma2(hi, mul2(r2, pk2(w.z, w.w)), pk2(b.z, b.w));
         } else {
-            lo = add2(lo, pk(b.x, b.y));
-            hi = add2(hi, pk(b.z, b.w));
+            lo = add2(lo, pk2(b.x, b.y));
+            hi = add2(hi, pk2(b.z, b.w));
         }
-        upk(lo, d[4 * q], d[4 * q + 1]);
-        upk(hi, d[4 * q + 2], d[4 * q + 3]);
+        upk2(lo, d[4 * q], d[4 * q + 1]);
+        upk2(hi, d[4 * q + 2], d[4 * q + 3]);
 #pragma unroll
         for (int i = 0; i < 4; ++i) d[4 * q + i] = fmaxf(d[4 * q + i], 0.0f);
     }
@@ -565,7 +555,7 @@ __device__ __noinline__ int tc_block(const Group G, int st, const Src src, const
         tmem_get<16>(G, kColHf, hf);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const u64 av = pk(p8[c], p8[c]), mx = pk(p8[3 + c], p8[3 + c]);
+            const f32x2 av = pk2(p8[c], p8[c]), mx = pk2(p8[3 + c], p8[3 + c]);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const float4 wa = lds4(aux + kAuxLSE1 + 16 * (bd.pid + c) + 4 * q);
@@ -578,7 +568,7 @@ __device__ __noinline__ int tc_block(const Group G, int st, const Src src, const
         }
         tmem_put<16>(G, kColHf, hf);
     }
-    u64 gate[3];
+    f32x2 gate[3];
     {
         float h[8], a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
@@ -586,7 +576,7 @@ __device__ __noinline__ int tc_block(const Group G, int st, const Src src, const
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const float4 u = lds4(aux + bd.se_off + 8 * j), v = lds4(aux + bd.se_off + 8 * j + 4);
-            const u64 p = pk(p8[j], p8[j]);
+            const f32x2 p = pk2(p8[j], p8[j]);
             fma_to(h[0], h[1], u.x, u.y, p);
             fma_to(h[2], h[3], u.z, u.w, p);
             fma_to(h[4], h[5], v.x, v.y, p);
@@ -596,13 +586,13 @@ __device__ __noinline__ int tc_block(const Group G, int st, const Src src, const
         for (int j = 0; j < 8; ++j) {
             const float4 u = lds4(aux + bd.se_off + 64 + 4 * j);
             h[j] = fmaxf(h[j], 0.0f);
-            fma_to(a[0], a[1], u.x, u.y, pk(h[j], h[j]));
+            fma_to(a[0], a[1], u.x, u.y, pk2(h[j], h[j]));
             a[2] = fmaf(h[j], u.z, a[2]);
         }
 #pragma unroll
         for (int o = 0; o < 3; ++o) {
             const float q = sigmoid_d(a[o]);
-            gate[o] = pk(q, q);
+            gate[o] = pk2(q, q);
         }
     }
     float rs[3];
@@ -615,7 +605,7 @@ __device__ __noinline__ int tc_block(const Group G, int st, const Src src, const
             for (int i = 0; i < W; i += 2) fma_to(in[i], in[i + 1], xs[c][i], xs[c][i + 1], gate[c]);
         } else {
 #pragma unroll
-            for (int i = 0; i < W; i += 2) upk(mul2(pk(xs[c][i], xs[c][i + 1]), gate[c]), in[i], in[i + 1]);
+            for (int i = 0; i < W; i += 2) upk2(mul2(pk2(xs[c][i], xs[c][i + 1]), gate[c]), in[i], in[i + 1]);
         }
         rs[c] = write_row<EB, W, KP>(G.a_s, c * SUB, G.t, in);
     }
@@ -728,9 +718,9 @@ __device__ __noinline__ TailOut tc_tail(const Group G, int st, const float* aux,
     float r = write_parts<EB, 128>(G, [&](int p, float (&v)[32]) {
         if (p < 3) {
             tmem_get<32>(G, kColComb<COL> + 32 * p, v);
-            const u64 q = pk(gf[p], gf[p]);
+            const f32x2 q = pk2(gf[p], gf[p]);
 #pragma unroll
-            for (int i = 0; i < 32; i += 2) upk(mul2(pk(v[i], v[i + 1]), q), v[i], v[i + 1]);
+            for (int i = 0; i < 32; i += 2) upk2(mul2(pk2(v[i], v[i + 1]), q), v[i], v[i + 1]);
         } else {
             float e[24];
             tmem_get<16>(G, kColComb<COL> + 96, e);
