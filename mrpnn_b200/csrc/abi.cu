@@ -290,17 +290,17 @@ mrp_status mrp_volume_create_ex(int res, mrp_storage storage, mrp_volume** out) 
                  nrow = std::max(occ_row_words(res), kMipOccRows);
     if ((storage == MRP_STORAGE_FP16 ? (e = mrp::dev_malloc(&v->density_h, n * sizeof(__half)))
                                      : (e = mrp::dev_malloc(&v->density, n * sizeof(float)))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->mips, (kMipFloats + kTrPadFloats + kPadLevelFloats) * sizeof(float))) != cudaSuccess ||
+        (e = mrp::dev_malloc(&v->mips, (kMipFloats + kPadLevelFloats) * sizeof(float))) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->trs, (kTrFloats + kPadLevelFloats) * sizeof(float))) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->lut, kLutAlloc * sizeof(float))) != cudaSuccess ||
         (e = mrp::dev_malloc(&v->occ_rows, nrow * sizeof(uint4) + 32 + kMipOccBytes + nocc + nocc2)) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->mip_tr, (mip_tr_offset(5) + kPadLevelFloats) * sizeof(float2))) != cudaSuccess)
+        (e = mrp::dev_malloc(&v->mip_tr, (mip_tr_offset(5) + kTrPadTexels + kPadLevelFloats) * sizeof(float2))) != cudaSuccess)
         return cleanup(fail(e == cudaErrorMemoryAllocation ? MRP_ERR_OOM : MRP_ERR_CUDA, "volume allocation: %s",
                             cudaGetErrorString(e)));
-    v->mips_tr = v->mips + kMipFloats;
-    v->mips_pad = v->mips_tr + kTrPadFloats;
+    v->mips_pad = v->mips + kMipFloats;
     v->trs_pad = v->trs + kTrFloats;
-    v->pad_pair = v->mip_tr + mip_tr_offset(5);
+    v->mips_tr = v->mip_tr + mip_tr_offset(5);
+    v->pad_pair = v->mips_tr + kTrPadTexels;
     v->d_stats = reinterpret_cast<int*>(v->occ_rows + nrow);
     v->mip_occ = reinterpret_cast<uint8_t*>(v->d_stats) + 32;
     v->occ = v->mip_occ + kMipOccBytes;

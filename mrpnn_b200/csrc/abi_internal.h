@@ -111,8 +111,8 @@ struct mrp_volume {
     uint8_t* occ2 = nullptr;      // coarse occupancy (4^3 bricks each), built with occ
     int occ2_res = 0;
     uint4* occ_rows = nullptr;    // scratch of the occupancy scans; d_stats, mip_occ, occ and occ2 follow it
-    // (mips_tr and mips_pad lie behind mips, trs_pad behind trs, pad_pair behind mip_tr)
-    float* mips_tr = nullptr;     // mips 1..8 with a border of zeros, built with the pyramid for the TR levels
+    // (mips_pad lies behind mips, trs_pad behind trs, mips_tr and pad_pair behind mip_tr)
+    float2* mips_tr = nullptr;    // mips 1..8 with a border of zeros, in z pairs, built with the pyramid for the TR levels
     float* mips_pad = nullptr;    // padded mips 5..7 (pad_offset layout), built with the pyramid
     float* trs_pad = nullptr;     // padded TR levels 4..6, built with the TR levels
     float2* mip_tr = nullptr;     // (mip L, TR L - 1) texel pairs, L = 1..4, built with the TR levels

@@ -401,7 +401,7 @@ MRP_HD size_t mip_offset(int m) { return (size_t)(((1u << 27) - (1u << (27 - 3 *
 MRP_HD size_t tr_offset(int m) { return (size_t)(((1u << 24) - (1u << (24 - 3 * m))) / 7u); }
 constexpr size_t kMipFloats = 19173961;   // sum_{m<9} (256>>m)^3
 constexpr size_t kTrFloats = 2396745;     // sum_{i<8} (128>>i)^3
-constexpr size_t kTrPadFloats = 2530939;  // sum_{i<8} ((128>>i) + 2)^3
+constexpr size_t kTrPadTexels = 2530939;  // sum_{i<8} ((128>>i) + 2)^3
 
 MRP_D float tex_lut_fast(const float* __restrict__ lut, float u, float v) {
     float px = fmaf(u, (float)kLut, -0.5f), py = fmaf(v, (float)kLut, -0.5f);

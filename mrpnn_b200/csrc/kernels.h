@@ -45,9 +45,9 @@ cudaError_t launch_interleave_mip_tr(const float* mips, const float* trs, float2
 // of edge 8, 4, 2; clamp: TR-level addressing, else border (density mips).
 cudaError_t launch_pad_levels(const float* l8, const float* l4, const float* l2, bool clamp, float* out,
                               cudaStream_t s);
-// Copies of mips 1..8 with a border of zeros (kTrPadFloats floats), which the
-// TR levels are marched through.
-cudaError_t launch_pad_pyramid(const float* mips, float* mips_tr, int sms, cudaStream_t s);
+// Copies of mips 1..8 with a border of zeros, a texel and its z neighbour side
+// by side (kTrPadTexels pairs), which the TR levels are marched through.
+cudaError_t launch_pad_pyramid(const float* mips, float2* mips_tr, int sms, cudaStream_t s);
 // The eight TR levels (trs: tr_offset layout) from the pyramid and its padded
 // copies; mip_occ may be null.
 struct TrArgs {
@@ -55,7 +55,7 @@ struct TrArgs {
     f3 L;             // toward the light
     f3 lo, hi;        // VolumeDev::nz_lo, nz_hi (anything that holds the cube when not known)
 };
-cudaError_t launch_tr_levels(float* trs, const float* mips, const float* mips_tr, const uint8_t* mip_occ,
+cudaError_t launch_tr_levels(float* trs, const float* mips, const float2* mips_tr, const uint8_t* mip_occ,
                              const TrArgs& args, cudaStream_t s);
 cudaError_t set_halton_permutations(const uint32_t perm[28]);
 cudaError_t launch_hg_lut(float* lut, float g, uint32_t seed, cudaStream_t s);
