@@ -62,7 +62,22 @@ __global__ void __launch_bounds__(256) k_fill_half(const __grid_constant__ FillT
     const int L = blockIdx.y, n = t.n[L];
     const float* __restrict__ src = t.src[L];
     const size_t total = t.flat[L] ? (size_t)n * n : (size_t)n * n * n;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    if (n % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+        // four texels of a row a thread: one 16-byte load, one 8-byte surface
+        // write (a 2-byte write per texel took 72 us for 256^3, this 29 us)
+        for (size_t q = first; q < total / 4; q += step) {
+            const size_t i = 4 * q;
+            const int z = (int)(i % n), y = (int)((i / n) % n), x = (int)(i / ((size_t)n * n));
+            const float4 f = __ldg(reinterpret_cast<const float4*>(src) + q);
+            const __half2 a = __floats2half2_rn(f.x, f.y), b = __floats2half2_rn(f.z, f.w);
+            const uint2 h = make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
+            if (t.flat[L]) surf2Dwrite(h, t.surf[L], z * 2, y);
+            else surf3Dwrite(h, t.surf[L], z * 2, y, x);
+        }
+        return;
+    }
+    for (size_t i = first; i < total; i += step) {
         const int z = (int)(i % n), y = (int)((i / n) % n), x = (int)(i / ((size_t)n * n));
         const unsigned short h = __half_as_ushort(__float2half_rn(__ldg(src + i)));
         if (t.flat[L]) surf2Dwrite(h, t.surf[L], z * (int)sizeof(h), y);
@@ -84,16 +99,21 @@ struct PairTable {
 __global__ void __launch_bounds__(256) k_fill_pairs(const __grid_constant__ PairTable t) {
     const int L = blockIdx.y, n = t.n[L], P = n + 2;
     if (n == 0) return;
-    const size_t total = (size_t)P * P * P;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const int zp = (int)(i % P), yp = (int)((i / P) % P), xp = (int)(i / ((size_t)P * P));
-        const int x = xp - 1, y = yp - 1, z = zp - 1;
-        const bool in = (unsigned)x < (unsigned)n && (unsigned)y < (unsigned)n && (unsigned)z < (unsigned)n;
-        const int cx = min(max(x, 0), n - 1), cy = min(max(y, 0), n - 1), cz = min(max(z, 0), n - 1);
-        const size_t c = ((size_t)cx * n + cy) * n + cz;
-        const float d = in ? __ldg(t.mip[L] + c) : 0.0f;
-        const __half2 h = __floats2half2_rn(d, __ldg(t.tr[L] + c));
-        surf3Dwrite(*reinterpret_cast<const unsigned*>(&h), t.surf[L], zp * 4, yp, xp);
+    const int total = P * P * P / 2;   // two texels a thread (P is even): an 8-byte surface write
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x) {
+        const int zp = 2 * (q % (P / 2)), yp = (q / (P / 2)) % P, xp = q / (P / 2 * P);
+        const int x = xp - 1, y = yp - 1, cx = min(max(x, 0), n - 1), cy = min(max(y, 0), n - 1);
+        const bool row_in = (unsigned)x < (unsigned)n && (unsigned)y < (unsigned)n;
+        const int row = (cx * n + cy) * n;
+        unsigned h[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int z = zp - 1 + e, c = row + min(max(z, 0), n - 1);
+            const float d = row_in && (unsigned)z < (unsigned)n ? __ldg(t.mip[L] + c) : 0.0f;
+            const __half2 v = __floats2half2_rn(d, __ldg(t.tr[L] + c));
+            h[e] = *reinterpret_cast<const unsigned*>(&v);
+        }
+        surf3Dwrite(make_uint2(h[0], h[1]), t.surf[L], zp * 4, yp, xp);
     }
 }
 }  // namespace
