@@ -231,6 +231,12 @@ struct LayerDesc {
     int soff;       // FP8 scale offset
 };
 __constant__ LayerDesc c_layer_desc[kLayers];
+// What issuing a layer's MMAs takes ([0] BF16, [1] E4M3): the weight image's
+// offset and the rows' group stride as the shared-memory descriptor holds
+// them (16-byte units), the instruction descriptor, the number of MMAs (32
+// bytes of K each).
+struct MmaDesc { uint32_t b_off, sbo, idesc, steps; };
+__constant__ uint4 c_mma_desc[2][kLayers];
 
 static void fill_layer_descs(LayerDesc* d) {
     for (int i = 0; i < kLayers; ++i) {
@@ -248,7 +254,16 @@ static void fill_layer_descs(LayerDesc* d) {
 static cudaError_t upload_layer_descs() {
     LayerDesc descs[kLayers];
     fill_layer_descs(descs);
-    return cudaMemcpyToSymbol(c_layer_desc, descs, sizeof descs);
+    MmaDesc mma[2][kLayers];
+    for (int e = 0; e < 2; ++e)
+        for (int i = 0; i < kLayers; ++i) {
+            const int eb = e == 0 ? 2 : 1, kb = descs[i].kp[e] * eb;   // bytes of a row
+            mma[e][i] = MmaDesc{(uint32_t)descs[i].b_off[e] >> 4, (uint32_t)(kb * 8) >> 4,
+                                tc::instr_desc(128, descs[i].np, eb == 2 ? tc::kFmtBF16 : tc::kFmtE4M3), (uint32_t)(kb / 32)};
+        }
+    static_assert(sizeof mma == sizeof c_mma_desc, "one 16-byte constant a layer");
+    cudaError_t e = cudaMemcpyToSymbol(c_mma_desc, mma, sizeof mma);
+    return e != cudaSuccess ? e : cudaMemcpyToSymbol(c_layer_desc, descs, sizeof descs);
 }
 
 __device__ __forceinline__ void group_bar(int g) {
@@ -269,35 +284,34 @@ struct Group {
 };
 constexpr int kStFailed = 2;
 
-// Up to three MMAs (layer, A sub-tile byte offset, D column), issued after
-// all A rows are in shared memory and awaited by the whole group.
-template <int EB>
-__device__ __noinline__ int mma_round(const Group G, int st, int count, int l0, int a_stride, int d0, int d_stride) {
+// The MMAs of one layer (COUNT = 1) or of the three channels' layers (3; A
+// sub-tiles a_stride bytes and accumulators d_stride columns apart), issued
+// after all A rows are in shared memory and awaited by the whole group.  The
+// first thread of warp q issues layer l0 + q, so three layers' issue runs side
+// by side; the mbarrier takes kArrivals arrivals a round.
+constexpr int kArrivals = 3;
+template <int EB, int COUNT>
+__device__ __noinline__ int mma_round(const Group G, int st, int l0, int a_stride, int d0, int d_stride) {
+    static_assert(COUNT == 1 || COUNT == kArrivals, "arrivals a round");
     tc::fence_proxy_async();
     tc::fence_before_sync();
     group_bar(G.g);
-    if (G.t == 0) {
+    if ((G.t & 31) == 0 && G.t < 32 * COUNT) {
         tc::fence_after_sync();
-        const uint32_t col0 = G.tmem & 0xFFFFu;   // lane 0, the group's column 0
-        const int e = EB == 2 ? 0 : 1;
+        const int q = G.t >> 5;
+        const uint4 m = c_mma_desc[EB == 2 ? 0 : 1][l0 + q];
+        // (LBO: 128 bytes between the two 16-byte K chunks of one MMA)
+        const uint64_t hi = ((uint64_t)(128 >> 4) << 16) | ((uint64_t)m.y << 32) | (1ull << 46);
+        uint64_t ad = hi | (((G.a_s + (uint32_t)(q * a_stride)) >> 4) & 0x3FFFu);
+        uint64_t bd = hi | (((G.wimg_s >> 4) + m.x) & 0x3FFFu);
+        const uint32_t dc = (G.tmem & 0xFFFFu) + (uint32_t)(d0 + q * d_stride);   // lane 0, the group's columns
 #pragma unroll 1
-        for (int q = 0; q < count; ++q) {
-            const int L = l0 + q;
-            int kp = c_layer_desc[L].kp[e];
-            uint32_t idesc = tc::instr_desc(128, c_layer_desc[L].np, EB == 2 ? tc::kFmtBF16 : tc::kFmtE4M3);
-            uint32_t sbo = (uint32_t)(kp * EB * 8);
-            int steps = kp * EB / 32;   // 32 bytes of K per MMA (16 BF16 / 32 E4M3)
-            uint32_t ab = G.a_s + (uint32_t)(q * a_stride), bb = G.wimg_s + (uint32_t)c_layer_desc[L].b_off[e];
-            uint32_t dc = col0 + (uint32_t)(d0 + q * d_stride);
-#pragma unroll 1
-            for (int s = 0; s < steps; ++s) {
-                uint64_t ad = tc::smem_desc(ab + s * 256, 128, sbo);
-                uint64_t bd = tc::smem_desc(bb + s * 256, 128, sbo);
-                if (EB == 2) tc::mma_bf16(dc, ad, bd, idesc, s > 0);
-                else tc::mma_fp8(dc, ad, bd, idesc, s > 0);
-            }
+        for (uint32_t s = 0; s < m.w; ++s, ad += 256 >> 4, bd += 256 >> 4) {
+            if (EB == 2) tc::mma_bf16(dc, ad, bd, m.z, s > 0);
+            else tc::mma_fp8(dc, ad, bd, m.z, s > 0);
         }
-        tc::mma_commit_s(G.mbar_s);
+#pragma unroll
+        for (int i = 0; i < kArrivals / COUNT; ++i) tc::mma_commit_s(G.mbar_s);
     }
     bool done = tc::mbar_wait_s(G.mbar_s, (uint32_t)(st & 1), kWaitLimit);
     st ^= 1;
@@ -609,7 +623,7 @@ __device__ __noinline__ int tc_block(const Group G, int st, const Src src, const
         }
         rs[c] = write_row<EB, W, KP>(G.a_s, c * SUB, G.t, in);
     }
-    st = mma_round<EB>(G, st, 3, bd.l0, SUB, bd.col, bd.stride);
+    st = mma_round<EB, 3>(G, st, bd.l0, SUB, bd.col, bd.stride);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         float d[W];
@@ -639,12 +653,12 @@ __device__ __noinline__ int tc_residual_pair(const Group G, int st, const float*
     float a16[16];
     tmem_get<16>(G, kColA16<COL>, a16);
     float r0 = write_row<EB, 16, KP>(G.a_s, 0, G.t, a16);
-    st = mma_round<EB>(G, st, 1, La, 0, 64, 0);
+    st = mma_round<EB, 1>(G, st, La, 0, 64, 0);
     float u[16];
     tmem_get<16>(G, 64, u);
     bias_relu<EB, 16>(u, La, r0, aux);
     float r1 = write_row<EB, 16, KP>(G.a_s, 0, G.t, u);
-    st = mma_round<EB>(G, st, 1, Lb, 0, 80, 0);
+    st = mma_round<EB, 1>(G, st, Lb, 0, 80, 0);
     float z[16];
     tmem_get<16>(G, 80, z);
     bias_relu<EB, 16>(z, Lb, r1, aux);
@@ -737,7 +751,7 @@ __device__ __noinline__ TailOut tc_tail(const Group G, int st, const float* aux,
             }
         }
     });
-    st = mma_round<EB>(G, st, 1, kLC0, 0, 0, 0);
+    st = mma_round<EB, 1>(G, st, kLC0, 0, 0, 0);
     float rn = write_parts<EB, 128>(G, [&](int p, float (&v)[32]) {
         tmem_get<32>(G, 32 * p, v);
         if (p == 0) bias_relu<EB, 32, 0>(v, kLC0, r, aux);
@@ -745,20 +759,20 @@ __device__ __noinline__ TailOut tc_tail(const Group G, int st, const float* aux,
         else if (p == 2) bias_relu<EB, 32, 64>(v, kLC0, r, aux);
         else bias_relu<EB, 32, 96>(v, kLC0, r, aux);
     });
-    st = mma_round<EB>(G, st, 1, kLC1, 0, 0, 0);
+    st = mma_round<EB, 1>(G, st, kLC1, 0, 0, 0);
     r = rn;
     rn = write_parts<EB, 64>(G, [&](int p, float (&v)[32]) {
         tmem_get<32>(G, 32 * p, v);
         if (p == 0) bias_relu<EB, 32, 0>(v, kLC1, r, aux);
         else bias_relu<EB, 32, 32>(v, kLC1, r, aux);
     });
-    st = mma_round<EB>(G, st, 1, kLC2, 0, 0, 0);
+    st = mma_round<EB, 1>(G, st, kLC2, 0, 0, 0);
     r = rn;
     rn = write_parts<EB, 32>(G, [&](int, float (&v)[32]) {
         tmem_get<32>(G, 0, v);
         bias_relu<EB, 32>(v, kLC2, r, aux);
     });
-    st = mma_round<EB>(G, st, 1, kLX, 0, 32, 0);
+    st = mma_round<EB, 1>(G, st, kLX, 0, 32, 0);
     float a16[16];
     tmem_get<16>(G, 32, a16);
     bias_relu<EB, 16>(a16, kLX, rn, aux);
@@ -804,7 +818,7 @@ MRP_D int tc_network(const Group& G, int st, const Src& src, const float* aux,
             tmem_get<32>(G, 32 * c, pv);
             rs_main[c] = write_row<EB, 32, KP>(G.a_s, c * SUB, G.t, pv);
         }
-        st = mma_round<EB>(G, st, 3, kL81, SUB, 0, 32);
+        st = mma_round<EB, 3>(G, st, kL81, SUB, 0, 32);
     }
     // direct-illumination branch, X[160:192], and its 8x8 finals
 #pragma unroll 1
@@ -818,7 +832,7 @@ MRP_D int tc_network(const Group& G, int st, const Src& src, const float* aux,
             tmem_get<8>(G, kColDi + 16 * c, pv);
             rs_di[c] = write_row<EB, 8, KP>(G.a_s, c * SUB, G.t, pv);
         }
-        st = mma_round<EB>(G, st, 3, kLD41, SUB, kColDi, 16);
+        st = mma_round<EB, 3>(G, st, kLD41, SUB, kColDi, 16);
     }
     // comb[120] = relu(finals + b): the direct-illumination part behind the
     // main one, once it and the LSEFin1 sums have been read
@@ -913,7 +927,7 @@ __global__ void __launch_bounds__(kGroups<COL> * kGroupThreads, 1) k_mlp_tc(cons
         tc::tmem_alloc(tslot, kTmemCols);
         tc::tmem_relinquish();
     }
-    if (tid < kGroups<COL>) tc::mbar_init(mbar + tid, 1);
+    if (tid < kGroups<COL>) tc::mbar_init(mbar + tid, kArrivals);
     if (STAGED && tid == 32) {
         int acc = 0;
         for (int q = 0; q < nseg; ++q) {
