@@ -7,8 +7,8 @@
 // for coloured albedos) each own one 128-pixel tile at a time; thread t of a
 // group owns pixel row t of its tile and TMEM lane t.  Per layer step the
 // group writes its A rows (activations, rounded to BF16 or quantised to
-// FP8-E4M3) to shared memory, one elected thread issues tcgen05.mma into the
-// group's TMEM columns and commits to an mbarrier, and every thread reads its
+// FP8-E4M3) to shared memory, an elected thread a layer issues tcgen05.mma into
+// the group's TMEM columns and commits to an mbarrier, and every thread reads its
 // row of the FP32 accumulator back with tcgen05.ld for the epilogue (bias,
 // ReLU, residuals, gates), all in FP32 on the CUDA cores.  The SE gate MLPs,
 // pooling, the LSEFin gate and the last 16->1 layer stay in FP32.
@@ -266,6 +266,10 @@ static cudaError_t upload_layer_descs() {
     return e != cudaSuccess ? e : cudaMemcpyToSymbol(c_layer_desc, descs, sizeof descs);
 }
 
+// barrier 0 is __syncthreads, 1 to 3 the groups', 4 the split tile's
+__device__ __forceinline__ void split_bar() {
+    asm volatile("bar.sync %0, %1;" ::"r"(4), "r"(3 * kGroupThreads) : "memory");
+}
 __device__ __forceinline__ void group_bar(int g) {
     asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(kGroupThreads) : "memory");
 }
@@ -289,14 +293,17 @@ constexpr int kStFailed = 2;
 // after all A rows are in shared memory and awaited by the whole group.  The
 // first thread of warp q issues layer l0 + q, so three layers' issue runs side
 // by side; the mbarrier takes kArrivals arrivals a round.
+// SPLIT: all three groups wrote the rows and wait (G.g is a thread's share of
+// its row there, and the first group's threads issue).
 constexpr int kArrivals = 3;
-template <int EB, int COUNT>
+template <int EB, int COUNT, bool SPLIT = false>
 __device__ __noinline__ int mma_round(const Group G, int st, int l0, int a_stride, int d0, int d_stride) {
     static_assert(COUNT == 1 || COUNT == kArrivals, "arrivals a round");
     tc::fence_proxy_async();
     tc::fence_before_sync();
-    group_bar(G.g);
-    if ((G.t & 31) == 0 && G.t < 32 * COUNT) {
+    if (SPLIT) split_bar();
+    else group_bar(G.g);
+    if ((G.t & 31) == 0 && G.t < 32 * COUNT && (!SPLIT || G.g == 0)) {
         tc::fence_after_sync();
         const int q = G.t >> 5;
         const uint4 m = c_mma_desc[EB == 2 ? 0 : 1][l0 + q];
@@ -387,12 +394,12 @@ MRP_D float sigmoid_d(float o) { return 1.0f / (1.0f + __expf(-o)); }
 // pointer; reading them with shared-space loads (the address converted once
 // per access) keeps them off the generic load path, whose results the
 // scheduler tracks like global loads.
-MRP_D float4 lds4(const float* p) {
-    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+MRP_D float4 lds4_at(uint32_t a) {
     float4 v;
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
     return v;
 }
+MRP_D float4 lds4(const float* p) { return lds4_at((uint32_t)__cvta_generic_to_shared(p)); }
 MRP_D float lds1(const float* p) {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
     float v;
@@ -407,11 +414,11 @@ MRP_D void add_to(float& a0, float& a1, float b0, float b1) { upk2(add2(pk2(a0, 
 MRP_D void fma_to(float& a0, float& a1, float x0, float x1, f32x2 g) { upk2(fma2(pk2(x0, x1), g, pk2(a0, a1)), a0, a1); }
 
 // Biases and scales start on 16-float boundaries (scale_off), so they are
-// read four at a time.  OFF: first output of the part at hand.
-template <int EB, int N, int OFF = 0>
-MRP_D void bias_relu(float* d, int L, float rs, const float* aux) {
+// read four at a time.  off: first output of the part at hand.
+template <int EB, int N>
+MRP_D void bias_relu(float* d, int L, float rs, const float* aux, int off = 0) {
     static_assert(N % 4 == 0, "layer widths are multiples of 4");
-    const int ab = c_layer_desc[L].abias + OFF, so = c_layer_desc[L].soff + OFF;
+    const int ab = c_layer_desc[L].abias + off, so = c_layer_desc[L].soff + off;
 #pragma unroll
     for (int q = 0; q < N / 4; ++q) {
         const float4 b = lds4(aux + ab + 4 * q);
@@ -441,6 +448,16 @@ MRP_D void aux_row(const float* aux, int off, float* out) {
     }
 }
 
+// Asynchronous copies into shared memory (dst a shared address).
+MRP_D void copy16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+MRP_D void copy4(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+constexpr int kStageStride = 3 * kGroupThreads * 16;   // bytes between a thread's chunks in SplitScratch::stage
+MRP_D void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Feature sources (rows may be invalid: zeros); FROM is a run-time offset.
 // Row-major features are read 16 bytes at a time where the rows start on 16
 // bytes: a load of 4 bytes a lane touches 32 lines for 128 bytes.  (100 001
@@ -462,6 +479,26 @@ struct RowFeatures {           // [n][576] row-major
             for (int i = 0; i < W; ++i) xs[i] = valid ? __ldg(p + i) : 0.0f;
         }
     }
+    // the slice as 16-byte chunks, chunk i at slot + i * kStageStride; staged
+    // reads them back
+    MRP_D void stage(int c, int from, int w, uint32_t slot) const {
+        if (!valid) return;
+        const float* p = x + c * 192 + from;
+        if (vec) {
+            for (int i = 0; i < w / 4; ++i) copy16(slot + i * kStageStride, p + 4 * i);
+        } else {
+            for (int i = 0; i < w; ++i) copy4(slot + (i >> 2) * kStageStride + (i & 3) * 4, p + i);
+        }
+    }
+    template <int W>
+    MRP_D void staged(uint32_t slot, float* xs) const {
+#pragma unroll
+        for (int i = 0; i < W / 4; ++i) {
+            float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (valid) q = lds4_at(slot + i * kStageStride);
+            xs[4 * i] = q.x; xs[4 * i + 1] = q.y; xs[4 * i + 2] = q.z; xs[4 * i + 3] = q.w;
+        }
+    }
 };
 struct TileFeatures {          // FP16 pairs of the staged predictor's tiled layout
     const __half2* x;          // already offset to (r / 32) * 288 * 32 + r % 32
@@ -473,6 +510,27 @@ struct TileFeatures {          // FP16 pairs of the staged predictor's tiled lay
             const float2 p = valid ? __half22float2(__ldg(x + (c * 96 + (from >> 1) + k) * 32)) : make_float2(0.0f, 0.0f);
             xs[2 * k] = p.x;
             xs[2 * k + 1] = p.y;
+        }
+    }
+    MRP_D void stage(int c, int from, int w, uint32_t slot) const {
+        if (!valid) return;
+        for (int k = 0; k < w / 2; ++k)
+            copy4(slot + (k >> 2) * kStageStride + (k & 3) * 4, x + (c * 96 + (from >> 1) + k) * 32);
+    }
+    template <int W>
+    MRP_D void staged(uint32_t slot, float* xs) const {
+#pragma unroll
+        for (int i = 0; i < W / 8; ++i) {
+            float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (valid) q = lds4_at(slot + i * kStageStride);
+            const float f[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t u = __float_as_uint(f[k]);
+                const float2 p = __half22float2(*reinterpret_cast<const __half2*>(&u));
+                xs[8 * i + 2 * k] = p.x;
+                xs[8 * i + 2 * k + 1] = p.y;
+            }
         }
     }
 };
@@ -669,6 +727,25 @@ __device__ __noinline__ int tc_residual_pair(const Group G, int st, const float*
     return st;
 }
 
+// The tail from LX's accumulator (columns 32..47) on: six residual pairs and
+// the 16 -> 1 head.
+struct TailOut { float p; int st; };
+template <int EB, bool COL>
+MRP_D TailOut tc_tail_end(const Group& G, int st, float r, const float* aux) {
+    float a16[16];
+    tmem_get<16>(G, 32, a16);
+    bias_relu<EB, 16>(a16, kLX, r, aux);
+    tmem_put<16>(G, kColA16<COL>, a16);
+    tc::tmem_wait_st();
+#pragma unroll 1
+    for (int k = 0; k < 6; ++k) st = tc_residual_pair<EB, COL>(G, st, aux, k);
+    tmem_get<16>(G, kColA16<COL>, a16);
+    float a = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) a = fmaf(a16[j], lds1(aux + kAuxLX12W + j), a);
+    return TailOut{fmaxf(a + lds1(aux + kAuxLX12B), 0.0f), st};
+}
+
 // An A row of N values that come in parts of 32: get(part, v) makes part
 // `part`.  FP8 rows take two passes, the first for the row's scale, so the
 // row is never held whole.
@@ -703,7 +780,6 @@ MRP_D float write_parts(const Group& G, F get) {
 // gate, LC0 over [comb * gate, LGGS], LC1, LC2, LX, six residual pairs and
 // the 16 -> 1 head.  comb (kColComb) and the LSEFin1 sums (kColHfTail) come
 // from TMEM.
-struct TailOut { float p; int st; };
 template <int EB, bool COL>
 __device__ __noinline__ TailOut tc_tail(const Group G, int st, const float* aux, float g, float gamma, float s4) {
     float gf[6];
@@ -754,17 +830,17 @@ __device__ __noinline__ TailOut tc_tail(const Group G, int st, const float* aux,
     st = mma_round<EB, 1>(G, st, kLC0, 0, 0, 0);
     float rn = write_parts<EB, 128>(G, [&](int p, float (&v)[32]) {
         tmem_get<32>(G, 32 * p, v);
-        if (p == 0) bias_relu<EB, 32, 0>(v, kLC0, r, aux);
-        else if (p == 1) bias_relu<EB, 32, 32>(v, kLC0, r, aux);
-        else if (p == 2) bias_relu<EB, 32, 64>(v, kLC0, r, aux);
-        else bias_relu<EB, 32, 96>(v, kLC0, r, aux);
+        if (p == 0) bias_relu<EB, 32>(v, kLC0, r, aux, 0);
+        else if (p == 1) bias_relu<EB, 32>(v, kLC0, r, aux, 32);
+        else if (p == 2) bias_relu<EB, 32>(v, kLC0, r, aux, 64);
+        else bias_relu<EB, 32>(v, kLC0, r, aux, 96);
     });
     st = mma_round<EB, 1>(G, st, kLC1, 0, 0, 0);
     r = rn;
     rn = write_parts<EB, 64>(G, [&](int p, float (&v)[32]) {
         tmem_get<32>(G, 32 * p, v);
-        if (p == 0) bias_relu<EB, 32, 0>(v, kLC1, r, aux);
-        else bias_relu<EB, 32, 32>(v, kLC1, r, aux);
+        if (p == 0) bias_relu<EB, 32>(v, kLC1, r, aux, 0);
+        else bias_relu<EB, 32>(v, kLC1, r, aux, 32);
     });
     st = mma_round<EB, 1>(G, st, kLC2, 0, 0, 0);
     r = rn;
@@ -773,20 +849,290 @@ __device__ __noinline__ TailOut tc_tail(const Group G, int st, const float* aux,
         bias_relu<EB, 32>(v, kLC2, r, aux);
     });
     st = mma_round<EB, 1>(G, st, kLX, 0, 32, 0);
-    float a16[16];
-    tmem_get<16>(G, 32, a16);
-    bias_relu<EB, 16>(a16, kLX, rn, aux);
-    tmem_put<16>(G, kColA16<COL>, a16);
-    tc::tmem_wait_st();
-#pragma unroll 1
-    for (int k = 0; k < 6; ++k) st = tc_residual_pair<EB, COL>(G, st, aux, k);
-    tmem_get<16>(G, kColA16<COL>, a16);
-    float a = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) a = fmaf(a16[j], lds1(aux + kAuxLX12W + j), a);
-    return TailOut{fmaxf(a + lds1(aux + kAuxLX12B), 0.0f), st};
+    return tc_tail_end<EB, COL>(G, st, rn, aux);
 }
 
+// ---------------------------------------------------------------------------
+// A tile split over the three groups, for calls of no more tiles than SMs,
+// where nothing hides the chain of a tile's dependent steps: three threads a
+// row, G.g the channel that a thread takes through the SE blocks and its part
+// of the rows behind them (all in the first group's A buffer and columns).
+// What they have to tell one another goes through the other groups' A
+// buffers.  Every value is made by the operations, in the order, that one
+// thread a row uses.  One FP8 tile of 300 sets: 111 k cycles with one thread
+// a row, two thirds of them in the SE blocks (9 to 10 k a block of width 32, a
+// third of that for its features to arrive); 70 k split, the next block's
+// features copied to shared memory meanwhile (4 k a block).  The call 83.5 ->
+// 63 us; a 163 x 97 FP8 frame of four launches 587 -> 528 us.
+// ---------------------------------------------------------------------------
+struct SplitScratch {
+    float4 stage[8][3 * kGroupThreads];   // the threads' slices of the next block (chunk, thread)
+    float hf[16][128];                    // LSEFin1 sums
+    union {
+        float pool[2][6][128];    // slice pools (block parity; average, maximum of a channel)
+        float amax[2][3][128];    // behind the blocks, FP8: largest value of a thread's part
+    };
+};
+static_assert(sizeof(SplitScratch) <= 2 * kABytes, "the other groups' A buffers hold it");
+
+template <int EB, int W, class Src>
+__device__ __noinline__ int split_block(const Group G, int st, const Src src, const float* aux, SplitScratch* X, int b,
+                                        float g, float gamma) {
+    const BlockDesc bd = c_blocks[b];
+    constexpr int KP = pad_to(W, EB == 2 ? 16 : 32);
+    const int c = G.g, col = bd.col + c * bd.stride;
+    float (*pool)[128] = X->pool[b & 1];
+    // (asked for a block ago)
+    float xs[W];
+    const uint32_t slot = tc::smem_addr(&X->stage[0][c * kGroupThreads + G.t]);
+    copies_wait();
+    src.template staged<W>(slot, xs);
+    {
+        float s = 0.0f, m = -10000.0f;
+#pragma unroll
+        for (int i = 0; i < W; ++i) { s += xs[i]; m = fmaxf(m, xs[i]); }
+        pool[c][G.t] = s / (float)W;
+        pool[3 + c][G.t] = m;
+    }
+    split_bar();
+    if (b < 11) src.stage(c, c_blocks[b + 1].from, c_blocks[b + 1].w, slot);
+    float p8[8];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) p8[i] = pool[i][G.t];
+    p8[6] = g;
+    p8[7] = gamma;
+    float gate;
+    {
+        float h[8], a = 0.0f;
+#pragma unroll
+        for (int o = 0; o < 8; ++o) h[o] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float4 u = lds4(aux + bd.se_off + 8 * j), v = lds4(aux + bd.se_off + 8 * j + 4);
+            const f32x2 p = pk2(p8[j], p8[j]);
+            fma_to(h[0], h[1], u.x, u.y, p);
+            fma_to(h[2], h[3], u.z, u.w, p);
+            fma_to(h[4], h[5], v.x, v.y, p);
+            fma_to(h[6], h[7], v.z, v.w, p);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a = fmaf(fmaxf(h[j], 0.0f), lds1(aux + bd.se_off + 64 + 4 * j + c), a);
+        gate = sigmoid_d(a);
+    }
+    float rs;
+    {
+        float in[W];
+        const f32x2 q = pk2(gate, gate);
+        if (bd.has_prev) {
+            tmem_get<W>(G, col, in);
+#pragma unroll
+            for (int i = 0; i < W; i += 2) fma_to(in[i], in[i + 1], xs[i], xs[i + 1], q);
+        } else {
+#pragma unroll
+            for (int i = 0; i < W; i += 2) upk2(mul2(pk2(xs[i], xs[i + 1]), q), in[i], in[i + 1]);
+        }
+        rs = write_row<EB, W, KP>(G.a_s, c * 128 * KP * EB, G.t, in);
+    }
+    // LSEFin1, eight outputs for each of two of a row's threads
+    if (c < 2) {
+        float hf[8];
+#pragma unroll
+        for (int o = 0; o < 8; ++o) hf[o] = b == 0 ? 0.0f : X->hf[8 * c + o][G.t];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const f32x2 av = pk2(p8[k], p8[k]), mx = pk2(p8[3 + k], p8[3 + k]);
+            const float* wa = aux + kAuxLSE1 + 16 * (bd.pid + k) + 8 * c;
+            const float* wm = wa + 16 * 36;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const float4 u = lds4(wa + 4 * q), v = lds4(wm + 4 * q);
+                fma_to(hf[4 * q], hf[4 * q + 1], u.x, u.y, av);
+                fma_to(hf[4 * q + 2], hf[4 * q + 3], u.z, u.w, av);
+                fma_to(hf[4 * q], hf[4 * q + 1], v.x, v.y, mx);
+                fma_to(hf[4 * q + 2], hf[4 * q + 3], v.z, v.w, mx);
+            }
+        }
+#pragma unroll
+        for (int o = 0; o < 8; ++o) X->hf[8 * c + o][G.t] = hf[o];
+    }
+    st = mma_round<EB, 3, true>(G, st, bd.l0, 128 * KP * EB, bd.col, bd.stride);
+    float d[W];
+    tmem_get<W>(G, col, d);
+    bias_relu<EB, W>(d, bd.l0 + c, rs, aux);
+    if (bd.widen) {
+        float nv[2 * W];
+#pragma unroll
+        for (int o = 0; o < W; ++o) { nv[o] = d[o]; nv[W + o] = xs[o]; }
+        tmem_put<2 * W>(G, col, nv);
+    } else {
+#pragma unroll
+        for (int o = 0; o < W; o += 2) add_to(d[o], d[o + 1], xs[o], xs[o + 1]);
+        tmem_put<W>(G, col, d);
+    }
+    tc::tmem_wait_st();
+    return st;
+}
+
+// The row's FP8 scale from what its three threads hold (1 in BF16).
+template <int EB>
+MRP_D float split_scale(const Group& G, float (&part)[3][128], float amax) {
+    if (EB == 2) return 1.0f;
+    part[G.g][G.t] = amax;
+    split_bar();
+    amax = fmaxf(fmaxf(part[0][G.t], part[1][G.t]), part[2][G.t]);
+    return amax > 0.0f ? amax * (1.0f / 448.0f) : 1.0f;
+}
+template <int N>
+MRP_D float abs_max(const float* v, float a) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) a = fmaxf(a, fabsf(v[i]));
+    return a;
+}
+// Values [k, k + N) of this row's A operand of KP (N 8 or a multiple of 16).
+template <int EB, int KP, int N>
+MRP_D void split_store(const Group& G, int k, const float* v, float inv) {
+    if (EB == 2) {
+#pragma unroll
+        for (int i = 0; i < N; i += 8)
+            tc::st_shared_v4(G.a_s + (uint32_t)op_off(G.t, k + i, KP, EB), tc::pack_bf16(v[i], v[i + 1]),
+                             tc::pack_bf16(v[i + 2], v[i + 3]), tc::pack_bf16(v[i + 4], v[i + 5]),
+                             tc::pack_bf16(v[i + 6], v[i + 7]));
+    } else {
+        uint32_t w[N / 4];
+#pragma unroll
+        for (int q = 0; q < N / 4; ++q)
+            w[q] = (uint32_t)tc::pack_e4m3(v[4 * q] * inv, v[4 * q + 1] * inv) |
+                   ((uint32_t)tc::pack_e4m3(v[4 * q + 2] * inv, v[4 * q + 3] * inv) << 16);
+        if constexpr (N == 8) {
+            tc::st_shared_v2(G.a_s + (uint32_t)op_off(G.t, k, KP, EB), w[0], w[1]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < N / 16; ++i)
+                tc::st_shared_v4(G.a_s + (uint32_t)op_off(G.t, k + 16 * i, KP, EB), w[4 * i], w[4 * i + 1], w[4 * i + 2],
+                                 w[4 * i + 3]);
+        }
+    }
+}
+// The next layer's A row (N values, relu(D + b) of layer L) from the
+// accumulator in columns [0, N), in parts of 16: thread c of a row takes parts
+// c, c + 3, ...; returns the row's scale.
+template <int EB, int N>
+MRP_D float split_relu_row(const Group& G, int L, float r, const float* aux, float (&part)[3][128]) {
+    constexpr int MINE = (N / 16 + 2) / 3;
+    float v[MINE][16], amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < MINE; ++i) {
+        const int p = G.g + 3 * i;
+        if (p < N / 16) {
+            tmem_get<16>(G, 16 * p, v[i]);
+            bias_relu<EB, 16>(v[i], L, r, aux, 16 * p);
+            if (EB == 1) amax = abs_max<16>(v[i], amax);
+        }
+    }
+    const float s = split_scale<EB>(G, part, amax), inv = 1.0f / s;
+#pragma unroll
+    for (int i = 0; i < MINE; ++i) {
+        const int p = G.g + 3 * i;
+        if (p < N / 16) split_store<EB, N, 16>(G, 16 * p, v[i], inv);
+    }
+    return s;
+}
+
+// tc_network of a grey albedo for a split tile; the first group's threads
+// return the result.
+template <int EB, class Src>
+__device__ __noinline__ TailOut split_network(const Group G, int st, const Src src, const float* aux, SplitScratch* X,
+                                              float gamma, float g, float s4) {
+    const int c = G.g;
+    src.stage(c, c_blocks[0].from, c_blocks[0].w, tc::smem_addr(&X->stage[0][c * kGroupThreads + G.t]));
+#pragma unroll 1
+    for (int b = 0; b < 8; ++b) {
+        const int w = c_blocks[b].w;
+        if (w == 8) st = split_block<EB, 8>(G, st, src, aux, X, b, g, gamma);
+        else if (w == 16) st = split_block<EB, 16>(G, st, src, aux, X, b, g, gamma);
+        else st = split_block<EB, 32>(G, st, src, aux, X, b, g, gamma);
+    }
+    float m[32], e[8], rs;
+    {
+        constexpr int KP = pad_to(32, EB == 2 ? 16 : 32), SUB = 128 * KP * EB;
+        tmem_get<32>(G, 32 * c, m);
+        rs = write_row<EB, 32, KP>(G.a_s, c * SUB, G.t, m);
+        st = mma_round<EB, 3, true>(G, st, kL81, SUB, 0, 32);
+    }
+    tmem_get<32>(G, 32 * c, m);
+    bias_relu<EB, 32>(m, kL81 + c, rs, aux);
+    tmem_put<32>(G, 32 * c, m);
+    tc::tmem_wait_st();
+#pragma unroll 1
+    for (int b = 8; b < 12; ++b) st = split_block<EB, 8>(G, st, src, aux, X, b, g, gamma);
+    {
+        constexpr int KP = pad_to(8, EB == 2 ? 16 : 32), SUB = 128 * KP * EB;
+        tmem_get<8>(G, kColDi + 16 * c, e);
+        rs = write_row<EB, 8, KP>(G.a_s, c * SUB, G.t, e);
+        st = mma_round<EB, 3, true>(G, st, kLD41, SUB, kColDi, 16);
+    }
+    tmem_get<8>(G, kColDi + 16 * c, e);
+    bias_relu<EB, 8>(e, kLD41 + c, rs, aux);
+    tmem_get<32>(G, 32 * c, m);
+    // LSEFin: of its six gates a thread needs its channel's two
+    float gf[2];
+    {
+        float h[16];
+#pragma unroll
+        for (int o = 0; o < 16; ++o) {
+            float a = X->hf[o][G.t];
+            a = fmaf(lds1(aux + kAuxLSE1 + 16 * 72 + o), g, a);
+            a = fmaf(lds1(aux + kAuxLSE1 + 16 * 73 + o), gamma, a);
+            a = fmaf(lds1(aux + kAuxLSE1 + 16 * 74 + o), s4, a);
+            h[o] = fmaxf(a, 0.0f);
+        }
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+            float w[16];
+            aux_row<16>(aux, kAuxLSE2 + (c + 3 * o) * 16, w);
+            float a = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) a = fmaf(h[j], w[j], a);
+            gf[o] = sigmoid_d(a);
+        }
+    }
+    // LC0's A row: a channel's 32 and 8 gated values each, LGGS by the last
+    {
+        const f32x2 q = pk2(gf[0], gf[0]);
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) upk2(mul2(pk2(m[i], m[i + 1]), q), m[i], m[i + 1]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) e[i] *= gf[1];
+    float lg[8];
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {
+        float a = 0.0f;
+        a = fmaf(g, lds1(aux + kAuxLGGSW + o * 3), a);
+        a = fmaf(gamma, lds1(aux + kAuxLGGSW + o * 3 + 1), a);
+        a = fmaf(s4, lds1(aux + kAuxLGGSW + o * 3 + 2), a);
+        lg[o] = fmaxf(a + lds1(aux + kAuxLGGSB + o), 0.0f);
+    }
+    float r;
+    {
+        float amax = 0.0f;
+        if (EB == 1) amax = abs_max<8>(lg, abs_max<8>(e, abs_max<32>(m, 0.0f)));
+        r = split_scale<EB>(G, X->amax[0], amax);
+        const float inv = 1.0f / r;
+        split_store<EB, 128, 32>(G, 32 * c, m, inv);
+        split_store<EB, 128, 8>(G, 96 + 8 * c, e, inv);
+        if (c == 2) split_store<EB, 128, 8>(G, 120, lg, inv);
+    }
+    st = mma_round<EB, 1, true>(G, st, kLC0, 0, 0, 0);
+    r = split_relu_row<EB, 128>(G, kLC0, r, aux, X->amax[1]);
+    st = mma_round<EB, 1, true>(G, st, kLC1, 0, 0, 0);
+    r = split_relu_row<EB, 64>(G, kLC1, r, aux, X->amax[0]);
+    st = mma_round<EB, 1, true>(G, st, kLC2, 0, 0, 0);
+    r = split_relu_row<EB, 32>(G, kLC2, r, aux, X->amax[1]);
+    st = mma_round<EB, 1, true>(G, st, kLX, 0, 32, 0);
+    // the 16-wide rest is one thread's work a row
+    return c == 0 ? tc_tail_end<EB, false>(G, st, r, aux) : TailOut{0.0f, st};
+}
 
 template <int EB, class Src>
 MRP_D int run_block(const Group& G, int st, const Src& src, const float* aux, int b, float g, float gamma) {
@@ -795,6 +1141,8 @@ MRP_D int run_block(const Group& G, int st, const Src& src, const float* aux, in
     if (w == 16) return tc_block<EB, 16>(G, st, src, aux, b, g, gamma);
     return tc_block<EB, 32>(G, st, src, aux, b, g, gamma);
 }
+
+MRP_D float radiance(float p, float s4) { return fmaxf(expf(p) - 1.0f, 0.0f) * s4; }
 
 template <int EB, bool COL, class Src>
 MRP_D int tc_network(const Group& G, int st, const Src& src, const float* aux,
@@ -875,7 +1223,7 @@ MRP_D int tc_network(const Group& G, int st, const Src& src, const float* aux,
     }
     if (!COL) P[1] = P[2] = P[0];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) out[c] = fmaxf(expf(P[c]) - 1.0f, 0.0f) * powf(srv[c], 4.0f);
+    for (int c = 0; c < 3; ++c) out[c] = radiance(P[c], powf(srv[c], 4.0f));
     return st;
 }
 
@@ -902,7 +1250,58 @@ struct TcArgs {
     TcSegment seg0;
 };
 
-template <int EB, bool STAGED, bool COL>
+// One tile of `rows` rows: st = eval(features, gamma, g, sr, o) for row t, and,
+// with `stores`, its result.
+template <bool STAGED, class F>
+MRP_D int tile_work(const TcArgs& A, const TcSegment* segs, const int* seg_start, int rows, int tile, int t, bool stores,
+                    F eval) {
+    int st;
+    float o[3];
+    if constexpr (STAGED) {
+        int q = 0;
+        while (tile >= seg_start[q + 1]) ++q;
+        const TcSegment* S = segs + q;
+        const int r = (tile - seg_start[q]) * rows + t;
+        const bool valid = t < rows && r < *S->rec_count;
+        const size_t cap = S->rec_cap;
+        float gamma = valid ? S->rec_f[15 * cap + r] : 0.0f;
+        TileFeatures src{reinterpret_cast<const __half2*>(S->feat) + (size_t)(r >> 5) * 288 * 32 + (r & 31), valid};
+        st = eval(src, gamma, S->g, S->sr, o);
+        if (valid && stores && !(st & kStFailed)) {
+            int pix = S->rec_pix[r];
+            f3 hit = mk3(S->rec_f[r], S->rec_f[cap + r], S->rec_f[2 * cap + r]);
+            f3 res = mul(mul(mk3(o[0], o[1], o[2]), S->light_color), S->scatter_rate);
+            float4 v4 = make_float4(fmaxf(res.x, 0.0f), fmaxf(res.y, 0.0f), fmaxf(res.z, 0.0f),
+                                    fmaxf(length(sub(S->ori, hit)), 0.0f));
+            const int mean_k = S->mean_k;
+            float rate = 1.0f / (float)(1 + mean_k);
+            float4 a = mean_k == 0 ? make_float4(0, 0, 0, 0) : S->accum[pix];
+            S->accum[pix] = make_float4(lerp(a.x, v4.x, rate), lerp(a.y, v4.y, rate), lerp(a.z, v4.z, rate),
+                                        lerp(a.w, v4.w, rate));
+        }
+    } else {
+        const int r = tile * rows + t;
+        const bool valid = t < rows && r < A.n;
+        float gamma = valid ? A.gamma[r] : 0.0f;
+        RowFeatures src{A.feat + (size_t)r * 576, valid, A.feat_vec};
+        st = eval(src, gamma, A.g, A.sr, o);
+        if (valid && stores && !(st & kStFailed)) {
+            A.out3[3 * (size_t)r] = o[0];
+            A.out3[3 * (size_t)r + 1] = o[1];
+            A.out3[3 * (size_t)r + 2] = o[2];
+        }
+    }
+    return st;
+}
+
+// Rows of a split tile: 32 or 64 of the 128 where the sets then still fit one
+// tile an SM (an SM takes a tile's features in at 64 bytes a cycle).
+MRP_D int split_rows(int tiles64, int tiles32, int sms) { return tiles32 <= sms ? 32 : tiles64 <= sms ? 64 : 128; }
+
+// SPLIT (grey albedos): the groups share each tile, for calls of at most one
+// tile an SM.  A form of its own: beside the other in one kernel it cost that
+// one 1 % of a 1080p frame.
+template <int EB, bool STAGED, bool COL, bool SPLIT>
 __global__ void __launch_bounds__(kGroups<COL> * kGroupThreads, 1) k_mlp_tc(const __grid_constant__ TcArgs A) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const int wbytes = (A.wimg_bytes + 1023) & ~1023;
@@ -918,8 +1317,8 @@ __global__ void __launch_bounds__(kGroups<COL> * kGroupThreads, 1) k_mlp_tc(cons
 
     const int tid = threadIdx.x, warp = tid / 32;
     // weights -> shared memory
-    for (int i = tid * 16; i < A.wimg_bytes; i += blockDim.x * 16)
-        *reinterpret_cast<uint4*>(wimg + i) = __ldg(reinterpret_cast<const uint4*>(A.wimg + i));
+    const uint32_t wimg_at = tc::smem_addr(wimg);
+    for (int i = tid * 16; i < A.wimg_bytes; i += blockDim.x * 16) copy16(wimg_at + (uint32_t)i, A.wimg + i);
     aux_s = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(aux_s) + 15) & ~(uintptr_t)15);
     for (int i = tid * 4; i < kAuxCount; i += blockDim.x * 4)
         *reinterpret_cast<float4*>(aux_s + i) = __ldg(reinterpret_cast<const float4*>(A.aux + i));
@@ -929,14 +1328,21 @@ __global__ void __launch_bounds__(kGroups<COL> * kGroupThreads, 1) k_mlp_tc(cons
     }
     if (tid < kGroups<COL>) tc::mbar_init(mbar + tid, kArrivals);
     if (STAGED && tid == 32) {
-        int acc = 0;
+        int acc[3] = {0, 0, 0}, rows = 128;   // tiles of 128, 64 and 32 rows
+        for (int q = 0; SPLIT && q < nseg; ++q)
+            for (int k = 0; k < 3; ++k) acc[k] += (*segs[q].rec_count + (128 >> k) - 1) >> (7 - k);
+        if (SPLIT) rows = split_rows(acc[1], acc[2], (int)gridDim.x);
+        int start = 0;
         for (int q = 0; q < nseg; ++q) {
-            seg_start[q] = acc;
-            acc += (*segs[q].rec_count + 127) / 128;
+            seg_start[q] = start;
+            start += (*segs[q].rec_count + rows - 1) / rows;
         }
-        seg_start[nseg] = acc;
+        seg_start[nseg] = start;
+        seg_start[kTcMaxSegments + 1] = rows;
     }
     tc::mbar_fence_init();
+    copies_wait();
+    tc::fence_proxy_async();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -952,10 +1358,30 @@ __global__ void __launch_bounds__(kGroups<COL> * kGroupThreads, 1) k_mlp_tc(cons
     G.err = A.err;
     int st = 0;
 
-    const int total_tiles = STAGED ? seg_start[nseg] : (A.n + 127) / 128;
-    // the first tiles go round the blocks (few tiles: each its own SM), the
-    // rest to whichever group is free
-    for (bool first = true;; first = false) {
+    const int rows = !SPLIT ? 128 : STAGED ? seg_start[kTcMaxSegments + 1]
+                                           : split_rows((A.n + 63) / 64, (A.n + 31) / 32, (int)gridDim.x);
+    const int total_tiles = STAGED ? seg_start[nseg] : (A.n + rows - 1) / rows;
+    if constexpr (SPLIT) {
+        static_assert(!COL, "three groups");
+        SplitScratch* X = reinterpret_cast<SplitScratch*>(abuf + kABytes);
+        G.a_s = tc::smem_addr(abuf);
+        G.mbar_s = tc::smem_addr(mbar);
+        G.tmem = tbase + ((uint32_t)(32 * (warp % 4)) << 16);
+        for (int tile = blockIdx.x; tile < total_tiles; tile += (int)gridDim.x) {
+            // (the first group's rounds alone are an even number, so all
+            // threads are at the same phase of its mbarrier here)
+            split_bar();
+            st = tile_work<STAGED>(A, segs, seg_start, rows, tile, G.t, G.g == 0,
+                                   [&](const auto& src, float gamma, float g, f3 sr, float* o) {
+                                       const float s4 = powf(sr.x, 4.0f);
+                                       const TailOut t = split_network<EB>(G, st, src, aux_s, X, gamma, g, s4);
+                                       o[0] = o[1] = o[2] = radiance(t.p, s4);
+                                       return t.st;
+                                   });
+        }
+    }
+    // the first tiles go round the blocks, the rest to whichever group is free
+    for (bool first = true; !SPLIT; first = false) {
         if (G.t == 0)
             tile_slot[G.g] = first ? G.g * (int)gridDim.x + (int)blockIdx.x
                                    : kGroups<COL> * (int)gridDim.x + atomicAdd(A.tile_counter, 1);
@@ -967,41 +1393,10 @@ __global__ void __launch_bounds__(kGroups<COL> * kGroupThreads, 1) k_mlp_tc(cons
         // features in record order just before, so the last tiles' features
         // are still in L2 when the first groups ask for them
         if (STAGED) tile = total_tiles - 1 - tile;
-        float o[3];
-        if (STAGED) {
-            int q = 0;
-            while (tile >= seg_start[q + 1]) ++q;
-            const TcSegment* S = segs + q;
-            const int r = (tile - seg_start[q]) * 128 + G.t;
-            const bool valid = r < *S->rec_count;
-            const size_t cap = S->rec_cap;
-            float gamma = valid ? S->rec_f[15 * cap + r] : 0.0f;
-            TileFeatures src{reinterpret_cast<const __half2*>(S->feat) + (size_t)(r >> 5) * 288 * 32 + (r & 31), valid};
-            st = tc_network<EB, COL>(G, st, src, aux_s, gamma, S->g, S->sr, o);
-            if (valid && !(st & kStFailed)) {
-                int pix = S->rec_pix[r];
-                f3 hit = mk3(S->rec_f[r], S->rec_f[cap + r], S->rec_f[2 * cap + r]);
-                f3 res = mul(mul(mk3(o[0], o[1], o[2]), S->light_color), S->scatter_rate);
-                float4 v4 = make_float4(fmaxf(res.x, 0.0f), fmaxf(res.y, 0.0f), fmaxf(res.z, 0.0f),
-                                        fmaxf(length(sub(S->ori, hit)), 0.0f));
-                const int mean_k = S->mean_k;
-                float rate = 1.0f / (float)(1 + mean_k);
-                float4 a = mean_k == 0 ? make_float4(0, 0, 0, 0) : S->accum[pix];
-                S->accum[pix] = make_float4(lerp(a.x, v4.x, rate), lerp(a.y, v4.y, rate), lerp(a.z, v4.z, rate),
-                                            lerp(a.w, v4.w, rate));
-            }
-        } else {
-            const int r = tile * 128 + G.t;
-            const bool valid = r < A.n;
-            float gamma = valid ? A.gamma[r] : 0.0f;
-            RowFeatures src{A.feat + (size_t)r * 576, valid, A.feat_vec};
-            st = tc_network<EB, COL>(G, st, src, aux_s, gamma, A.g, A.sr, o);
-            if (valid && !(st & kStFailed)) {
-                A.out3[3 * (size_t)r] = o[0];
-                A.out3[3 * (size_t)r + 1] = o[1];
-                A.out3[3 * (size_t)r + 2] = o[2];
-            }
-        }
+        st = tile_work<STAGED>(A, segs, seg_start, rows, tile, G.t, true,
+                               [&](const auto& src, float gamma, float g, f3 sr, float* o) {
+                                   return tc_network<EB, COL>(G, st, src, aux_s, gamma, g, sr, o);
+                               });
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -1016,18 +1411,25 @@ static size_t tc_smem_bytes(int eb, int groups) {
            (kTcMaxSegments + 1 + 3) * sizeof(int) + 16 + kAuxCount * sizeof(float);
 }
 
-template <int EB, bool STAGED, bool COL>
+template <int EB, bool STAGED, bool COL, bool SPLIT = false>
 static cudaError_t launch_tc(TcArgs& a, int sms, cudaStream_t s) {
+    auto kernel = k_mlp_tc<EB, STAGED, COL, SPLIT>;
     size_t smem = tc_smem_bytes(EB, kGroups<COL>);
-    cudaError_t e = cudaFuncSetAttribute(k_mlp_tc<EB, STAGED, COL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(a.tile_counter, 0, sizeof(int), s)) != cudaSuccess) return e;
-    k_mlp_tc<EB, STAGED, COL><<<sms, kGroups<COL> * kGroupThreads, smem, s>>>(a);
+    if (!SPLIT && (e = cudaMemsetAsync(a.tile_counter, 0, sizeof(int), s)) != cudaSuccess) return e;
+    kernel<<<sms, kGroups<COL> * kGroupThreads, smem, s>>>(a);
     return cudaGetLastError();
 }
+// most: the most sets or records there can be (how many there are may be
+// known on the device only).  Up to one tile an SM a tile's latency is the
+// call's, and the groups share it; from there on more tiles in flight are
+// worth more.
 template <bool STAGED>
-static cudaError_t launch_tc(TcArgs& a, bool fp8, bool coloured, int sms, cudaStream_t s) {
+static cudaError_t launch_tc(TcArgs& a, bool fp8, bool coloured, size_t most, int sms, cudaStream_t s) {
     if (coloured) return fp8 ? launch_tc<1, STAGED, true>(a, sms, s) : launch_tc<2, STAGED, true>(a, sms, s);
+    if (most <= (size_t)sms * 128)
+        return fp8 ? launch_tc<1, STAGED, false, true>(a, sms, s) : launch_tc<2, STAGED, false, true>(a, sms, s);
     return fp8 ? launch_tc<1, STAGED, false>(a, sms, s) : launch_tc<2, STAGED, false>(a, sms, s);
 }
 static bool is_coloured(f3 sr) { return !(sr.x == sr.y && sr.x == sr.z); }
@@ -1053,7 +1455,7 @@ cudaError_t tc_launch_mlp(const TcWeights& w, bool fp8, const float* feat, const
     a.g = g;
     a.sr = mk3(sr[0], sr[1], sr[2]);
     a.out3 = out3;
-    return launch_tc<false>(a, fp8, is_coloured(a.sr), sms, s);
+    return launch_tc<false>(a, fp8, is_coloured(a.sr), (size_t)n, sms, s);
 }
 
 cudaError_t tc_launch_mlp_at(const TcWeights& w, bool fp8, const float* feat, const float* gamma, float g,
@@ -1072,7 +1474,7 @@ cudaError_t tc_launch_mlp_at(const TcWeights& w, bool fp8, const float* feat, co
     a.out3 = out3;
     cudaError_t e = cudaMemsetAsync(err, 0, sizeof(int), s);
     if (e != cudaSuccess) return e;
-    return launch_tc<false>(a, fp8, is_coloured(a.sr), sms, s);
+    return launch_tc<false>(a, fp8, is_coloured(a.sr), (size_t)n, sms, s);
 }
 
 TcSegment tc_segment(const VolumeDev& v, const ViewDev& view, const HitRecords& rec, const float* feat,
@@ -1090,6 +1492,7 @@ TcSegment tc_segment(const VolumeDev& v, const ViewDev& view, const HitRecords& 
     q.ori = view.ori;
     q.g = view.g;
     q.mean_k = view.mean_k;
+    q.most = (size_t)view.width * view.height;
     return q;
 }
 
@@ -1103,7 +1506,7 @@ cudaError_t tc_launch_mlp_rec(const TcWeights& w, bool fp8, const VolumeDev& v, 
     a.segs = nullptr;
     a.nseg = 1;
     a.seg0 = tc_segment(v, view, rec, feat, accum);
-    return launch_tc<true>(a, fp8, is_coloured(a.seg0.sr), sms, s);
+    return launch_tc<true>(a, fp8, is_coloured(a.seg0.sr), a.seg0.most, sms, s);
 }
 
 cudaError_t tc_launch_mlp_segments(const TcWeights& w, bool fp8, const TcSegment* d_segs, const TcSegment* h_segs,
@@ -1116,8 +1519,12 @@ cudaError_t tc_launch_mlp_segments(const TcWeights& w, bool fp8, const TcSegment
     a.segs = d_segs;
     a.nseg = nseg;
     bool coloured = false;
-    for (int q = 0; q < nseg; ++q) coloured = coloured || is_coloured(h_segs[q].sr);
-    return launch_tc<true>(a, fp8, coloured, sms, s);
+    size_t most = 0;   // (up to 127 rows of a segment's last tile stay empty)
+    for (int q = 0; q < nseg; ++q) {
+        coloured = coloured || is_coloured(h_segs[q].sr);
+        most += (h_segs[q].most + 127) / 128 * 128;
+    }
+    return launch_tc<true>(a, fp8, coloured, most, sms, s);
 }
 
 // ---------------------------------------------------------------------------

@@ -36,6 +36,7 @@ struct TcSegment {
     f3 light_color, scatter_rate, ori;
     float g;
     int mean_k;
+    size_t most;                 // records there can be (the view's pixels)
 };
 constexpr int kTcMaxSegments = 64;
 struct HitRecords;
@@ -47,7 +48,7 @@ void tc_free_scratch(TcScratch& s);
 cudaError_t tc_launch_mlp(const TcWeights& w, bool fp8, const float* feat, const float* gamma, float g, const float sr[3],
                           int n, float* out3, int sms, cudaStream_t s);
 // Same launch with the tile counter and the error flag at caller-given device
-// addresses instead of the ones in TcWeights (both zeroed on `s` first).
+// addresses instead of the ones in TcWeights (zeroed on `s` first where used).
 cudaError_t tc_launch_mlp_at(const TcWeights& w, bool fp8, const float* feat, const float* gamma, float g,
                              const float sr[3], int n, float* out3, int* tile_counter, int* err, int sms,
                              cudaStream_t s);

@@ -37,3 +37,16 @@ def test_forms_agree(n, precision):
     np.testing.assert_array_equal(a[:, 2], b[:, 0])
     k = n // 2
     np.testing.assert_array_equal(run(feat[k:], gamma[k:], (0.99,) * 3, precision), grey[k:])
+
+
+@pytest.mark.parametrize("precision", [1, 2])   # BF16, FP8
+def test_split_tiles_agree(precision):
+    """Calls of no more tiles than SMs give a row three threads: the same bits
+    as the same sets among more tiles."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    feat, gamma = sets(sms * 128 + 1)
+    grey = run(feat, gamma, (0.97,) * 3, precision)
+    for k in (1, 31, 128, 129, 300, sms * 128):
+        np.testing.assert_array_equal(run(feat[:k], gamma[:k], (0.97,) * 3, precision), grey[:k])
+    np.testing.assert_array_equal(run(feat[-77:], gamma[-77:], (0.97,) * 3, precision, shift=1), grey[-77:])
