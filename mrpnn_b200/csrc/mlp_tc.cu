@@ -455,6 +455,7 @@ MRP_D void copy16(uint32_t dst, const void* src) {
 MRP_D void copy4(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
+MRP_D void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 constexpr int kStageStride = 3 * kGroupThreads * 16;   // bytes between a thread's chunks in SplitScratch::stage
 MRP_D void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
@@ -479,6 +480,7 @@ struct RowFeatures {           // [n][576] row-major
             for (int i = 0; i < W; ++i) xs[i] = valid ? __ldg(p + i) : 0.0f;
         }
     }
+    MRP_D void prefetch(int, int) const {}   // (a line holds several blocks' slices: no gain)
     // the slice as 16-byte chunks, chunk i at slot + i * kStageStride; staged
     // reads them back
     MRP_D void stage(int c, int from, int w, uint32_t slot) const {
@@ -511,6 +513,15 @@ struct TileFeatures {          // FP16 pairs of the staged predictor's tiled lay
             xs[2 * k] = p.x;
             xs[2 * k + 1] = p.y;
         }
+    }
+    // Asks L2 for the next block's slices, a lane a line (a pair's 32 lanes
+    // share it): the features of a large frame come from HBM.  1080p frame
+    // 2.480 -> 2.461 ms; two blocks ahead 2.467.
+    MRP_D void prefetch(int from, int w) const {
+        const int k = threadIdx.x & 31;
+        if (!valid || k >= w / 2) return;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) prefetch_l2(x + (c * 96 + (from >> 1) + k) * 32);
     }
     MRP_D void stage(int c, int from, int w, uint32_t slot) const {
         if (!valid) return;
@@ -617,6 +628,7 @@ __device__ __noinline__ int tc_block(const Group G, int st, const Src src, const
         p8[c] = s / (float)W;
         p8[3 + c] = m;
     }
+    if (b < 11) src.prefetch(c_blocks[b + 1].from, c_blocks[b + 1].w);
     p8[6] = g;
     p8[7] = gamma;
     // LSEFin1 (75 -> 16) accumulated block by block in TMEM: pool[pid + c] =
