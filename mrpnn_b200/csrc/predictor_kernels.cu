@@ -371,7 +371,7 @@ MRP_D void gather_sample(const VolumeDev& v, const PixelFrame& f, int i, float* 
 struct HgFast {
     f3 q;
     float u1L, u2L;          // LUT coordinates of the light-ray points
-    const float* lut_dirs;   // null: compute X_Hg the exact way
+    const float* lut_dirs;
 };
 MRP_D HgFast hg_fast(const VolumeDev& v, const PixelFrame& f) {
     HgFast h;
@@ -383,10 +383,26 @@ MRP_D HgFast hg_fast(const VolumeDev& v, const PixelFrame& f) {
 }
 __global__ void k_lut_dirs(const float* __restrict__ lut, float* __restrict__ out) {
     int i = threadIdx.x;
-    if (i < 160) out[i] = tex_lut_fast(lut, fmaf(c_udirs[3 * i], 0.5f, 0.5f), c_lutv[i]);
+    if (blockIdx.x == 192) {
+        if (i < 160) out[i] = tex_lut_fast(lut, fmaf(c_udirs[3 * i], 0.5f, 0.5f), c_lutv[i]);
+        return;
+    }
+    // point blockIdx.x's row: tex_lut_fast's y and its blend of two texels
+    const float py = fmaf(c_lutv[blockIdx.x], (float)kLut, -0.5f), fly = floorf(py), wy = py - fly;
+    const int y = (int)fly;
+    const float* r0 = lut + min(max(y, 0), kLut - 1) * kLut;
+    const float* r1 = lut + min(max(y + 1, 0), kLut - 1) * kLut;
+    float* row = out + (kLutRows - kLut * kLut) + blockIdx.x * kLutRow;
+    for (int x = i - 1; x <= kLut; x += blockDim.x) {
+        const int x0 = min(max(x, 0), kLut - 1);
+        row[x + 1] = lerp_fast(r0[x0], r1[x0], wy);
+    }
+}
+MRP_D const float* lut_row(const VolumeDev& v, int i) {
+    return v.lut_dirs + (kLutRows - kLut * kLut) + i * kLutRow;
 }
 cudaError_t launch_lut_dirs(const float* lut, float* out, cudaStream_t s) {
-    k_lut_dirs<<<1, 160, 0, s>>>(lut, out);
+    k_lut_dirs<<<193, 256, 0, s>>>(lut, out);
     return cudaGetLastError();
 }
 
@@ -439,16 +455,16 @@ MRP_D void gather_point_fast(const VolumeDev& v, const PixelFrame& f, const RunL
     *fd_ = feature_log<FP16>(fmaf(f.alpha * dens, 0.015625f, 1.0f));
     if (i == 0) {
         *fh_ = feature_log<FP16>(hg(dot(f.X, f.L), f.g) + 1.0f);
-    } else if (FP16 && H.lut_dirs) {
-        const float lv = p1.w;
+    } else if (FP16) {
+        const float* row = lut_row(v, i);
         float a, b;
         if (!R.light) {
             const float c2 = fmaf(H.q.z, p1.z, fmaf(H.q.y, p1.y, H.q.x * p1.x));
             a = __ldg(H.lut_dirs + i);
-            b = tex_lut_fast(v.lut, fmaf(c2, 0.5f, 0.5f), lv);
+            b = lut_row_fast(row, fmaf(c2, 0.5f, 0.5f));
         } else {
-            a = tex_lut_fast(v.lut, H.u1L, lv);
-            b = tex_lut_fast(v.lut, H.u2L, lv);
+            a = lut_row_fast(row, H.u1L);
+            b = lut_row_fast(row, H.u2L);
         }
         *fh_ = feature_log<FP16>(fmaf(a, b, 1.0f));
     } else {
@@ -457,9 +473,8 @@ MRP_D void gather_point_fast(const VolumeDev& v, const PixelFrame& f, const RunL
         ms = mk3(ms.x * rl, ms.y * rl, ms.z * rl);
         float c1 = fmaf(f.X.z, ms.z, fmaf(f.X.y, ms.y, f.X.x * ms.x));
         float c2 = fmaf(f.LX.z, ms.z, fmaf(f.LX.y, ms.y, f.LX.x * ms.x));
-        float lv = p1.w;
-        *fh_ = feature_log<FP16>(fmaf(tex_lut_fast(v.lut, fmaf(c1, 0.5f, 0.5f), lv), tex_lut_fast(v.lut, fmaf(c2, 0.5f, 0.5f), lv),
-                         1.0f));
+        const float* row = lut_row(v, i);
+        *fh_ = feature_log<FP16>(fmaf(lut_row_fast(row, fmaf(c1, 0.5f, 0.5f)), lut_row_fast(row, fmaf(c2, 0.5f, 0.5f)), 1.0f));
     }
     // ShadowTerm_TRs: outside the box, the TR where the light ray enters it
     const f3 p = cur, light = f.LX;

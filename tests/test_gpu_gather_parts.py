@@ -31,3 +31,25 @@ def test_parts_do_not_show(precision, hardware):
     assert (whole.sum(1) > 0.2).mean() > 0.3   # a good part of the rays hit the cloud
     for n in (1, 127, 129, 1000):
         np.testing.assert_array_equal(radiances(n), whole[:n])
+
+
+@pytest.mark.parametrize("g", [0.3, 0.857])
+@pytest.mark.parametrize("sign", [1, -1])
+def test_phase_rows_at_the_ends(sign, g):
+    """The phase features with the light along the view, whose cosines lie at
+    the ends of the points' rows of the phase table.  A cosine differs from the
+    oracle's by a few ulp, 2e-7, which is 5e-5 of a texel; neighbouring texels
+    of the cone-averaged table differ by less than a factor of 2, two factors:
+    1e-4, and once more for their blend's rounding."""
+    from oracle import oracle as O
+    sc = Scene(R=64, g=g)
+    W = 32
+    ori, up, right = view_frame()
+    light = (sign * ori / np.linalg.norm(ori)).astype(np.float32)
+    _, aux, feat = sc.vol.predict_debug(sc.vol.make_view((W, W), ori, up, right, light, g, sc.alpha, seed=3))
+    view = O.make_view(W, W, ori, up, right, light, alpha=sc.alpha, g=g, seed=3, frame=0)
+    _, ref, _, hits = O.predict_pixels(sc.orc, view, np.arange(W * W, dtype=np.int32), want_features=True)
+    hit = hits[:, 3] > 0
+    assert hit.sum() > 100
+    np.testing.assert_array_equal(aux[:, 3] > 0, hit)
+    np.testing.assert_allclose(feat[hit, 384:], ref[hit, 384:], rtol=2e-4, atol=1e-6)
