@@ -735,27 +735,27 @@ MRP_D void hit_pixels(const VolumeDev& v, const ViewDev& w, const HitRecords& re
 #pragma unroll
     for (int k = 0; k < 16; ++k) f[k * cap] = vals[k];
 }
-// Persistent warps: each takes the next tile of 8 x 4 pixels from a
-// counter (rec.count[1]) as soon as its previous 32 rays have ended, so a
+// Persistent warps: each takes the next tile of 2^lsx x 2^lsy pixels (8 x 4;
+// fewer in small launches, launch_hit) from a counter (rec.count[1]) as soon
+// as its previous rays have ended, so a
 // long march holds one warp, not a whole block, and the SMs stay full until
 // the last tiles are handed out; the rays of a square-ish tile march more
 // alike than 32 pixels of a row.  (Explicit rays, a width x 1 launch, come
-// 32 in a row.)
+// in a row.)
 template <bool COUNT, class DT, bool ENV = false>
-__global__ void __launch_bounds__(kHitThreads, 8) k_hit(VolumeDev v, ViewDev w, HitRecords rec, float4* __restrict__ accum) {
-    const int tx = w.height > 1 ? (w.width + 7) >> 3 : (w.width + 31) >> 5;
-    const int ty = w.height > 1 ? (w.height + 3) >> 2 : 1;
-    const int nchunks = tx * ty;
+__global__ void __launch_bounds__(kHitThreads, 8) k_hit(VolumeDev v, ViewDev w, HitRecords rec, float4* __restrict__ accum,
+                                                       int lsx, int lsy) {
+    const int sx = 1 << lsx, sy = 1 << lsy;
+    const int tx = (w.width + sx - 1) >> lsx, nchunks = tx * ((w.height + sy - 1) >> lsy);
     const int lane = (int)(threadIdx.x & 31);
-    const int lx = w.height > 1 ? lane & 7 : lane, ly = w.height > 1 ? lane >> 3 : 0;
-    const int sx = w.height > 1 ? 8 : 32, sy = w.height > 1 ? 4 : 1;
+    const int lx = lane & (sx - 1), ly = lane >> lsx;
     for (;;) {
         int c = 0;
         if (lane == 0) c = atomicAdd(rec.count + 1, 1);
         c = __shfl_sync(0xffffffffu, c, 0);
         if (c >= nchunks) return;
         const int col = (c % tx) * sx + lx, row = (c / tx) * sy + ly;
-        hit_pixels<COUNT, DT, ENV>(v, w, rec, accum, col < w.width && row < w.height ? row * w.width + col : -1);
+        hit_pixels<COUNT, DT, ENV>(v, w, rec, accum, ly < sy && col < w.width && row < w.height ? row * w.width + col : -1);
     }
 }
 
@@ -836,19 +836,28 @@ cudaError_t launch_hit(const VolumeDev& v, const ViewDev& view, HitRecords rec, 
     if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
         return e;
-    const int need = (n + kHitThreads - 1) / kHitThreads;
+    // A warp's pixels: 8 x 4, or 4 x 4 or 4 x 2 (explicit rays: in a row) where
+    // that makes at most sixteen warps an SM.  There the longest march of a
+    // warp is the launch's time, and fewer lanes share its branches: 163 x 97
+    // over 100^3, four launches, 529 -> 510 us, 128 x 128 over 256^3 228 -> 213;
+    // from 256 x 256 on full warps are as fast (268 both) and then faster
+    // (512 x 512: 500 against 543 with half of the lanes).
+    const int lp = n <= sms * 128 ? 3 : n <= sms * 256 ? 4 : 5;
+    const int lsy = view.height > 1 ? lp / 2 : 0, lsx = lp - lsy;
+    const int chunks = ((view.width + (1 << lsx) - 1) >> lsx) * ((view.height + (1 << lsy) - 1) >> lsy);
+    const int need = (chunks + kHitThreads / 32 - 1) / (kHitThreads / 32);
     const int blocks = need < sms * 8 ? need : sms * 8;   // eight resident per SM
     // one copy of the march per counting mode and density storage type, and
     // for volumes with an environment map
     if (v.hdri) {
-        if (v.density_h) k_hit<false, __half, true><<<blocks, kHitThreads, 0, s>>>(v, view, rec, accum);
-        else k_hit<false, float, true><<<blocks, kHitThreads, 0, s>>>(v, view, rec, accum);
+        if (v.density_h) k_hit<false, __half, true><<<blocks, kHitThreads, 0, s>>>(v, view, rec, accum, lsx, lsy);
+        else k_hit<false, float, true><<<blocks, kHitThreads, 0, s>>>(v, view, rec, accum, lsx, lsy);
     } else if (v.density_h) {
-        if (view.counters) k_hit<true, __half><<<blocks, kHitThreads, 0, s>>>(v, view, rec, accum);
-        else k_hit<false, __half><<<blocks, kHitThreads, 0, s>>>(v, view, rec, accum);
+        if (view.counters) k_hit<true, __half><<<blocks, kHitThreads, 0, s>>>(v, view, rec, accum, lsx, lsy);
+        else k_hit<false, __half><<<blocks, kHitThreads, 0, s>>>(v, view, rec, accum, lsx, lsy);
     } else {
-        if (view.counters) k_hit<true, float><<<blocks, kHitThreads, 0, s>>>(v, view, rec, accum);
-        else k_hit<false, float><<<blocks, kHitThreads, 0, s>>>(v, view, rec, accum);
+        if (view.counters) k_hit<true, float><<<blocks, kHitThreads, 0, s>>>(v, view, rec, accum, lsx, lsy);
+        else k_hit<false, float><<<blocks, kHitThreads, 0, s>>>(v, view, rec, accum, lsx, lsy);
     }
     return cudaGetLastError();
 }

@@ -53,3 +53,24 @@ def test_phase_rows_at_the_ends(sign, g):
     assert hit.sum() > 100
     np.testing.assert_array_equal(aux[:, 3] > 0, hit)
     np.testing.assert_allclose(feat[hit, 384:], ref[hit, 384:], rtol=2e-4, atol=1e-6)
+
+
+@pytest.mark.parametrize("W,H", [(37, 23), (163, 149), (201, 190)])
+def test_march_tiles(W, H):
+    """8, 16 and 32 pixels a warp, over images that their tiles do not divide:
+    pixels all over the frame, its last rows and columns among them, against the
+    oracle to the FP32 predictor's bound."""
+    import mrpnn_b200 as M
+    from oracle import oracle as O
+    sc = Scene(R=64)
+    ori, up, right = view_frame()
+    got = sc.vol.Render((W, H), ori, up, right, LIGHT, M.VolumeRender.MRPNN, sc.g, sc.alpha, sampleNum=1,
+                        seed=3).reshape(-1, 4)
+    yx = np.random.default_rng(W).integers(0, (H, W), (300, 2))
+    yx[:40, 0] = H - 1 - np.arange(40) % 2
+    yx[40:80, 1] = W - 1 - np.arange(40) % 2
+    pix = np.unique(yx[:, 0] * W + yx[:, 1]).astype(np.int32)
+    view = O.make_view(W, H, ori, up, right, LIGHT, alpha=sc.alpha, g=sc.g, seed=3, frame=0)
+    ref = O.predict_pixels(sc.orc, view, pix)
+    assert (ref[:, 3] > 0).sum() > 50
+    np.testing.assert_allclose(got[pix], ref, rtol=1e-4, atol=1e-6)
