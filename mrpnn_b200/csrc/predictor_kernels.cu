@@ -35,16 +35,19 @@ __constant__ float4 c_pt0[192], c_pt1[192];
 
 // The 192 points as the runs of GetSamples23_'s layout: layers 0..7 over the
 // 160 rotated directions (8, 8, 16, 16, 16, 32, 32, 32 points), then layers
-// 0..3 on the light ray (8 points each).  set_stencil_tables checks that the
-// tables it loads have this layout.
-constexpr int kStencilRuns[12][3] = {{0, 0, 8},     {1, 8, 16},    {2, 16, 32},   {3, 32, 48},
-                                     {4, 48, 64},   {5, 64, 96},   {6, 96, 128},  {7, 128, 160},
-                                     {0, 160, 168}, {1, 168, 176}, {2, 176, 184}, {3, 184, 192}};
-__constant__ int c_stencil_runs[12][3] = {{0, 0, 8},     {1, 8, 16},    {2, 16, 32},   {3, 32, 48},
-                                          {4, 48, 64},   {5, 64, 96},   {6, 96, 128},  {7, 128, 160},
-                                          {0, 160, 168}, {1, 168, 176}, {2, 176, 184}, {3, 184, 192}};
-// The runs in six parts of 32 points each: first run of part p, and the end.
-__constant__ int c_stencil_parts[7] = {0, 3, 5, 6, 7, 8, 12};
+// 0..3 on the light ray (8 points each); the runs of 32 in halves, for the
+// parts below.  set_stencil_tables checks that the tables it loads have this
+// layout.
+constexpr int kRuns = 15;
+#define MRP_STENCIL_RUNS                                                                                              \
+    {{0, 0, 8}, {1, 8, 16}, {2, 16, 32}, {3, 32, 48}, {4, 48, 64}, {5, 64, 80}, {5, 80, 96}, {6, 96, 112},            \
+     {6, 112, 128}, {7, 128, 144}, {7, 144, 160}, {0, 160, 168}, {1, 168, 176}, {2, 176, 184}, {3, 184, 192}}
+constexpr int kStencilRuns[kRuns][3] = MRP_STENCIL_RUNS;
+__constant__ int c_stencil_runs[kRuns][3] = MRP_STENCIL_RUNS;
+#undef MRP_STENCIL_RUNS
+// The runs in six parts of 32 points each and in twelve of 16: first run of
+// part p, and the end.
+__constant__ int c_stencil_parts[2][13] = {{0, 3, 5, 7, 9, 11, kRuns}, {0, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 13, kRuns}};
 cudaError_t set_stencil_tables(const StencilTables& t) {
     cudaError_t e;
     // the staged gather is compiled for the runs of kStencilRuns
@@ -493,7 +496,7 @@ MRP_D void gather_point_fast(const VolumeDev& v, const PixelFrame& f, const RunL
     }
     *fs_ = tr;
 }
-// The points of runs [first_run, end_run) (0, 12: all 192), run by run (GetSamples23_'s layout: layers 0..7 over the
+// The points of runs [first_run, end_run) (0, kRuns: all 192), run by run (GetSamples23_'s layout: layers 0..7 over the
 // 160 rotated directions, then layers 0..3 on the light ray), into a tiled
 // feature layout: fp32 (record r, channel c, sample i at word
 // ((r / 32) * 576 + c * 192 + i) * 32 + r % 32), or FP16 pairs (samples 2k,
@@ -779,10 +782,11 @@ __global__ void __launch_bounds__(128) k_gather_rec(VolumeDev v, ViewDev w, HitR
     int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= *rec.count) return;
     PixelFrame pf = record_frame(rec, r, normalize(w.light_dir), w.g, w.alpha);
-    int first_run = 0, end_run = 12;
-    if (gridDim.y > 1) {   // one of the six parts of the stencil
-        first_run = c_stencil_parts[blockIdx.y];
-        end_run = c_stencil_parts[blockIdx.y + 1];
+    int first_run = 0, end_run = kRuns;
+    if (gridDim.y > 1) {   // one of six or twelve parts of the stencil
+        const int* parts = c_stencil_parts[gridDim.y == 6 ? 0 : 1];
+        first_run = parts[blockIdx.y];
+        end_run = parts[blockIdx.y + 1];
     }
     if (TEX) gather_all_tex(v, pf, feat, r, first_run, end_run);
     else gather_all_fast<FP16>(v, pf, feat, r, first_run, end_run);
@@ -1170,14 +1174,22 @@ cudaError_t launch_gather_rec(const VolumeDev& v, const ViewDev& view, HitRecord
                               cudaStream_t s) {
     int n = view.width * view.height;
     if (n <= 0) return cudaSuccess;
+    int dev = 0, sms = 0;
+    cudaError_t e;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        return e;
     // A record's 192 points in series take 100 us (texture form; 170 us the
     // FP32 form) however few records there are; six threads a record, 32
     // points each, take 28 us (53 us) for small frames and still 239 against
     // 249 us at 724^2 pixels.  At 1024^2 (half of them hits) the records fill
     // the SMs by themselves: 465 against 444 us for the texture form, while
     // the FP32 form, waiting for its loads, still gains (961 against 978 us).
-    const bool parts = !fp16 || n <= 600000;
-    const dim3 grid((n + 127) / 128, parts ? 6 : 1);
+    // Twelve threads of 16 points where even six leave the SMs short of warps:
+    // 163 x 97, four launches, 510 -> 487 us, 128 x 128 213 -> 208, 256 x 256
+    // 269 -> 266, 320 x 240 as before, 384 x 384 451 -> 460.
+    const int parts = n <= sms * 512 ? 12 : !fp16 || n <= 600000 ? 6 : 1;
+    const dim3 grid((n + 127) / 128, parts);
     if (fp16 && v.glut_tex) k_gather_rec<true, true><<<grid, 128, 0, s>>>(v, view, rec, feat);
     else if (fp16) k_gather_rec<true><<<grid, 128, 0, s>>>(v, view, rec, feat);
     else k_gather_rec<false><<<grid, 128, 0, s>>>(v, view, rec, feat);

@@ -74,3 +74,26 @@ def test_march_tiles(W, H):
     ref = O.predict_pixels(sc.orc, view, pix)
     assert (ref[:, 3] > 0).sum() > 50
     np.testing.assert_allclose(got[pix], ref, rtol=1e-4, atol=1e-6)
+
+
+@pytest.mark.parametrize("precision,hardware", [(1, True), (1, False), (0, False)])
+def test_six_and_twelve_parts(precision, hardware):
+    """Launches on either side of the line between six and twelve threads a
+    record: the same rays, the same bits."""
+    import torch
+
+    import mrpnn_b200 as M
+    sc = Scene(R=64)
+    sc.vol.SetPrecision(precision)
+    sc.vol.SetGatherFilter(hardware)
+    ori, up, right = view_frame()
+    n = 512 * torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(8)
+    d = -ori / np.linalg.norm(ori) + rng.uniform(-1, 1, (n + 1, 1)) * right + rng.uniform(-1, 1, (n + 1, 1)) * up
+    d = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+
+    def radiances(k):
+        return sc.vol.GetRadiances(np.broadcast_to(ori, (k, 3)), d[:k], LIGHT, (1, 1, 1), sc.alpha, 1, sc.g, 1,
+                                   M.VolumeRender.MRPNN)
+
+    np.testing.assert_array_equal(radiances(n), radiances(n + 1)[:n])
