@@ -585,13 +585,6 @@ MRP_D float density_occ(const VolumeDev& v, f3 p) {
         return v.occ ? tex3_occ(v.density_h, v.res, v.occ, v.occ_res, p) : tex3<false>(v.density_h, v.res, p);
     else return v.density_h ? density_occ<__half>(v, p) : density_occ<float>(v, p);
 }
-// Mip level m of the pyramid (256 >> m) at p, with bricks for m < kOccMips.
-MRP_D float mip_density(const VolumeDev& v, int m, f3 p) {
-    const float* g = v.mips + mip_offset(m);
-    int n = 256 >> m;
-    if (v.mip_occ && m < kOccMips) return tex3_occ(g, n, v.mip_occ + mip_occ_offset(m), 32 >> m, p);
-    return tex3<false>(g, n, p);
-}
 
 // ---------------------------------------------------------------------------
 // Tr (core/render.cuh:60-103): ratio tracking while tr > 0.5, then delta

@@ -386,7 +386,6 @@ MRP_D void store_part(const Group& G, int p, const float (&v)[32], float inv) {
     }
 }
 
-MRP_D float wl(const float* __restrict__ w, int i) { return __ldg(w + i); }
 MRP_D float sigmoid_d(float o) { return 1.0f / (1.0f + __expf(-o)); }
 
 // relu(D * scale + b) for N columns of layer L (runtime), in place.
@@ -875,7 +874,8 @@ __device__ __noinline__ TailOut tc_tail(const Group G, int st, const float* aux,
 // a row, two thirds of them in the SE blocks (9 to 10 k a block of width 32, a
 // third of that for its features to arrive); 70 k split, the next block's
 // features copied to shared memory meanwhile (4 k a block).  The call 83.5 ->
-// 63 us; a 163 x 97 FP8 frame of four launches 587 -> 528 us.
+// 70 us; a 163 x 97 FP8 frame of four launches 587 -> 528 us.  (With twice as
+// many sets, two tiles in turn an SM: 107 us the other form, 127 split.)
 // ---------------------------------------------------------------------------
 struct SplitScratch {
     float4 stage[8][3 * kGroupThreads];   // the threads' slices of the next block (chunk, thread)
