@@ -613,6 +613,7 @@ MRP_D float density(const VolumeDev& v, f3 p) { return density_tex(v, p); }
 // of a voxel is far above the rounding here); t_in > t_out when the ray
 // misses it, everything when no box was computed.
 struct BoxSpan { float t_in, t_out; };
+constexpr BoxSpan kOpenSpan{-INFINITY, INFINITY};
 MRP_D BoxSpan nonzero_span(const VolumeDev& v, f3 p, f3 L) {
     BoxSpan b{0.0f, 3.0e38f};
     if (!v.has_bounds) return b;
@@ -635,7 +636,8 @@ MRP_D BoxSpan nonzero_span(const VolumeDev& v, f3 p, f3 L) {
 // draws and the same estimate.  Density 0 leaves tr as it is in both loops,
 // so no texel is read before t_in, and past t_out the walk can end: its
 // remaining steps only use up draws that nobody reads.  (Needs t to grow,
-// smax > 0 and tr_scale > 0; the caller opens the span otherwise.)
+// smax > 0 and tr_scale > 0; kOpenSpan, which takes nothing from the walk,
+// is for the walks that go backwards or stand still.)
 template <class DT>
 MRP_D float transmittance_span(const VolumeDev& v, Stream& st, f3 pos, f3 dir, float dis, float alpha, BoxSpan span) {
     const float smax = fm(v.max_density, alpha);
@@ -687,7 +689,7 @@ __global__ void __launch_bounds__(128) k_baked_tr(float* __restrict__ out, const
         f3 p = subs(uv, 0.5f);
         uint32_t hi = (uint32_t)(vi >> 32) * 8u;
         const float md = ray_box_distance(p, L);
-        const BoxSpan span = grows ? nonzero_span(v, p, L) : BoxSpan{0.0f, 3.0e38f};
+        const BoxSpan span = grows ? nonzero_span(v, p, L) : kOpenSpan;
         float res;
         if (replicate) {
             Stream st(kBakeStream, (uint32_t)vi, hi, 0, seed);

@@ -137,3 +137,32 @@ def test_pyramid_levels(R):
     ref = O.split_levels(O.build_pyramid(data, R), O.mip_sizes())
     for m in range(9):
         np.testing.assert_array_equal(v.read(M.api.RES_MIP, m), ref[m].ravel(), err_msg=f"mip {m}")
+
+
+def bake(R, data, B, light, alpha, replicate, tr_scale=1.0, majorant=None):
+    """A baked grid and the oracle's, from the same draws."""
+    import mrpnn_b200 as M
+    M.init()
+    v = M.VolumeRender(R)
+    v.set_data(data)
+    v.Update()
+    if majorant is not None:
+        v.max_density = majorant
+    v.SetTrScale(tr_scale)
+    v.SetBakeResolution(B, replicate)
+    v.Update_CachedTR(light, alpha)
+    sc = O.SceneBuf(data.ravel(), R, v.max_density, tr_scale=tr_scale)
+    return (v.read(M.api.RES_BAKED_TR),
+            O.baked_tr_voxels(sc, alpha, np.array(light, np.float32), B, 0, np.arange(B ** 3), replicate))
+
+
+@pytest.mark.parametrize("replicate", [True, False])
+@pytest.mark.parametrize("alpha,tr_scale", [(-40.0, 1.0), (40.0, -0.5)])
+def test_bake_walks_backwards(alpha, tr_scale, replicate):
+    """A negative extinction or step scale, which the entry points accept,
+    walks away from the light: the oracle's draws and its estimate.  The bar
+    is test_baked_voxels'; a third of the voxels and more see the blob
+    behind them."""
+    got, ref = bake(24, blob(24, (6, 6, 6), (18, 18, 18)), 9, (0.36, -0.48, 0.8), alpha, replicate, tr_scale)
+    assert np.mean(ref < 1.0) > 0.2
+    assert np.mean(np.abs(got - ref) > 1e-4) < 0.01
