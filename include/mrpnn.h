@@ -110,7 +110,10 @@ typedef struct mrp_volume_info {
     float max_density;
     int has_pyramid, has_lut, has_tr, has_baked_tr;
     float lut_g, tr_alpha, tr_light[3];
-    size_t device_bytes;
+    size_t device_bytes;     /* device memory held for the grid, everything
+                                derived from it and the baked grid; render
+                                buffers and textures, which the first call
+                                that needs them allocates, not counted */
 } mrp_volume_info;
 
 /* Resource selector for mrp_volume_read (readback for checking). */

@@ -288,13 +288,15 @@ mrp_status mrp_volume_create_ex(int res, mrp_storage storage, mrp_volume** out) 
     const size_t nocc = (size_t)v->occ_res * v->occ_res * v->occ_res,
                  nocc2 = (size_t)v->occ2_res * v->occ2_res * v->occ2_res,
                  nrow = std::max(occ_row_words(res), kMipOccRows);
-    if ((storage == MRP_STORAGE_FP16 ? (e = mrp::dev_malloc(&v->density_h, n * sizeof(__half)))
-                                     : (e = mrp::dev_malloc(&v->density, n * sizeof(float)))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->mips, (kMipFloats + kPadLevelFloats) * sizeof(float))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->trs, (kTrFloats + kPadLevelFloats) * sizeof(float))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->lut, kLutAlloc * sizeof(float))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->occ_rows, nrow * sizeof(uint4) + 32 + kMipOccBytes + nocc + nocc2)) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->mip_tr, (mip_tr_offset(5) + kTrPadTexels + kPadLevelFloats) * sizeof(float2))) != cudaSuccess)
+    auto hold = [&](auto** p, size_t bytes) {   // (get_info's device_bytes)
+        if ((e = mrp::dev_malloc(p, bytes)) == cudaSuccess) v->held_bytes += bytes;
+        return e == cudaSuccess;
+    };
+    if (!(storage == MRP_STORAGE_FP16 ? hold(&v->density_h, n * sizeof(__half)) : hold(&v->density, n * sizeof(float))) ||
+        !hold(&v->mips, (kMipFloats + kPadLevelFloats) * sizeof(float)) ||
+        !hold(&v->trs, (kTrFloats + kPadLevelFloats) * sizeof(float)) || !hold(&v->lut, kLutAlloc * sizeof(float)) ||
+        !hold(&v->occ_rows, nrow * sizeof(uint4) + 32 + kMipOccBytes + nocc + nocc2) ||
+        !hold(&v->mip_tr, (mip_tr_offset(5) + kTrPadTexels + kPadLevelFloats) * sizeof(float2)))
         return cleanup(fail(e == cudaErrorMemoryAllocation ? MRP_ERR_OOM : MRP_ERR_CUDA, "volume allocation: %s",
                             cudaGetErrorString(e)));
     v->mips_pad = v->mips + kMipFloats;
@@ -605,9 +607,7 @@ mrp_status mrp_volume_get_info(const mrp_volume* v, mrp_volume_info* info) {
     info->lut_g = v->lut_g;
     info->tr_alpha = v->tr_alpha;
     for (int i = 0; i < 3; ++i) info->tr_light[i] = v->tr_light[i];
-    size_t R = v->res;
-    info->device_bytes = R * R * R * (v->density_h ? 2 : 4) + kMipFloats * 4 + kTrFloats * 4 + kLut * kLut * 4 +
-                         (size_t)v->baked_alloc_res * v->baked_alloc_res * v->baked_alloc_res * 4;
+    info->device_bytes = v->held_bytes + (size_t)v->baked_alloc_res * v->baked_alloc_res * v->baked_alloc_res * sizeof(float);
     return MRP_OK;
 }
 

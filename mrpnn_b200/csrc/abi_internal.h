@@ -105,6 +105,7 @@ struct mrp_volume {
     float* lut = nullptr;
     float* baked = nullptr;
     int baked_alloc_res = 0;
+    size_t held_bytes = 0;          // device memory allocated at creation
     uint8_t* occ = nullptr;
     uint8_t* mip_occ = nullptr;   // bricks of mip levels 0..kOccMips-1
     int occ_shift = 3, occ_res = 0;

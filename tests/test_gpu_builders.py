@@ -166,3 +166,29 @@ def test_bake_walks_backwards(alpha, tr_scale, replicate):
     got, ref = bake(24, blob(24, (6, 6, 6), (18, 18, 18)), 9, (0.36, -0.48, 0.8), alpha, replicate, tr_scale)
     assert np.mean(ref < 1.0) > 0.2
     assert np.mean(np.abs(got - ref) > 1e-4) < 0.01
+
+
+@pytest.mark.parametrize("R,storage", [(2, "fp32"), (64, "fp16"), (200, "fp32"), (1030, "fp16")])
+def test_device_bytes(R, storage):
+    """mrp_volume_info counts what a volume holds from its creation on and
+    the baked grid: the grid, the pyramid and TR levels with their padded,
+    paired and z-paired copies, the LUT with its tables, the occupancy with
+    its scratch rows."""
+    import mrpnn_b200 as M
+    M.init()
+    pad = 11 ** 3 + 7 ** 3 + 5 ** 3
+    floats = sum((256 >> m) ** 3 for m in range(9)) + pad + sum((128 >> m) ** 3 for m in range(8)) + pad
+    floats += 512 * 512 + 160 + 192 * 514
+    pairs = sum((256 >> m) ** 3 for m in range(1, 5)) + sum(((128 >> m) + 2) ** 3 for m in range(8)) + pad
+    rows = max(R * R * -(-R // 1024), sum((256 >> m) ** 2 for m in range(5)))
+    nb = -(-R // 8)
+    flags = sum((32 >> m) ** 3 for m in range(5)) + nb ** 3 + (-(-nb // 4)) ** 3 + 32
+    want = R ** 3 * (2 if storage == "fp16" else 4) + 4 * floats + 8 * pairs + 16 * rows + flags
+    v = M.VolumeRender(R, storage=storage)
+    assert v.info().device_bytes == want
+    if R == 64:
+        v.set_data(np.zeros((R, R, R), np.float32))
+        v.Update()
+        v.SetBakeResolution(21)
+        v.Update_CachedTR((0.0, 1.0, 0.0), 1.0)
+        assert v.info().device_bytes == want + 21 ** 3 * 4
