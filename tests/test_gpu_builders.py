@@ -192,3 +192,78 @@ def test_device_bytes(R, storage):
         v.SetBakeResolution(21)
         v.Update_CachedTR((0.0, 1.0, 0.0), 1.0)
         assert v.info().device_bytes == want + 21 ** 3 * 4
+
+
+@pytest.mark.parametrize("light", [(0.0, 1.0, 0.0), (0.0, 0.0, -1.0), (0.36, -0.48, 0.8)])
+@pytest.mark.parametrize("R,lo,hi,B", [(40, (30, 26, 12), (31, 27, 13), 53), (24, (17, 3, 9), (20, 6, 12), 29),
+                                       (32, (3, 9, 20), (4, 28, 21), 41)])
+def test_bake_small_boxes(light, R, lo, hi, B):
+    """One voxel, a small cube and a line of voxels, and a bake grid fine
+    enough that a hundred voxels and more see them.  The steps are far
+    shorter than a voxel, so the estimates' bar of 1e-4 holds as in
+    test_baked_voxels, and walks that take another course stay below 1 % of
+    the voxels that see the box."""
+    got, ref = bake(R, blob(R, lo, hi), B, light, 400.0, True)
+    seen = int(np.count_nonzero(ref < 1.0))
+    assert seen >= 100
+    assert np.count_nonzero(np.abs(got - ref) > 1e-4) <= 0.01 * seen
+
+
+@pytest.mark.parametrize("replicate", [True, False])
+def test_bake_majorant_below_density(replicate):
+    """A majorant set below the density makes single estimates negative (the
+    ratio factor 1 - S / majorant is); they enter the mean as they are."""
+    got, ref = bake(24, blob(24, (6, 6, 6), (18, 18, 18)), 13, (0.36, -0.48, 0.8), 40.0, replicate, majorant=0.4)
+    assert np.mean(ref < 0.0) > 0.01
+    assert np.mean(np.abs(got - ref) > 1e-4) < 0.01
+
+
+@pytest.mark.parametrize("light", [(float("nan"), 0.6, 0.8), (0.6, 0.8, float("nan")), (0.0, 0.0, 0.0)])
+def test_tr_levels_odd_lights(light):
+    """A light with a component that is not a number, whose rays have no place
+    in the cube and go by the general fetches, and one of no length, whose
+    steps stay where they are: what the oracle's fetches give (not a number
+    for the first two)."""
+    import mrpnn_b200 as M
+    M.init()
+    v = M.VolumeRender(24)
+    v.set_data(blob(24, (6, 6, 6), (18, 18, 18)))
+    v.Update()
+    v.Update_TR(light, 48.0)
+    mips = np.concatenate([v.read(M.api.RES_MIP, m) for m in range(9)])
+    got = np.concatenate([v.read(M.api.RES_TR, m) for m in range(8)])
+    ref = O.tr_mips(mips, 48.0, np.array(light, np.float32))
+    np.testing.assert_allclose(got, ref, rtol=2e-6, atol=1e-7)
+
+
+@pytest.mark.parametrize("axis,start", [(0, 0), (0, 1027), (1, 1027), (2, 0), (2, 1022), (2, 1027)])
+def test_scan_long_rows(axis, start):
+    """Rows longer than one mask segment (1024 voxels) in fp32: the occupancy
+    of a slab of three voxels, and its bounds, which decide where the walks of
+    a bake begin and end.  A ray toward the slab has 11 expected steps in it
+    (3 voxels of 1 / 1030 at 4000 a unit length) and reads 1 only where none
+    falls there: one voxel of 100 000; with bounds that miss the slab, every
+    one does."""
+    import torch
+
+    import mrpnn_b200 as M
+    M.init()
+    R, nb = 1030, 129
+    d = torch.zeros((R, R, R), device="cuda")
+    d.narrow(axis, start, 3).fill_(1.0)
+    v = M.VolumeRender(R)
+    torch.cuda.synchronize()
+    v.set_data(d)
+    del d
+    torch.cuda.empty_cache()
+    v.Update(process_mips=False)
+    want = np.zeros((nb, nb, nb), np.uint8)
+    bricks = [b for b in range(nb) if 8 * b - 1 <= start + 2 and start <= 8 * b + 9]
+    np.moveaxis(want, axis, 0)[bricks] = 1
+    np.testing.assert_array_equal(v.read(M.api.RES_OCCUPANCY).reshape(nb, nb, nb), want)
+    assert v.max_density == 1.0
+    light = np.zeros(3, np.float32)
+    light[axis] = 1.0 if start else -1.0
+    v.SetBakeResolution(13)
+    v.Update_CachedTR(light, 4000.0)
+    assert np.mean(v.read(M.api.RES_BAKED_TR) < 1.0) > 0.99
