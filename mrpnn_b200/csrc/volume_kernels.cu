@@ -613,7 +613,6 @@ MRP_D float density(const VolumeDev& v, f3 p) { return density_tex(v, p); }
 // of a voxel is far above the rounding here); t_in > t_out when the ray
 // misses it, everything when no box was computed.
 struct BoxSpan { float t_in, t_out; };
-constexpr BoxSpan kOpenSpan{-INFINITY, INFINITY};
 MRP_D BoxSpan nonzero_span(const VolumeDev& v, f3 p, f3 L) {
     BoxSpan b{0.0f, 3.0e38f};
     if (!v.has_bounds) return b;
@@ -635,9 +634,8 @@ MRP_D BoxSpan nonzero_span(const VolumeDev& v, f3 p, f3 L) {
 // Tr (transmittance, common.cuh) over the steps that can change it: the same
 // draws and the same estimate.  Density 0 leaves tr as it is in both loops,
 // so no texel is read before t_in, and past t_out the walk can end: its
-// remaining steps only use up draws that nobody reads.  (Needs t to grow,
-// smax > 0 and tr_scale > 0; kOpenSpan, which takes nothing from the walk,
-// is for the walks that go backwards or stand still.)
+// remaining steps only use up draws that nobody reads.  (Needs t to grow:
+// smax > 0 and tr_scale > 0.)
 template <class DT>
 MRP_D float transmittance_span(const VolumeDev& v, Stream& st, f3 pos, f3 dir, float dis, float alpha, BoxSpan span) {
     const float smax = fm(v.max_density, alpha);
@@ -676,12 +674,18 @@ MRP_D float transmittance_span(const VolumeDev& v, Stream& st, f3 pos, f3 dir, f
 // Bound by the walks' instructions (Philox, log and division per step, lanes
 // of a warp ending apart).  768^3 over a 128^3 cloud: 262 -> 63 ms from one walk instead of 2 or 5 and
 // from walks that end with the box.
-template <class DT>
+//
+// GROWS: every step moves the walk on (launch_baked_tr).  A walk that goes
+// backwards or stands still (a negative or zero extinction or step scale)
+// takes transmittance as it is: it reads the density behind the voxel, and
+// carried past the far side by a negative density it comes back.  An instance
+// of its own: with a way back out of its first loop the other took 175 instead
+// of 125 ms for two bakes of 768^3.
+template <class DT, bool GROWS>
 __global__ void __launch_bounds__(128) k_baked_tr(float* __restrict__ out, const __grid_constant__ VolumeDev v,
                                                   int bake_res, float alpha, f3 L, uint32_t seed, int replicate,
                                                   int64_t first, int64_t count) {
     float rf = (float)bake_res;
-    const bool grows = v.max_density * alpha > 0.0f && v.tr_scale > 0.0f;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < count; q += (int64_t)gridDim.x * blockDim.x) {
         int64_t vi = first + q;
         int x = (int)(vi / ((int64_t)bake_res * bake_res)), y = (int)((vi / bake_res) % bake_res), z = (int)(vi % bake_res);
@@ -689,11 +693,15 @@ __global__ void __launch_bounds__(128) k_baked_tr(float* __restrict__ out, const
         f3 p = subs(uv, 0.5f);
         uint32_t hi = (uint32_t)(vi >> 32) * 8u;
         const float md = ray_box_distance(p, L);
-        const BoxSpan span = grows ? nonzero_span(v, p, L) : kOpenSpan;
+        const BoxSpan span = GROWS ? nonzero_span(v, p, L) : BoxSpan{};
+        auto walk = [&](Stream& st) {
+            if constexpr (GROWS) return transmittance_span<DT>(v, st, p, L, md, alpha, span);
+            else return transmittance<DT>(v, st, p, L, md, alpha);
+        };
         float res;
         if (replicate) {
             Stream st(kBakeStream, (uint32_t)vi, hi, 0, seed);
-            res = transmittance_span<DT>(v, st, p, L, md, alpha, span);
+            res = walk(st);
             // five equal terms: 0 and 1 sum exactly, others round on the way
             if (res != 0.0f && res != 1.0f && density(v, p) > 0) {
                 float acc = 0.0f;
@@ -705,7 +713,7 @@ __global__ void __launch_bounds__(128) k_baked_tr(float* __restrict__ out, const
             float acc = 0.0f;
             for (int i = 0; i < cnt; ++i) {
                 Stream st(kBakeStream, (uint32_t)vi, hi + (uint32_t)i, 0, seed);
-                acc = fa(acc, transmittance_span<DT>(v, st, p, L, md, alpha, span));
+                acc = fa(acc, walk(st));
             }
             res = fd(acc, (float)cnt);
         }
@@ -831,12 +839,14 @@ cudaError_t launch_baked_tr(float* out, const VolumeDev& v, int bake_res, float 
     int64_t total = (int64_t)bake_res * bake_res * bake_res;
     // bounded chunks keep every launch short
     const int64_t chunk = (int64_t)1 << 26;
+    const bool grows = v.max_density * alpha > 0.0f && v.tr_scale > 0.0f;   // every step's length is positive
     for (int64_t first = 0; first < total; first += chunk) {
         int64_t cnt = total - first < chunk ? total - first : chunk;
         const int grid = grid_for((size_t)cnt, 128, sms);
         const f3 l = mk3(L[0], L[1], L[2]);
-        if (v.density_h) k_baked_tr<__half><<<grid, 128, 0, s>>>(out, v, bake_res, alpha, l, seed, replicate, first, cnt);
-        else k_baked_tr<float><<<grid, 128, 0, s>>>(out, v, bake_res, alpha, l, seed, replicate, first, cnt);
+        auto kernel = v.density_h ? (grows ? k_baked_tr<__half, true> : k_baked_tr<__half, false>)
+                                  : (grows ? k_baked_tr<float, true> : k_baked_tr<float, false>);
+        kernel<<<grid, 128, 0, s>>>(out, v, bake_res, alpha, l, seed, replicate, first, cnt);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

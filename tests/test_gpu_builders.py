@@ -168,6 +168,21 @@ def test_bake_walks_backwards(alpha, tr_scale, replicate):
     assert np.mean(np.abs(got - ref) > 1e-4) < 0.01
 
 
+@pytest.mark.parametrize("replicate", [True, False])
+@pytest.mark.parametrize("alpha,tr_scale", [(-8.0, 1.0), (8.0, -0.5)])
+def test_bake_walks_back_and_forth(alpha, tr_scale, replicate):
+    """A backward walk into a negative density (a distance) is carried forward
+    by it, here past the far side, from where its next steps bring it back
+    into the cloud.  Both densities are constant, so a jump moves by no more
+    than its step's rounding; only in the one voxel between them does it
+    stretch that (by 2 a voxel's length, 48), once or twice a walk: below
+    1e-4, and the bar of the other walks holds."""
+    data = np.full((24, 24, 24), -1.5, np.float32)
+    data[:, :, 12:] = 0.25
+    got, ref = bake(24, data, 9, (0.0, 0.0, 1.0), alpha, replicate, tr_scale)
+    assert np.mean(np.abs(got - ref) > 1e-4) < 0.01
+
+
 @pytest.mark.parametrize("R,storage", [(2, "fp32"), (64, "fp16"), (200, "fp32"), (1030, "fp16")])
 def test_device_bytes(R, storage):
     """mrp_volume_info counts what a volume holds from its creation on and
