@@ -100,12 +100,13 @@ struct mrp_volume {
     bool stages_valid = false;
     float* density = nullptr;       // fp32 storage, or
     __half* density_h = nullptr;    // fp16 storage (MRP_STORAGE_FP16)
+    uint8_t* derived = nullptr;     // one allocation: mips, trs, lut, mip_tr, occ_rows and what follows each of them
     float* mips = nullptr;
     float* trs = nullptr;
     float* lut = nullptr;
     float* baked = nullptr;
     int baked_alloc_res = 0;
-    size_t held_bytes = 0;          // device memory allocated at creation
+    size_t held_bytes = 0;          // of the grid and derived
     uint8_t* occ = nullptr;
     uint8_t* mip_occ = nullptr;   // bricks of mip levels 0..kOccMips-1
     int occ_shift = 3, occ_res = 0;

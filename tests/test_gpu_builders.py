@@ -200,13 +200,14 @@ def test_device_bytes(R, storage):
     flags = sum((32 >> m) ** 3 for m in range(5)) + nb ** 3 + (-(-nb // 4)) ** 3 + 32
     want = R ** 3 * (2 if storage == "fp16" else 4) + 4 * floats + 8 * pairs + 16 * rows + flags
     v = M.VolumeRender(R, storage=storage)
-    assert v.info().device_bytes == want
+    held = v.info().device_bytes
+    assert want <= held < want + 5 * 256      # (five parts, each from a 256-byte boundary on)
     if R == 64:
         v.set_data(np.zeros((R, R, R), np.float32))
         v.Update()
         v.SetBakeResolution(21)
         v.Update_CachedTR((0.0, 1.0, 0.0), 1.0)
-        assert v.info().device_bytes == want + 21 ** 3 * 4
+        assert v.info().device_bytes == held + 21 ** 3 * 4
 
 
 @pytest.mark.parametrize("light", [(0.0, 1.0, 0.0), (0.0, 0.0, -1.0), (0.36, -0.48, 0.8)])
