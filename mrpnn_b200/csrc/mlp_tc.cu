@@ -758,31 +758,34 @@ MRP_D TailOut tc_tail_end(const Group& G, int st, float r, const float* aux) {
 }
 
 // An A row of N values that come in parts of 32: get(part, v) makes part
-// `part`.  FP8 rows take two passes, the first for the row's scale, so the
-// row is never held whole.
-template <int EB, int N, class F>
+// `part`.  FP8 rows need their scale first: with HOLD the row is held
+// meanwhile (the coloured form's threads have the registers: one set 119 ->
+// 108 us, 100 001 sets 353 -> 345); otherwise it is made twice and never held
+// whole.
+template <int EB, int N, bool HOLD, class F>
 MRP_D float write_parts(const Group& G, F get) {
-    float v[32];
+    constexpr int PARTS = N / 32, KEEP = EB == 1 && HOLD ? PARTS : 1;
+    float v[KEEP][32];
     if (EB == 2) {
 #pragma unroll
-        for (int p = 0; p < N / 32; ++p) {
-            get(p, v);
-            store_part<EB, N>(G, p, v, 1.0f);
+        for (int p = 0; p < PARTS; ++p) {
+            get(p, v[0]);
+            store_part<EB, N>(G, p, v[0], 1.0f);
         }
         return 1.0f;
     }
     float amax = 0.0f;
 #pragma unroll
-    for (int p = 0; p < N / 32; ++p) {
-        get(p, v);
+    for (int p = 0; p < PARTS; ++p) {
+        get(p, v[p % KEEP]);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(v[i]));
+        for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(v[p % KEEP][i]));
     }
     const float s = amax > 0.0f ? amax * (1.0f / 448.0f) : 1.0f, inv = 1.0f / s;
 #pragma unroll
-    for (int p = 0; p < N / 32; ++p) {
-        get(p, v);
-        store_part<EB, N>(G, p, v, inv);
+    for (int p = 0; p < PARTS; ++p) {
+        if (!HOLD) get(p, v[0]);
+        store_part<EB, N>(G, p, v[p % KEEP], inv);
     }
     return s;
 }
@@ -816,7 +819,7 @@ __device__ __noinline__ TailOut tc_tail(const Group G, int st, const float* aux,
         }
     }
     // LC0's A row: [comb * gate segment, LGGS (3 -> 8)]
-    float r = write_parts<EB, 128>(G, [&](int p, float (&v)[32]) {
+    float r = write_parts<EB, 128, COL>(G, [&](int p, float (&v)[32]) {
         if (p < 3) {
             tmem_get<32>(G, kColComb<COL> + 32 * p, v);
             const f32x2 q = pk2(gf[p], gf[p]);
@@ -839,7 +842,7 @@ __device__ __noinline__ TailOut tc_tail(const Group G, int st, const float* aux,
         }
     });
     st = mma_round<EB, 1>(G, st, kLC0, 0, 0, 0);
-    float rn = write_parts<EB, 128>(G, [&](int p, float (&v)[32]) {
+    float rn = write_parts<EB, 128, COL>(G, [&](int p, float (&v)[32]) {
         tmem_get<32>(G, 32 * p, v);
         if (p == 0) bias_relu<EB, 32>(v, kLC0, r, aux, 0);
         else if (p == 1) bias_relu<EB, 32>(v, kLC0, r, aux, 32);
@@ -848,14 +851,14 @@ __device__ __noinline__ TailOut tc_tail(const Group G, int st, const float* aux,
     });
     st = mma_round<EB, 1>(G, st, kLC1, 0, 0, 0);
     r = rn;
-    rn = write_parts<EB, 64>(G, [&](int p, float (&v)[32]) {
+    rn = write_parts<EB, 64, COL>(G, [&](int p, float (&v)[32]) {
         tmem_get<32>(G, 32 * p, v);
         if (p == 0) bias_relu<EB, 32>(v, kLC1, r, aux, 0);
         else bias_relu<EB, 32>(v, kLC1, r, aux, 32);
     });
     st = mma_round<EB, 1>(G, st, kLC2, 0, 0, 0);
     r = rn;
-    rn = write_parts<EB, 32>(G, [&](int, float (&v)[32]) {
+    rn = write_parts<EB, 32, COL>(G, [&](int, float (&v)[32]) {
         tmem_get<32>(G, 0, v);
         bias_relu<EB, 32>(v, kLC2, r, aux);
     });
