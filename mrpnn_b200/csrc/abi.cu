@@ -223,7 +223,6 @@ mrp_status mrp_load_model(const char* path) {
     if (!g.d_weights) CU(mrp::dev_malloc(&g.d_weights, sizeof(float) * fp32_weight_floats()));
     CU(fp32_prepare_weights(w.data(), g.d_weights));
     CU(tc_prepare_weights(w.data(), g.tc));
-    g.tc.d_fp32 = g.d_weights;
     g.model = std::move(m);
     g.h_weights = std::move(w);
     return MRP_OK;

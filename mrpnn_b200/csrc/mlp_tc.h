@@ -8,9 +8,7 @@ namespace mrp {
 // Weight images for the tensor-core kernels, built once per model.
 struct TcWeights {
     void* d_bf16 = nullptr;    // BF16 operand images of the 58 tensor-core layers
-    void* d_fp8 = nullptr;     // FP8-E4M3 operand images (weights / per-layer scale)
-    float* d_scales = nullptr; // FP8 weight scales per output channel (row amax / 448)
-    const float* d_fp32 = nullptr;   // the FP32 form's weights (set once a model is loaded; not read here)
+    void* d_fp8 = nullptr;     // FP8-E4M3 operand images (weights / scale of their output channel)
     float* d_aux = nullptr;    // fp32 constants of the CUDA-core parts, staged into shared memory
     int* d_err = nullptr;      // set to 1 when an MMA round times out
     int* d_counter = nullptr;  // tile counter of the persistent kernel
