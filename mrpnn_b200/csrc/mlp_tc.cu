@@ -858,9 +858,11 @@ __device__ __noinline__ TailOut tc_tail(const Group G, int st, const float* aux,
 // buffers.  Every value is made by the operations, in the order, that one
 // thread a row uses.  One FP8 tile of 300 sets: 111 k cycles with one thread
 // a row, two thirds of them in the SE blocks (9 to 10 k a block of width 32, a
-// third of that for its features to arrive); 70 k split, the next block's
-// features copied to shared memory meanwhile (4 k a block).  The call 83.5 ->
-// 70 us; a 163 x 97 FP8 frame of four launches 587 -> 528 us.  (With twice as
+// third of that for its features to arrive; 4 k split, the next block's
+// features copied to shared memory meanwhile).  The call 83.5 -> 70 us, and a
+// 163 x 97 FP8 frame of four launches 587 -> 528; since there is no loop over
+// tiles, around which its state spilled, another 63.6 -> 60.6 and 475 -> 468.
+// (With twice as
 // many sets, two tiles in turn an SM: 107 us the other form, 127 split.)
 // ---------------------------------------------------------------------------
 struct SplitScratch {
@@ -1365,18 +1367,14 @@ __global__ void __launch_bounds__(kGroups<COL> * kGroupThreads, 1) k_mlp_tc(cons
         G.a_s = tc::smem_addr(abuf);
         G.mbar_s = tc::smem_addr(mbar);
         G.tmem = tbase + ((uint32_t)(32 * (warp % 4)) << 16);
-        for (int tile = blockIdx.x; tile < total_tiles; tile += (int)gridDim.x) {
-            // (the first group's rounds alone are an even number, so all
-            // threads are at the same phase of its mbarrier here)
-            split_bar();
-            st = tile_work<STAGED>(A, segs, seg_start, rows, tile, G.t, G.g == 0,
+        if ((int)blockIdx.x < total_tiles)   // at most one tile a block (launch_tc)
+            st = tile_work<STAGED>(A, segs, seg_start, rows, (int)blockIdx.x, G.t, G.g == 0,
                                    [&](const auto& src, float gamma, float g, f3 sr, float* o) {
                                        const float s4 = powf(sr.x, 4.0f);
                                        const TailOut t = split_network<EB>(G, st, src, aux_s, X, gamma, g, s4);
                                        o[0] = o[1] = o[2] = radiance(t.p, s4);
                                        return t.st;
                                    });
-        }
     }
     // the first tiles go round the blocks, the rest to whichever group is free
     for (bool first = true; !SPLIT; first = false) {
@@ -1419,8 +1417,8 @@ static cudaError_t launch_tc(TcArgs& a, int sms, cudaStream_t s) {
     kernel<<<sms, kGroups<COL> * kGroupThreads, smem, s>>>(a);
     return cudaGetLastError();
 }
-// most: the most sets or records there can be (how many there are may be
-// known on the device only).  Up to one tile an SM a tile's latency is the
+// most: the most sets or records there can be, each segment's rounded up to a
+// tile (how many there are may be known on the device only).  Up to one tile an SM a tile's latency is the
 // call's, and the groups share it; from there on more tiles in flight are
 // worth more.
 template <bool STAGED>
