@@ -503,7 +503,7 @@ MRP_D float frac2(float f) { return f >= 1.0f ? fs(f, 1.0f) : f; }
 // One texel's constants and its two sample estimators.  The arithmetic is
 // Fill_Hg's; terms that its vectors carry without effect are left out: the
 // view direction is (1, 0, 0) and the texel's direction has no z, so of
-// sample_hg's vector only x = cos and y = -sin sin(phi) enter the dot
+// sample_hg's vector only x = cos and y = -sin sin(phi) + 0 cos enter the dot
 // product, and dot(normalize(p), view) is p.x / length(p).
 struct HgTexel {
     float g, radius, bn;
@@ -520,7 +520,8 @@ struct HgTexel {
         }
         const float phi = (float)(2.0 * 3.14159265359 * (double)e1);
         const float sint = fsq(fmaxf(0.0f, fs(1.0f, fm(cost, cost))));
-        const float sdotl = fa(fm(dir.x, cost), fm(dir.y, -fm(sint, sinf(phi))));
+        const float y = fa(-fm(sint, sinf(phi)), fm(0.0f, cost));   // (not a number where cost is infinite, |g| > 1)
+        const float sdotl = fa(fm(dir.x, cost), fm(dir.y, y));
         const float p = fa(fs(fm(radius, radius), 1.0f), fm(sdotl, sdotl));
         if (p <= 0) return 0.0f;
         const float w = fsq(p);

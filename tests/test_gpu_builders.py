@@ -67,6 +67,24 @@ def test_hg_table_texels(g, seed):
     assert np.max(rel) < 0.05
 
 
+@pytest.mark.parametrize("g,texels", [(2.0, (224430, 245486, 246279, 250037, 251486)), (-3.0, (242611, 250729)),
+                                      (-1.25, (254390, 261580)), (40.0, (220822, 233584, 234644))])
+def test_hg_table_infinite_cosine(g, texels):
+    """An asymmetry above 1, which the entry points accept: one phase sample
+    of each of these texels divides by 1 - g + 2 g e = 0.  Its direction is
+    not a number and counts as 0.  The texels are 1e9 and more from samples
+    beside the pole, whose cosine takes IEEE operations alone, so the bar is
+    that of the table test's texels without a flipped sample."""
+    import mrpnn_b200 as M
+    M.init()
+    tex = np.array(texels, np.int32)
+    v = M.VolumeRender(16)
+    v.UpdateHGLut(g)
+    ref = O.hg_lut_texels(g, 0, tex)
+    assert np.all(ref > 1e9) and np.all(np.isfinite(ref))
+    np.testing.assert_allclose(v.read(M.api.RES_LUT)[tex], ref, rtol=1e-4)
+
+
 @pytest.mark.parametrize("light", [(0.0, 1.0, 0.0), (0.0, 0.0, -1.0), (0.36, -0.48, 0.8), (-0.99, 0.1, 0.1)])
 @pytest.mark.parametrize("R,lo,hi", [(64, (0, 0, 0), (64, 64, 64)), (40, (30, 1, 12), (31, 2, 13)),
                                      (33, (0, 31, 7), (5, 33, 26)), (24, (0, 0, 0), (0, 0, 0))])
