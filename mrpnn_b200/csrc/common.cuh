@@ -199,6 +199,14 @@ MRP_D float fetch_clamp(const float* __restrict__ g, int n, int x, int y, int z)
     x = min(max(x, 0), n - 1); y = min(max(y, 0), n - 1); z = min(max(z, 0), n - 1);
     return __ldg(g + ((size_t)x * n + y) * n + z);
 }
+// x and x + 1 clamped to [0, n).  The sum is taken of a coordinate that is
+// clamped already: one that comes from an infinite or a huge position is the
+// largest int (a hit behind a density of -infinity lies there).
+MRP_D void clamp_pair(int x, int n, int* a, int* b) {
+    const int c = min(max(x, -1), n - 1);
+    *a = max(c, 0);
+    *b = min(c + 1, n - 1);
+}
 // lerp with 1 - v computed once by the caller (same operations, same result).
 MRP_D float lerp_w(float a, float b, float v, float omv) {
     // (both products in one instruction, each rounded as fm rounds it)
@@ -227,17 +235,20 @@ MRP_D float tex3(const T* __restrict__ g, int n, f3 pos) {
         t000 = ldg_f(b); t001 = ldg_f(b + 1); t010 = ldg_f(b + n); t011 = ldg_f(b + n + 1);
         t100 = ldg_f(b + nn); t101 = ldg_f(b + nn + 1); t110 = ldg_f(b + nn + n); t111 = ldg_f(b + nn + n + 1);
     } else {
-        int x0 = min(max(x, 0), n - 1), x1 = min(max(x + 1, 0), n - 1);
-        int y0 = min(max(y, 0), n - 1) * n, y1 = min(max(y + 1, 0), n - 1) * n;
-        int z0 = min(max(z, 0), n - 1), z1 = min(max(z + 1, 0), n - 1);
+        int x0, x1, y0, y1, z0, z1;
+        clamp_pair(x, n, &x0, &x1);
+        clamp_pair(y, n, &y0, &y1);
+        clamp_pair(z, n, &z0, &z1);
+        y0 *= n;
+        y1 *= n;
         const T* p0 = g + (size_t)x0 * nn;
         const T* p1 = g + (size_t)x1 * nn;
         t000 = ldg_f(p0 + y0 + z0); t001 = ldg_f(p0 + y0 + z1); t010 = ldg_f(p0 + y1 + z0); t011 = ldg_f(p0 + y1 + z1);
         t100 = ldg_f(p1 + y0 + z0); t101 = ldg_f(p1 + y0 + z1); t110 = ldg_f(p1 + y1 + z0); t111 = ldg_f(p1 + y1 + z1);
         if (!Clamp) {
-            bool vx0 = (unsigned)x < (unsigned)n, vx1 = (unsigned)(x + 1) < (unsigned)n;
-            bool vy0 = (unsigned)y < (unsigned)n, vy1 = (unsigned)(y + 1) < (unsigned)n;
-            bool vz0 = (unsigned)z < (unsigned)n, vz1 = (unsigned)(z + 1) < (unsigned)n;
+            bool vx0 = (unsigned)x < (unsigned)n, vx1 = (unsigned)x + 1u < (unsigned)n;
+            bool vy0 = (unsigned)y < (unsigned)n, vy1 = (unsigned)y + 1u < (unsigned)n;
+            bool vz0 = (unsigned)z < (unsigned)n, vz1 = (unsigned)z + 1u < (unsigned)n;
             t000 = vx0 && vy0 && vz0 ? t000 : 0.0f; t001 = vx0 && vy0 && vz1 ? t001 : 0.0f;
             t010 = vx0 && vy1 && vz0 ? t010 : 0.0f; t011 = vx0 && vy1 && vz1 ? t011 : 0.0f;
             t100 = vx1 && vy0 && vz0 ? t100 : 0.0f; t101 = vx1 && vy0 && vz1 ? t101 : 0.0f;
@@ -347,17 +358,20 @@ template <bool Clamp>
 __device__ __noinline__ float tex3_edge(const float* __restrict__ g, int n, int x, int y, int z, float wx, float wy,
                                         float wz) {
     const int nn = n * n;
-    int x0 = min(max(x, 0), n - 1) * nn, x1 = min(max(x + 1, 0), n - 1) * nn;
-    int y0 = min(max(y, 0), n - 1) * n, y1 = min(max(y + 1, 0), n - 1) * n;
-    int z0 = min(max(z, 0), n - 1), z1 = min(max(z + 1, 0), n - 1);
+    int x0, x1, y0, y1, z0, z1;
+    clamp_pair(x, n, &x0, &x1);
+    clamp_pair(y, n, &y0, &y1);
+    clamp_pair(z, n, &z0, &z1);
+    x0 *= nn; x1 *= nn;
+    y0 *= n; y1 *= n;
     float t000 = __ldg(g + x0 + y0 + z0), t001 = __ldg(g + x0 + y0 + z1);
     float t010 = __ldg(g + x0 + y1 + z0), t011 = __ldg(g + x0 + y1 + z1);
     float t100 = __ldg(g + x1 + y0 + z0), t101 = __ldg(g + x1 + y0 + z1);
     float t110 = __ldg(g + x1 + y1 + z0), t111 = __ldg(g + x1 + y1 + z1);
     if (!Clamp) {
-        bool vx0 = (unsigned)x < (unsigned)n, vx1 = (unsigned)(x + 1) < (unsigned)n;
-        bool vy0 = (unsigned)y < (unsigned)n, vy1 = (unsigned)(y + 1) < (unsigned)n;
-        bool vz0 = (unsigned)z < (unsigned)n, vz1 = (unsigned)(z + 1) < (unsigned)n;
+        bool vx0 = (unsigned)x < (unsigned)n, vx1 = (unsigned)x + 1u < (unsigned)n;
+        bool vy0 = (unsigned)y < (unsigned)n, vy1 = (unsigned)y + 1u < (unsigned)n;
+        bool vz0 = (unsigned)z < (unsigned)n, vz1 = (unsigned)z + 1u < (unsigned)n;
         t000 = vx0 && vy0 && vz0 ? t000 : 0.0f; t001 = vx0 && vy0 && vz1 ? t001 : 0.0f;
         t010 = vx0 && vy1 && vz0 ? t010 : 0.0f; t011 = vx0 && vy1 && vz1 ? t011 : 0.0f;
         t100 = vx1 && vy0 && vz0 ? t100 : 0.0f; t101 = vx1 && vy0 && vz1 ? t101 : 0.0f;
@@ -390,8 +404,9 @@ MRP_D float tex_lut(const float* __restrict__ lut, float u, float v) {
     float px = fs(fm(u, (float)kLut), 0.5f), py = fs(fm(v, (float)kLut), 0.5f);
     int x = (int)floorf(px), y = (int)floorf(py);
     float wx = fs(px, (float)x), wy = fs(py, (float)y);
-    int x0 = min(max(x, 0), kLut - 1), x1 = min(max(x + 1, 0), kLut - 1);
-    int y0 = min(max(y, 0), kLut - 1), y1 = min(max(y + 1, 0), kLut - 1);
+    int x0, x1, y0, y1;
+    clamp_pair(x, kLut, &x0, &x1);
+    clamp_pair(y, kLut, &y0, &y1);
     float r0 = lerp(__ldg(lut + y0 * kLut + x0), __ldg(lut + y1 * kLut + x0), wy);
     float r1 = lerp(__ldg(lut + y0 * kLut + x1), __ldg(lut + y1 * kLut + x1), wy);
     return lerp(r0, r1, wx);
@@ -415,8 +430,11 @@ MRP_D float tex_lut_fast(const float* __restrict__ lut, float u, float v) {
         const float* p = lut + y * kLut + x;
         a = __ldg(p); b = __ldg(p + kLut); c = __ldg(p + 1); d = __ldg(p + kLut + 1);
     } else {
-        int x0 = min(max(x, 0), kLut - 1), x1 = min(max(x + 1, 0), kLut - 1);
-        int y0 = min(max(y, 0), kLut - 1) * kLut, y1 = min(max(y + 1, 0), kLut - 1) * kLut;
+        int x0, x1, y0, y1;
+        clamp_pair(x, kLut, &x0, &x1);
+        clamp_pair(y, kLut, &y0, &y1);
+        y0 *= kLut;
+        y1 *= kLut;
         a = __ldg(lut + y0 + x0); b = __ldg(lut + y1 + x0); c = __ldg(lut + y0 + x1); d = __ldg(lut + y1 + x1);
     }
     return lerp_fast(lerp_fast(a, b, wy), lerp_fast(c, d, wy), wx);

@@ -97,3 +97,51 @@ def test_six_and_twelve_parts(precision, hardware):
                                    M.VolumeRender.MRPNN)
 
     np.testing.assert_array_equal(radiances(n), radiances(n + 1)[:n])
+
+
+@pytest.mark.parametrize("precision,hardware", [(1, True), (1, False), (2, False), (0, False)])
+def test_hits_at_infinity(precision, hardware):
+    """A density of -infinity takes a march to an infinite position, the hit
+    the reference's arithmetic gives there; the gathers read no texel for it
+    (a coordinate made of it is the largest integer).  Hits as the oracle's:
+    the march's order is the reference's up to the last bits of a logarithm."""
+    import mrpnn_b200 as M
+    from oracle import oracle as O
+    M.init()
+    R, W, H = 5, 33, 18
+    data = np.random.default_rng(3).uniform(0.05, 3.0, (R, R, R)).astype(np.float32)
+    data.ravel()[13] = -np.inf
+    v = M.VolumeRender(R)
+    v.set_data(data)
+    v.Update()
+    v.SetPrecision(precision)
+    v.SetGatherFilter(hardware)
+    ori, up, right = view_frame()
+    view = v.make_view((W, H), ori, up, right, LIGHT, 0.857, 64.0, seed=8)
+    rgba, aux, _ = v.predict_debug(view)
+    mips = np.concatenate([v.read(M.api.RES_MIP, m) for m in range(9)])
+    sc = O.SceneBuf(data.ravel(), R, v.max_density, mips, np.concatenate([v.read(M.api.RES_TR, m) for m in range(8)]),
+                    v.read(M.api.RES_LUT))
+    ov = O.make_view(W, H, ori, up, right, LIGHT, alpha=64.0, g=0.857, seed=8, frame=0)
+    _, _, _, hits = O.predict_pixels(sc, ov, np.arange(W * H, dtype=np.int32), want_features=True)
+    hit = hits[:, 3] > 0
+    assert np.isinf(hits[hit, :3]).any() and np.isfinite(hits[hit, :3]).all(1).sum() > 20
+    np.testing.assert_array_equal(aux[:, 3] > 0, hit)
+    np.testing.assert_allclose(aux[hit, :3], hits[hit, :3], rtol=1e-5, atol=1e-6)
+    frame = v.Render((W, H), ori, up, right, LIGHT, v.MRPNN, 0.857, 64.0, sampleNum=1, seed=8)
+    np.testing.assert_array_equal(frame.reshape(-1, 4), rgba)
+
+
+def test_features_far_away():
+    """Points beyond any integer texel coordinate: no density, and no shadow
+    where the light ray misses the box."""
+    sc = Scene(R=64)
+    far = [1e12, 1e30, 1e35, float("inf")]
+    pos = np.zeros((3 * len(far), 3), np.float32)
+    for a in range(3):
+        pos[a * len(far):(a + 1) * len(far), a] = far
+    frame = np.tile(np.array([1, 0, 0, 0, 1, 0, 0, 0, 1, *LIGHT], np.float32), (len(pos), 1))
+    feat, _ = sc.vol.gather_features(pos, frame, np.abs(LIGHT), sc.g, sc.alpha)
+    finite = np.isfinite(pos).all(1)
+    np.testing.assert_array_equal(feat[finite, :192], 0.0)
+    np.testing.assert_array_equal(feat[finite, 192:384], 1.0)
