@@ -256,6 +256,13 @@ __device__ __forceinline__ void split_bar() {
 __device__ __forceinline__ void group_bar(int g) {
     asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(kGroupThreads) : "memory");
 }
+// The same barrier; true for the whole group when `x` is for one of its threads.
+__device__ __forceinline__ bool group_any(int g, bool x) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %3, 0;\n\tbar.red.or.pred p, %1, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(r) : "r"(1 + g), "r"(kGroupThreads), "r"((uint32_t)x) : "memory");
+    return r != 0;
+}
 
 // Per-thread constants of a group, passed by value into the per-block
 // routines (a reference would put them in local memory and make every use a
@@ -1383,8 +1390,10 @@ __global__ void __launch_bounds__(kGroups<COL> * kGroupThreads, 1) k_mlp_tc(cons
                                    : kGroups<COL> * (int)gridDim.x + atomicAdd(A.tile_counter, 1);
         group_bar(G.g);
         int tile = tile_slot[G.g];
-        group_bar(G.g);
-        if (tile >= total_tiles || (st & kStFailed)) break;
+        // (a wait may have timed out for some of a group's threads only: they
+        // stop together, or the others would wait at the barrier for them)
+        const bool lost = group_any(G.g, st & kStFailed);
+        if (tile >= total_tiles || lost) break;
         // staged records from the last tile down: the gather wrote its
         // features in record order just before, so the last tiles' features
         // are still in L2 when the first groups ask for them
