@@ -1185,10 +1185,11 @@ cudaError_t launch_gather_rec(const VolumeDev& v, const ViewDev& view, HitRecord
     // 249 us at 724^2 pixels.  At 1024^2 (half of them hits) the records fill
     // the SMs by themselves: 465 against 444 us for the texture form, while
     // the FP32 form, waiting for its loads, still gains (961 against 978 us).
+    // The line lies between them, at 4054 pixels an SM (600 000 of 148).
     // Twelve threads of 16 points where even six leave the SMs short of warps:
     // 163 x 97, four launches, 510 -> 487 us, 128 x 128 213 -> 208, 256 x 256
     // 269 -> 266, 320 x 240 as before, 384 x 384 451 -> 460.
-    const int parts = n <= sms * 512 ? 12 : !fp16 || n <= 600000 ? 6 : 1;
+    const int parts = n <= sms * 512 ? 12 : !fp16 || n <= sms * 4054 ? 6 : 1;
     const dim3 grid((n + 127) / 128, parts);
     if (fp16 && v.glut_tex) k_gather_rec<true, true><<<grid, 128, 0, s>>>(v, view, rec, feat);
     else if (fp16) k_gather_rec<true><<<grid, 128, 0, s>>>(v, view, rec, feat);
