@@ -869,8 +869,8 @@ __device__ __noinline__ TailOut tc_tail(const Group G, int st, const float* aux,
 // features copied to shared memory meanwhile).  The call 83.5 -> 70 us, and a
 // 163 x 97 FP8 frame of four launches 587 -> 528; since there is no loop over
 // tiles, around which its state spilled, another 63.6 -> 60.6 and 475 -> 468.
-// (With twice as
-// many sets, two tiles in turn an SM: 107 us the other form, 127 split.)
+// (With twice as many sets, two tiles in turn an SM, that loop took 127 us, the
+// other form 107.)
 // ---------------------------------------------------------------------------
 struct SplitScratch {
     float4 stage[8][3 * kGroupThreads];   // the threads' slices of the next block (chunk, thread)
@@ -1427,9 +1427,10 @@ static cudaError_t launch_tc(TcArgs& a, int sms, cudaStream_t s) {
     return cudaGetLastError();
 }
 // most: the most sets or records there can be, each segment's rounded up to a
-// tile (how many there are may be known on the device only).  Up to one tile an SM a tile's latency is the
-// call's, and the groups share it; from there on more tiles in flight are
-// worth more.
+// tile.  Up to one tile an SM a tile's latency is the call's, and the groups
+// share it; from there on more tiles in flight are worth more.  Of a frame the
+// host knows its pixels only, not how many of them hit: one whose hits would
+// fit but whose pixels do not takes the other form.
 template <bool STAGED>
 static cudaError_t launch_tc(TcArgs& a, bool fp8, bool coloured, size_t most, int sms, cudaStream_t s) {
     if (coloured) return fp8 ? launch_tc<1, STAGED, true>(a, sms, s) : launch_tc<2, STAGED, true>(a, sms, s);

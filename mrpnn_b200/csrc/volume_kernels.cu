@@ -6,8 +6,9 @@
 // The reference builds the pyramid on the CPU (VolumeRender::Update,
 // core/volume.cu:1474-1515) and the TR mips / LUT / baked TR with legacy
 // texture + surface references (core/volume.cu:1322-1400, 1535-1696).  Here
-// every resource is a plain z-fastest fp32 array in HBM produced by one
-// kernel launch per level, on the volume's stream.
+// every resource is a plain z-fastest fp32 array in HBM, built on the volume's
+// stream: the pyramid's levels by a launch each, the TR levels by one, the
+// occupancy of the grid and of the mips by two each.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -196,9 +197,10 @@ __global__ void k_pad_levels(const float* __restrict__ l8, const float* __restri
 // every sample whose base voxel is in it or within one voxel of it (border
 // texels are 0 by addressing).
 //
-// DRAM bound: each voxel is read once (k_scan_rows), then the rows' masks,
-// a 32nd of the grid at most, are combined over 11 x 11 rows per brick column
-// (k_occ_bricks).  512^3 fp32 and the five mips: 160 us (the grid alone
+// DRAM bound: each voxel is read once (k_scan_rows), then the rows' masks are
+// combined over 11 x 11 rows per brick column (k_occ_bricks).  A row's masks
+// take 16 bytes per started 1024 voxels: a 32nd of the grid from 128^3 in fp32
+// and 256^3 in fp16 on, more below (an eighth at 32^3).  512^3 fp32 and the five mips: 160 us (the grid alone
 // 118 us, 4.6 TB/s) against 1.94 ms when the majorant, the bounds and each
 // brick's 11^3 voxels were read by kernels of their own.
 // ---------------------------------------------------------------------------
