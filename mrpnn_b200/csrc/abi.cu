@@ -285,28 +285,31 @@ mrp_status mrp_volume_create_ex(int res, mrp_storage storage, mrp_volume** out) 
     const size_t nocc = (size_t)v->occ_res * v->occ_res * v->occ_res,
                  nocc2 = (size_t)v->occ2_res * v->occ2_res * v->occ2_res,
                  nrow = std::max(occ_row_words(res), kMipOccRows);
-    // One allocation for everything derived from the grid: an allocation and
-    // its free cost about half a millisecond each (a volume of 64^3 created
-    // and destroyed: 2.8 ms with fourteen, most of them small, 3.5 with six
-    // of a megabyte and more, 0.95 with two).
+    // One allocation for everything derived from the grid but the LUT: an
+    // allocation and its free cost about half a millisecond each (a volume of
+    // 64^3 created and destroyed: 2.8 ms with fourteen, most of them small,
+    // 3.4 with six of a megabyte and more, 1.5 with three, 0.95 with two).  The
+    // LUT, below two megabytes, lies in a page of the driver's that has room
+    // for the small buffers of the first render; without it those took a new
+    // page then (a 512^2 animation step, set_data to frame: 3.8 -> 4.1 ms).
     size_t held = 0;
     auto part = [&](size_t bytes) { const size_t at = held; held += (bytes + 255) / 256 * 256; return at; };
     const size_t at_mips = part((kMipFloats + kPadLevelFloats) * sizeof(float)),
-                 at_trs = part((kTrFloats + kPadLevelFloats) * sizeof(float)), at_lut = part(kLutAlloc * sizeof(float)),
+                 at_trs = part((kTrFloats + kPadLevelFloats) * sizeof(float)),
                  at_pairs = part((mip_tr_offset(5) + kTrPadTexels + kPadLevelFloats) * sizeof(float2)),
                  at_rows = part(nrow * sizeof(uint4) + 32 + kMipOccBytes + nocc + nocc2);
     const size_t grid_bytes = n * (storage == MRP_STORAGE_FP16 ? sizeof(__half) : sizeof(float));
     if ((storage == MRP_STORAGE_FP16 ? (e = mrp::dev_malloc(&v->density_h, grid_bytes))
                                      : (e = mrp::dev_malloc(&v->density, grid_bytes))) != cudaSuccess ||
-        (e = mrp::dev_malloc(&v->derived, held)) != cudaSuccess)
+        (e = mrp::dev_malloc(&v->derived, held)) != cudaSuccess ||
+        (e = mrp::dev_malloc(&v->lut, kLutAlloc * sizeof(float))) != cudaSuccess)
         return cleanup(fail(e == cudaErrorMemoryAllocation ? MRP_ERR_OOM : MRP_ERR_CUDA, "volume allocation: %s",
                             cudaGetErrorString(e)));
-    v->held_bytes = grid_bytes + held;
+    v->held_bytes = grid_bytes + held + kLutAlloc * sizeof(float);
     v->mips = reinterpret_cast<float*>(v->derived + at_mips);
     v->mips_pad = v->mips + kMipFloats;
     v->trs = reinterpret_cast<float*>(v->derived + at_trs);
     v->trs_pad = v->trs + kTrFloats;
-    v->lut = reinterpret_cast<float*>(v->derived + at_lut);
     v->mip_tr = reinterpret_cast<float2*>(v->derived + at_pairs);
     v->mips_tr = v->mip_tr + mip_tr_offset(5);
     v->pad_pair = v->mips_tr + kTrPadTexels;
@@ -329,13 +332,12 @@ mrp_status mrp_volume_destroy(mrp_volume* v) {
     if (v->stream) cudaStreamSynchronize(v->stream);
     if (v->stream_copy) cudaStreamSynchronize(v->stream_copy);
     mrp::dev_free(v->accum_alt);
-    mrp::dev_free(v->density); mrp::dev_free(v->density_h); mrp::dev_free(v->derived); mrp::dev_free(v->baked); mrp::dev_free(v->accum); mrp::dev_free(v->sum3); mrp::dev_free(v->first_pos);
-    mrp::dev_free(v->counter);
+    mrp::dev_free(v->density); mrp::dev_free(v->density_h); mrp::dev_free(v->derived); mrp::dev_free(v->lut); mrp::dev_free(v->baked); mrp::dev_free(v->accum); mrp::dev_free(v->sum3);
     mrp::dev_free(v->hdri);
     drop_density_texture(v);
     drop_gather_textures(v);
     gtex_free(&v->baked_gtex);
-    mrp::dev_free(v->rec_count); mrp::dev_free(v->rec_pix); mrp::dev_free(v->rec_f); mrp::dev_free(v->feat);
+    mrp::dev_free(v->feat);
     tc_free_scratch(v->tc);
     free_multiview(v);
     if (v->ev0) cudaEventDestroy(v->ev0);
@@ -808,12 +810,15 @@ mrp_status mrp_update_baked_tr(mrp_volume* v, const float light_dir[3], float al
 namespace mrpi {
 mrp_status ensure_predictor_buffers(mrp_volume* v, size_t npix) {
     if (v->rec_cap >= npix) return MRP_OK;
-    mrp::dev_free(v->rec_count); mrp::dev_free(v->rec_pix); mrp::dev_free(v->rec_f); mrp::dev_free(v->feat);
+    mrp::dev_free(v->feat);
     v->rec_count = nullptr; v->rec_pix = nullptr; v->rec_f = nullptr; v->feat = nullptr; v->rec_cap = 0;
-    CU(mrp::dev_malloc(&v->rec_count, 2 * sizeof(int)));   // records, the march's pixel chunks
-    CU(mrp::dev_malloc(&v->rec_pix, npix * sizeof(int)));
-    CU(mrp::dev_malloc(&v->rec_f, npix * 16 * sizeof(float)));
-    CU(mrp::dev_malloc(&v->feat, tiled_feature_floats(npix) * sizeof(float)));
+    // one allocation, as above: a new volume's first animation step 3.9 -> 3.3
+    // ms, relighting 5.7 -> 5.3
+    const size_t nfeat = tiled_feature_floats(npix);
+    CU(mrp::dev_malloc(&v->feat, (nfeat + 17 * npix + 2) * sizeof(float)));
+    v->rec_f = v->feat + nfeat;
+    v->rec_pix = reinterpret_cast<int*>(v->rec_f + 16 * npix);
+    v->rec_count = v->rec_pix + npix;   // records, the march's pixel chunks
     CU(tc_ensure_scratch(v->tc));
     v->rec_cap = npix;
     return MRP_OK;
@@ -929,11 +934,11 @@ static mrp_status render_impl(mrp_volume* v, const mrp_view* w, mrp_render_type 
         TRY(mrp_render_wait(v, 0));
     TRY(ensure_accum(v, npix));
     if (type == MRP_PT && v->trace_pix < npix) {
-        mrp::dev_free(v->sum3); mrp::dev_free(v->first_pos); mrp::dev_free(v->counter);
+        mrp::dev_free(v->sum3);
         v->sum3 = nullptr; v->first_pos = nullptr; v->counter = nullptr; v->trace_pix = 0;
-        CU(mrp::dev_malloc(&v->sum3, npix * 3 * sizeof(double)));
-        CU(mrp::dev_malloc(&v->first_pos, npix * sizeof(int)));
-        CU(mrp::dev_malloc(&v->counter, sizeof(unsigned long long)));
+        CU(mrp::dev_malloc(&v->sum3, npix * 3 * sizeof(double) + sizeof(unsigned long long) + npix * sizeof(int)));
+        v->counter = reinterpret_cast<unsigned long long*>(v->sum3 + npix * 3);
+        v->first_pos = reinterpret_cast<int*>(v->counter + 1);
         v->trace_pix = npix;
     }
     // caches first (the reference updates them inside its launch loop,

@@ -100,13 +100,13 @@ struct mrp_volume {
     bool stages_valid = false;
     float* density = nullptr;       // fp32 storage, or
     __half* density_h = nullptr;    // fp16 storage (MRP_STORAGE_FP16)
-    uint8_t* derived = nullptr;     // one allocation: mips, trs, lut, mip_tr, occ_rows and what follows each of them
+    uint8_t* derived = nullptr;     // one allocation: mips, trs, mip_tr, occ_rows and what follows each of them
     float* mips = nullptr;
     float* trs = nullptr;
     float* lut = nullptr;
     float* baked = nullptr;
     int baked_alloc_res = 0;
-    size_t held_bytes = 0;          // of the grid and derived
+    size_t held_bytes = 0;          // of the grid, derived and lut
     uint8_t* occ = nullptr;
     uint8_t* mip_occ = nullptr;   // bricks of mip levels 0..kOccMips-1
     int occ_shift = 3, occ_res = 0;
@@ -143,11 +143,12 @@ struct mrp_volume {
     int async_slot = 0;
     int async_inflight = 0;
     bool async_tc = false;   // a tensor-core network ran since the last wait
-    double* sum3 = nullptr;
+    double* sum3 = nullptr;         // one allocation: counter and first_pos follow it
     int* first_pos = nullptr;
     unsigned long long* counter = nullptr;
     size_t trace_pix = 0;
-    // staged predictor buffers (records of hit pixels, tiled features)
+    // staged predictor buffers (tiled features, records of hit pixels): one
+    // allocation, at feat
     int* rec_count = nullptr;
     int* rec_pix = nullptr;
     float* rec_f = nullptr;
